@@ -14,9 +14,9 @@
  *   ME      - reference mode: SAD over the 11x11 coarse grid of
  *             megpu_kernels.cuh:27-166, then the 7x7 refinement of :307-446
  *             around its winner; full mode: every vector of [-15,15]^2;
- *           four packed pixels per step (__vabsdiffu4 + __dp4a on funnel-
- *           shifted words), two candidates interleaved per lane with split
- *           accumulators.  The reference picks a winner with a 2-D tree of
+ *           four packed pixels per step (vabsdiff4.add on funnel-shifted
+ *           words), each window row aligned once for a column of vectors.
+ *           The reference picks a winner with a 2-D tree of
  *           strict '<' comparisons in the order self, right, below, diagonal
  *           (:95-154); that tree returns the minimum cost and, among equal
  *           costs, the cell with the smallest Z-order index (x bits on even
@@ -161,6 +161,13 @@ __device__ __forceinline__ uint32_t spread8(uint32_t v)
     return v;
 }
 
+/* spread8 of a value below 16 */
+__device__ __forceinline__ constexpr uint32_t spread4(uint32_t v)
+{
+    v = (v | (v << 2)) & 0x33u;
+    return (v | (v << 1)) & 0x55u;
+}
+
 __device__ __forceinline__ uint32_t compact8(uint32_t v)
 {
     v &= 0x5555u;
@@ -296,105 +303,211 @@ __device__ __forceinline__ bool mbar_wait_bounded(uint64_t *bar, uint32_t parity
     return false;
 }
 
-/* sum of |a_i - b_i| over the four bytes, added to acc: per-byte absolute
- * difference, then a dot product with 1,1,1,1 (measured on B200 faster
- * than __vsadu4) */
+/* sum of |a_i - b_i| over the four bytes, added to acc: one instruction,
+ * one ALU-pipe slot (2.1 cycles a warp on an SM quarter).  The accumulating
+ * form is written in PTX because acc += __vsadu4(a, b) compiles to a
+ * separate add (5.1 against 4.05 cycles a word with its funnel shift), and
+ * __vabsdiffu4 + __dp4a issues two instructions for the same ALU time. */
 __device__ __forceinline__ uint32_t sad4(uint32_t a, uint32_t b, uint32_t acc)
 {
-    return __dp4a(__vabsdiffu4(a, b), 0x01010101u, acc);
+    uint32_t d;
+    asm("vabsdiff4.u32.u32.u32.add %0, %1, %2, %3;" : "=r"(d) : "r"(a), "r"(b), "r"(acc));
+    return d;
 }
 
-/* SADs of the source MB against the window blocks at two vectors, computed
- * together: four accumulators keep the dependency chains short */
-__device__ __forceinline__ void sad16x16_pair(const StageBuf s, int vx0, int vy0, int vx1, int vy1, uint32_t &s0,
-                                              uint32_t &s1)
+__device__ __forceinline__ uint32_t sad16(uint4 c, const uint32_t w[4], uint32_t acc)
 {
-    const int b0 = 16 + vx0, b1 = 16 + vx1;
-    const uint32_t *p0 = s.win(15 + vy0, b0 >> 2);
-    const uint32_t *p1 = s.win(15 + vy1, b1 >> 2);
-    const uint32_t sh0 = (uint32_t)(b0 & 3) * 8u, sh1 = (uint32_t)(b1 & 3) * 8u;
-    uint32_t a0 = 0, a1 = 0, c0 = 0, c1 = 0;
-#pragma unroll 4
-    for (int r = 0; r < 16; r++) {
-        const uint4 c = *reinterpret_cast<const uint4 *>(s.cur(r, 0));
-        const uint32_t x0 = p0[0], x1 = p0[1], x2 = p0[2], x3 = p0[3], x4 = p0[4];
-        const uint32_t y0 = p1[0], y1 = p1[1], y2 = p1[2], y3 = p1[3], y4 = p1[4];
-        a0 = sad4(c.x, __funnelshift_r(x0, x1, sh0), a0);
-        c0 = sad4(c.x, __funnelshift_r(y0, y1, sh1), c0);
-        a1 = sad4(c.y, __funnelshift_r(x1, x2, sh0), a1);
-        c1 = sad4(c.y, __funnelshift_r(y1, y2, sh1), c1);
-        a0 = sad4(c.z, __funnelshift_r(x2, x3, sh0), a0);
-        c0 = sad4(c.z, __funnelshift_r(y2, y3, sh1), c0);
-        a1 = sad4(c.w, __funnelshift_r(x3, x4, sh0), a1);
-        c1 = sad4(c.w, __funnelshift_r(y3, y4, sh1), c1);
-        p0 += WIN_PITCH_W;
-        p1 += WIN_PITCH_W;
+    return sad4(c.w, w[3], sad4(c.z, w[2], sad4(c.y, w[1], sad4(c.x, w[0], acc))));
+}
+
+/* sixteen window pixels of a row from word q on, `sh` bits into it */
+__device__ __forceinline__ void align16(const uint32_t *q, uint32_t sh, uint32_t w[4])
+{
+    const uint32_t x0 = q[0], x1 = q[1], x2 = q[2], x3 = q[3], x4 = q[4];
+    w[0] = __funnelshift_r(x0, x1, sh);
+    w[1] = __funnelshift_r(x1, x2, sh);
+    w[2] = __funnelshift_r(x2, x3, sh);
+    w[3] = __funnelshift_r(x3, x4, sh);
+}
+
+__device__ __forceinline__ uint4 cur_row(const StageBuf s, int r) { return *reinterpret_cast<const uint4 *>(s.cur(r, 0)); }
+
+/* window rows R0 .. R0 + NR - 1 of a column of five vectors three rows
+ * apart (row R of the column serves vector k with source row R - 3k), for
+ * the vectors K0 .. K1 that those rows reach */
+template <int R0, int NR, int K0, int K1>
+__device__ __forceinline__ void grid_rows(const StageBuf s, const uint32_t *p, uint32_t sh, uint32_t sad[5])
+{
+#pragma unroll
+    for (int i = 0; i < NR; i++) {
+        uint32_t w[4];
+        align16(p + (R0 + i) * WIN_PITCH_W, sh, w);
+#pragma unroll
+        for (int k = K0; k <= K1; k++)
+            sad[k] = sad16(cur_row(s, R0 + i - 3 * k), w, sad[k]);
     }
-    s0 = a0 + a1;
-    s1 = c0 + c1;
 }
 
-/* SADs of the source MB against N window blocks stacked one row apart:
- * the vectors (vx, vy0 + k), k < N, with vx in [-15, 15] and vy0 in
- * [-15, 16 - N].  Window row R serves candidate k with source row R - k,
- * so each of the 15 + N window rows is loaded and aligned once for all N
- * candidates (the pair above loads and aligns 16 rows per candidate).
- * Rows R < N - 1 and R > 15 reach only some candidates; they are unrolled
- * apart from the steady rows in between. */
-template <int N>
-__device__ __forceinline__ void sad16x16_column(const StageBuf s, int vx, int vy0, uint32_t sad[N])
+/* the 11x11 coarse grid; returns the smallest (cost << 10 | Z-order) key of
+ * the vectors inside the limits.
+ *
+ * The search's time is its ALU-pipe time: each 4-pixel difference and each
+ * funnel shift that aligns a window word takes one slot.  So a lane takes a
+ * column of vectors and aligns each window row once for all of them: lanes
+ * 0-10 the rows -14, -11, -8, -5, -2 of column `lane`, lanes 11-21 the rows
+ * 2, 5, 8, 11, 14, and lanes 22-31 row 0 of the ten columns other than x = 0
+ * (the first vector of the same instruction stream; what it computes for
+ * the other four is not used).  The zero vector, which needs no alignment,
+ * is summed by all lanes, half a row each.  28 window rows instead of 64
+ * are loaded and aligned a lane: 432 ALU slots and 690 instructions against
+ * 512 and 1,150 for two vectors a lane at a time (with the refinement below,
+ * 4,923 -> 3,808 instructions a macroblock and 113.9 -> 105.6 us for the
+ * encode launch of 13,464 macroblocks; unrolled, the rows run 3 % faster
+ * there than as loops).  Every row and word read is staged: rows 1 .. 44,
+ * words 0 .. 11. */
+__device__ __forceinline__ uint32_t grid_search(const StageBuf s, int lminx, int lmaxx, int lminy, int lmaxy, int lane)
 {
-    const int b = 16 + vx;
-    const uint32_t *p = s.win(15 + vy0, b >> 2);
+    const int g = lane >= 22 ? 2 : lane >= 11 ? 1 : 0;
+    const int c = lane - 11 * g, tx = g == 2 && c >= 5 ? c + 1 : c;
+    const int x = stage1_offset(tx), b = 16 + x;
+    const int y0 = g == 0 ? -14 : g == 1 ? 2 : 0;
+    const uint32_t *p = s.win(15 + y0, b >> 2);
     const uint32_t sh = (uint32_t)(b & 3) * 8u;
-    uint32_t lo[N], hi[N];   /* two accumulators per candidate: shorter chains */
+    uint32_t sad[5] = { 0u, 0u, 0u, 0u, 0u };
+    grid_rows<0, 3, 0, 0>(s, p, sh, sad);
+    grid_rows<3, 3, 0, 1>(s, p, sh, sad);
+    grid_rows<6, 3, 0, 2>(s, p, sh, sad);
+    grid_rows<9, 3, 0, 3>(s, p, sh, sad);
+    grid_rows<12, 4, 0, 4>(s, p, sh, sad);
+    grid_rows<16, 3, 1, 4>(s, p, sh, sad);
+    grid_rows<19, 3, 2, 4>(s, p, sh, sad);
+    grid_rows<22, 3, 3, 4>(s, p, sh, sad);
+    grid_rows<25, 3, 4, 4>(s, p, sh, sad);
+
+    /* the zero vector: words 2h, 2h + 1 of row r */
+    const int r = lane >> 1, h = lane & 1;
+    const uint2 wz = *reinterpret_cast<const uint2 *>(s.win(15 + r, 4 + 2 * h));
+    const uint2 cz = *reinterpret_cast<const uint2 *>(s.cur(r, 2 * h));
+    const uint32_t zero = __reduce_add_sync(FULL, sad4(cz.y, wz.y, sad4(cz.x, wz.x, 0u)));
+    uint32_t best = zero << 10 | zorder(5, 5);
+
+    /* Z-order bits of the rows: 0..4, 6..10 (lanes 11-21), 5 (lanes 22-31) */
+    const uint32_t zx = spread4((uint32_t)tx);
+    const bool okx = x >= lminx && x <= lmaxx;
 #pragma unroll
-    for (int k = 0; k < N; k++)
-        lo[k] = hi[k] = 0u;
-    auto row = [&](const uint32_t *q, uint32_t w[4]) {
-        const uint32_t x0 = q[0], x1 = q[1], x2 = q[2], x3 = q[3], x4 = q[4];
-        w[0] = __funnelshift_r(x0, x1, sh);
-        w[1] = __funnelshift_r(x1, x2, sh);
-        w[2] = __funnelshift_r(x2, x3, sh);
-        w[3] = __funnelshift_r(x3, x4, sh);
-    };
-    auto add = [&](int k, int r, const uint32_t w[4]) {
-        const uint4 c = *reinterpret_cast<const uint4 *>(s.cur(r, 0));
-        lo[k] = sad4(c.x, w[0], lo[k]);
-        hi[k] = sad4(c.y, w[1], hi[k]);
-        lo[k] = sad4(c.z, w[2], lo[k]);
-        hi[k] = sad4(c.w, w[3], hi[k]);
-    };
-    /* rows 0 .. N-2: candidates k <= R */
-#pragma unroll
-    for (int R = 0; R < N - 1; R++) {
-        uint32_t w[4];
-        row(p + R * WIN_PITCH_W, w);
-#pragma unroll
-        for (int k = 0; k <= R; k++)
-            add(k, R - k, w);
+    for (int k = 0; k < 5; k++) {
+        const int y = y0 + 3 * k;
+        const uint32_t zy = k == 0 ? (g == 0 ? spread4(0) : g == 1 ? spread4(6) : spread4(5))
+                                   : (g == 0 ? spread4(k) : spread4(6 + k));
+        const bool ok = okx && y >= lminy && y <= lmaxy && (k == 0 || g != 2);
+        best = min(best, ok ? (sad[k] << 10) | zx | (zy << 1) : FULL);
     }
-    /* rows N-1 .. 15: every candidate */
+    return __reduce_min_sync(FULL, best);
+}
+
+/* the 7x7 refinement around (v1x, v1y); returns the smallest key, whose
+ * Z-order counts from (v1x - 3, v1y - 3).
+ *
+ * Lane 4 tx + q sums rows 4q .. 4q + 3 of the block for the seven vectors of
+ * column tx: ten window rows aligned for 28 rows of differences, the four
+ * source rows in registers, then a reduce-scatter of the sums, two to a
+ * word, over the four lanes of a column (206 + 20 instructions, 152 ALU
+ * slots; two whole vectors a lane took 313 and 196).  A column that would
+ * reach past +-15 starts at the nearest one inside, and each vector takes
+ * its sum from there. */
+__device__ __forceinline__ uint32_t refine_search(const StageBuf s, int v1x, int v1y, int lminx, int lmaxx, int lminy,
+                                                  int lmaxy, int lane)
+{
+    const int tx = lane >> 2, q = lane & 3;
+    const int x = v1x + tx - 3, ylo = v1y - 3;
+    const int base = min(max(ylo, -15), 9);
+    const int b = 16 + min(max(x, -15), 15);
+    const uint32_t *p = s.win(15 + base + 4 * q, b >> 2);
+    const uint32_t sh = (uint32_t)(b & 3) * 8u;
+    uint4 c[4];
+#pragma unroll
+    for (int i = 0; i < 4; i++)
+        c[i] = cur_row(s, 4 * q + i);
+    uint32_t sad[8] = { 0u, 0u, 0u, 0u, 0u, 0u, 0u, 0u };
+#pragma unroll
+    for (int R = 0; R < 10; R++) {
+        uint32_t w[4];
+        align16(p + R * WIN_PITCH_W, sh, w);
+#pragma unroll
+        for (int k = 0; k < 7; k++)
+            if (R - k >= 0 && R - k < 4)
+                sad[k] = sad16(c[R - k], w, sad[k]);
+    }
+    /* sums of the block are at most 65,280: two fit a word */
+    uint32_t pk[4];
+#pragma unroll
+    for (int i = 0; i < 4; i++)
+        pk[i] = sad[2 * i] + (sad[2 * i + 1] << 16);
+    const bool up = (q & 2) != 0, odd = (q & 1) != 0;
+    uint32_t a0 = up ? pk[2] : pk[0], a1 = up ? pk[3] : pk[1];
+    a0 += __shfl_xor_sync(FULL, up ? pk[0] : pk[2], 2);
+    a1 += __shfl_xor_sync(FULL, up ? pk[1] : pk[3], 2);
+    const uint32_t v = (odd ? a1 : a0) + __shfl_xor_sync(FULL, odd ? a0 : a1, 1);
+    /* this lane's pair of the column: vectors base + 2q and base + 2q + 1 */
+    const uint32_t zx = spread4((uint32_t)tx);
+    const bool okx = tx < 7 && x >= lminx && x <= lmaxx;
+    uint32_t best = FULL;
+#pragma unroll
+    for (int k = 0; k < 2; k++) {
+        const int i = 2 * q + k, y = base + i, ty = y - ylo;
+        const bool ok = okx && i < 7 && ty >= 0 && ty < 7 && y >= lminy && y <= lmaxy;
+        const uint32_t cost = k ? v >> 16 : v & 0xFFFFu;
+        best = min(best, ok ? (cost << 10) | zx | (spread4((uint32_t)ty) << 1) : FULL);
+    }
+    return __reduce_min_sync(FULL, best);
+}
+
+/* window rows W0 .. W1 - 1 of the exhaustive search, source rows R0 .. R1 - 1 */
+template <int W0, int W1, int R0, int R1>
+__device__ __forceinline__ void full_rows(const StageBuf s, const uint32_t *p, uint32_t sh, int lminy, int lmaxy,
+                                          uint32_t acc[16], uint32_t &best)
+{
 #pragma unroll 1
-    for (int R = N - 1; R < 16; R++) {
+    for (int W = W0; W < W1; W++) {
         uint32_t w[4];
-        row(p + R * WIN_PITCH_W, w);
+        align16(p + W * WIN_PITCH_W, sh, w);
 #pragma unroll
-        for (int k = 0; k < N; k++)
-            add(k, R - k, w);
+        for (int r = R1 - 1; r >= R0; r--)
+            acc[r] = sad16(cur_row(s, r), w, r ? acc[r - 1] : 0u);
+        if (R1 == 16 && W - 30 >= lminy && W - 30 <= lmaxy)
+            best = min(best, (acc[15] << 10) | (spread8((uint32_t)(W - 15)) << 1));
     }
-    /* rows 16 .. 14+N: candidates k >= R - 15 */
+}
+
+/* every vector of [-15, 15]^2: lane tx takes column tx - 15 (lane 31 repeats
+ * column 15) and aligns each of the 46 window rows once for the sixteen
+ * vectors that it can serve.  acc[r] holds the sum over source rows 0 .. r of
+ * the vector whose row r is the window row at hand, so that one row of
+ * differences moves each sum one place on, and acc[15] is complete: 2,224
+ * differences and 184 alignments a lane, where columns of four vectors took
+ * 2,048 and 608, and half the instructions (64 QCIF pictures: 111.2 -> 95.5
+ * us for the encode launch).  Returns the smallest key (Z-order from
+ * (-15, -15)). */
+__device__ __forceinline__ uint32_t full_search(const StageBuf s, int lminx, int lmaxx, int lminy, int lmaxy, int lane)
+{
+    const int tx = min(lane, 30), x = tx - 15, b = 16 + x;
+    const uint32_t *p = s.win(0, b >> 2);
+    const uint32_t sh = (uint32_t)(b & 3) * 8u;
+    uint32_t acc[16], best = FULL;
 #pragma unroll
-    for (int R = 16; R < 15 + N; R++) {
-        uint32_t w[4];
-        row(p + R * WIN_PITCH_W, w);
-#pragma unroll
-        for (int k = R - 15; k < N; k++)
-            add(k, R - k, w);
-    }
-#pragma unroll
-    for (int k = 0; k < N; k++)
-        sad[k] = lo[k] + hi[k];
+    for (int r = 0; r < 16; r++)
+        acc[r] = 0u;
+    /* vectors -15 .. 15 start at window rows 0 .. 30: the first rows serve
+     * only the first source rows, the last rows only the last */
+    full_rows<0, 4, 0, 4>(s, p, sh, lminy, lmaxy, acc, best);
+    full_rows<4, 8, 0, 8>(s, p, sh, lminy, lmaxy, acc, best);
+    full_rows<8, 12, 0, 12>(s, p, sh, lminy, lmaxy, acc, best);
+    full_rows<12, 35, 0, 16>(s, p, sh, lminy, lmaxy, acc, best);
+    full_rows<35, 39, 4, 16>(s, p, sh, lminy, lmaxy, acc, best);
+    full_rows<39, 43, 8, 16>(s, p, sh, lminy, lmaxy, acc, best);
+    full_rows<43, 46, 12, 16>(s, p, sh, lminy, lmaxy, acc, best);
+    best = x >= lminx && x <= lmaxx && best != FULL ? best | spread8((uint32_t)tx) : FULL;
+    return __reduce_min_sync(FULL, best);
 }
 
 /* 4x4 Hadamard SATD, megpu_kernels.cuh:467-500 */
@@ -606,73 +719,20 @@ __device__ __forceinline__ void motion_estimate(const StageBuf s, const h261b_se
     const int lminx = max(-15, -bx), lmaxx = min(15, (S.mbw - 1) * 16 - bx);
     const int lminy = max(-15, -by), lmaxy = min(15, (S.mbh - 1) * 16 - by);
     int vx, vy;
-    /* every lane computes two SADs per iteration; a vector outside the
-     * limits is replaced by (0, 0) so no address leaves the window, and its
-     * cost discarded (65535, as the reference marks skipped candidates) */
+    /* a vector outside the limits never wins (the reference marks it with
+     * the cost 65535, above every block's): its sum, from staged or
+     * zero-filled pixels, is discarded; the zero vector is always inside */
     if (FULL_SEARCH) {
-        /* columns of four vertically adjacent vectors: 31 columns x 8
-         * groups, the last group (vy 13..15) started at vy 12, which the
-         * group before holds too (a repeated key changes no minimum) */
-        uint32_t best = FULL;
-        for (int t = lane; t < 31 * 8; t += 32) {
-            const int gy = t / 31, tx = t - gy * 31;
-            const int x = tx - 15, y0 = min(-15 + 4 * gy, 12);
-            uint32_t sad[4];
-            sad16x16_column<4>(s, x, y0, sad);
-            const bool ox = x >= lminx && x <= lmaxx;
-#pragma unroll
-            for (int k = 0; k < 4; k++) {
-                const int y = y0 + k;
-                const bool ok = ox && y >= lminy && y <= lmaxy;
-                best = min(best, ((ok ? sad[k] : 65535u) << 10) | zorder(tx, y + 15));
-            }
-        }
-        best = __reduce_min_sync(FULL, best) & 1023u; /* Z-order index only */
+        const uint32_t best = full_search(s, lminx, lmaxx, lminy, lmaxy, lane) & 1023u;
         vx = (int)compact8(best) - 15;
         vy = (int)compact8(best >> 1) - 15;
         s1x = s1y = 0;
     } else {
-        uint32_t best = FULL;
-        for (int c = lane; c < 121; c += 64) {
-            const int c1 = c + 32;
-            const bool has1 = c1 < 121;
-            const int ty0 = c / 11, tx0 = c - ty0 * 11, ty1 = (has1 ? c1 : c) / 11, tx1 = (has1 ? c1 : c) - ty1 * 11;
-            const int x0 = stage1_offset(tx0), y0 = stage1_offset(ty0), x1 = stage1_offset(tx1), y1 = stage1_offset(ty1);
-            const bool o0 = x0 >= lminx && x0 <= lmaxx && y0 >= lminy && y0 <= lmaxy;
-            const bool o1 = has1 && x1 >= lminx && x1 <= lmaxx && y1 >= lminy && y1 <= lmaxy;
-            uint32_t s0, s1;
-            sad16x16_pair(s, o0 ? x0 : 0, o0 ? y0 : 0, o1 ? x1 : 0, o1 ? y1 : 0, s0, s1);
-            best = min(best, ((o0 ? s0 : 65535u) << 10) | zorder(tx0, ty0));
-            if (has1)
-                best = min(best, ((o1 ? s1 : 65535u) << 10) | zorder(tx1, ty1));
-        }
-        best = __reduce_min_sync(FULL, best) & 1023u; /* Z-order index only */
-        const int v1x = stage1_offset((int)compact8(best)), v1y = stage1_offset((int)compact8(best >> 1));
+        const uint32_t coarse = grid_search(s, lminx, lmaxx, lminy, lmaxy, lane) & 1023u; /* Z-order index only */
+        const int v1x = stage1_offset((int)compact8(coarse)), v1y = stage1_offset((int)compact8(coarse >> 1));
         s1x = (int8_t)v1x;
         s1y = (int8_t)v1y;
-        /* the 7x7 refinement as 28 vertical pairs, lanes 0-27: column tx,
-         * rows 2gy and 2gy+1 (row 7 of the last pair is past the grid).  A
-         * pair reaching past +-15 is computed from the nearest in-window
-         * rows and each vector takes its SAD from there; vectors outside
-         * the limits are discarded as before */
-        best = FULL;
-        if (lane < 28) {
-            const int gy = lane / 7, tx = lane - gy * 7;
-            const int x = v1x + tx - 3, y0 = v1y + 2 * gy - 3;
-            const int base = min(max(y0, -15), 14);
-            uint32_t sad[2];
-            sad16x16_column<2>(s, min(max(x, -15), 15), base, sad);
-            const bool ox = x >= lminx && x <= lmaxx;
-#pragma unroll
-            for (int k = 0; k < 2; k++) {
-                const int y = y0 + k, ty = 2 * gy + k;
-                const bool ok = ox && ty < 7 && y >= lminy && y <= lmaxy;
-                const uint32_t v = (y - base) == 0 ? sad[0] : sad[1];
-                if (ty < 7)
-                    best = min(best, ((ok ? v : 65535u) << 10) | zorder(tx, ty));
-            }
-        }
-        best = __reduce_min_sync(FULL, best) & 1023u;
+        const uint32_t best = refine_search(s, v1x, v1y, lminx, lmaxx, lminy, lmaxy, lane) & 1023u;
         vx = v1x + (int)compact8(best) - 3;
         vy = v1y + (int)compact8(best >> 1) - 3;
     }
