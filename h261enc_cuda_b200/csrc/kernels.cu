@@ -23,7 +23,7 @@
  *           positions).  Each lane therefore folds (cost << 10 | zorder) into
  *           one 32-bit key and a single redux.sync min picks the same winner.
  *           Then the three 16x16 SATD costs of :617-987 (inter, inter with
- *           the 3x3 interior filter, intra).
+ *           the 3x3 interior filter, intra), each a small matrix product.
  *   MD      the decision of h261_moded.c:53-95.
  *   ENCDEC  per 8x8 block, one lane per row then per column: prediction
  *           with the H.261 loop filter, the reference's float/double AAN
@@ -510,27 +510,126 @@ __device__ __forceinline__ uint32_t full_search(const StageBuf s, int lminx, int
     return __reduce_min_sync(FULL, best);
 }
 
-/* 4x4 Hadamard SATD, megpu_kernels.cuh:467-500 */
-__device__ __forceinline__ int32_t satd4x4(const int32_t d[16])
+/* ------------------------------------------------ SATD (megpu_kernels.cuh:467-500)
+ *
+ * The 4x4 Hadamard of a macroblock's sixteen sub-blocks is one matrix
+ * product, [16 sub-blocks x 16 pixels] x [16 pixels x 16 signs], and its
+ * terms are small integers: pixel differences are exact in half precision
+ * (255 at most), the signs are +-1 and the sums (4,080 at most) exact in
+ * float, so two mma.sync m16n8k16 give the reference's integers.  The A
+ * fragment is one macroblock of pixels: lane 4g + t holds row t of sub-block
+ * g (sub-blocks 0-7, the upper half) and of sub-block g + 8, pixels 0 and 2
+ * of the row in one register, 1 and 3 in another (columns 2t, 2t + 1 and
+ * 2t + 8, 2t + 9 of A).
+ *
+ * tcgen05.mma is not used here: a product this small would wait longer for
+ * its operands to reach shared memory and its result to leave TMEM than the
+ * two mma.sync take (8.6 cycles each on an SM quarter).  Against one 4x4
+ * transform a lane in integers the costs take some 150 instructions a
+ * macroblock instead of 560: 105.6 -> 98.9 us for the encode launch of
+ * 13,464 macroblocks of mixed streams, 756 -> 716 us for 1024 QCIF streams. */
+
+/* D = A x B + C, half inputs, float sums */
+__device__ __forceinline__ void mma_16n8k16(float d[4], const uint32_t a[4], uint32_t b0, uint32_t b1, float c02)
 {
-    int32_t t[16];
+    asm("mma.sync.aligned.m16n8k16.row.col.f32.f16.f16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%10,%11,%10,%11};"
+        : "=f"(d[0]), "=f"(d[1]), "=f"(d[2]), "=f"(d[3])
+        : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b0), "r"(b1), "f"(c02), "f"(0.0f));
+}
+
+/* the SATD of a macroblock from its A fragment; `bias` is what every pixel
+ * of it has on top (it reaches only the sums with all signs +, the first
+ * column of the product) */
+__device__ __forceinline__ int32_t satd16x16(const uint32_t a[4], float bias, int lane)
+{
+    const int g = lane >> 2, t = lane & 3;
+    /* sign of pixel (x, y) in the transform (u, v): the parity of u & x and
+     * v & y; column g has u = g & 3 and v = g >> 2, then v + 2 */
+    const uint32_t neg = 0x80008000u;
+    const uint32_t b0 = (0x3C003C00u ^ ((g & 2) ? 0x80000000u : 0u)) ^ (((g >> 2) & t & 1) ? neg : 0u);
+    const uint32_t b1 = b0 ^ ((g & 1) ? neg : 0u), flip = (t & 2) ? neg : 0u;
+    float d[8];
+    mma_16n8k16(d, a, b0, b1, t == 0 ? -16.0f * bias : 0.0f);
+    mma_16n8k16(d + 4, a, b0 ^ flip, b1 ^ flip, 0.0f);
+    /* 2^23 + the lane's sum (32,640 at most): the integer is the float's low bits */
+    float sum = 8388608.0f;
+#pragma unroll
+    for (int i = 0; i < 8; i++)
+        sum = __fadd_rn(sum, fabsf(d[i]));
+    /* the 32 exponents add up to 32 * 0x4B000000 = 0x60000000 (mod 2^32) */
+    return (int32_t)(__reduce_add_sync(FULL, __float_as_uint(sum)) - 0x60000000u);
+}
+
+/* four pixels as halves 1024 + x: pixels 0 and 2, pixels 1 and 3 */
+__device__ __forceinline__ void half_pixels(uint32_t w, uint32_t &even, uint32_t &odd)
+{
+    even = __byte_perm(w, 0x64646464u, 0x4240);
+    odd = __byte_perm(w, 0x64646464u, 0x4341);
+}
+
+__device__ __forceinline__ uint32_t half_sub(uint32_t a, uint32_t b)
+{
+    uint32_t d;
+    asm("sub.rn.f16x2 %0, %1, %2;" : "=r"(d) : "r"(a), "r"(b));
+    return d;
+}
+
+/* the source MB as an A fragment of halves 1024 + x */
+__device__ __forceinline__ void source_halves(const StageBuf s, int lane, uint32_t c[4])
+{
+    const int g = lane >> 2, row = (g >> 2) * 4 + (lane & 3);
+    half_pixels(*s.cur(row, g & 3), c[0], c[2]);
+    half_pixels(*s.cur(row + 8, g & 3), c[1], c[3]);
+}
+
+__device__ __forceinline__ int32_t intra_cost(const StageBuf s, int lane)
+{
+    uint32_t c[4];
+    source_halves(s, lane, c);
+    return satd16x16(c, 1024.0f, lane);
+}
+
+/* the 16x16 SATD costs at vector (vx, vy): inter, and inter with the 3x3
+ * interior filter (megpu_kernels.cuh:617-987) */
+__device__ __forceinline__ void inter_costs(const StageBuf s, int vx, int vy, int lane, me_gpu_mb_t &res)
+{
+    const int g = lane >> 2, t = lane & 3, sx = g & 3, row = (g >> 2) * 4 + t;
+    uint32_t c[4], p[4], f[4];
+    source_halves(s, lane, c);
+    /* horizontal [1 2 1] sums of the lane's two rows of four pixels, 16 bits
+     * each, from the eight bytes that start one pixel to their left; the
+     * rows above and below belong to neighbouring lanes (t - 1, t + 1, or
+     * the sub-block four on) */
+    const int col = 15 + vx + 4 * sx;
+    const uint32_t *q = s.win(15 + vy + row, col >> 2);
+    const uint32_t sh = (uint32_t)(col & 3) * 8u;
+    const int up = t ? lane - 1 : lane - 13, down = t < 3 ? lane + 1 : lane + 13;
+    /* the filter applies to the interior (1..6) of each 8x8 block */
+    const int ly = (g & 4) + t;
+    const uint32_t rows = ly >= 1 && ly <= 6 ? 0x00FF00FFu : 0u;
+    const uint32_t even_in = rows & ((sx & 1) ? 0x00FF00FFu : 0x00FF0000u);
+    const uint32_t odd_in = rows & ((sx & 1) ? 0x000000FFu : 0x00FF00FFu);
+#pragma unroll
+    for (int h = 0; h < 2; h++) {
+        const uint32_t w0 = q[8 * h * WIN_PITCH_W], w1 = q[8 * h * WIN_PITCH_W + 1], w2 = q[8 * h * WIN_PITCH_W + 2];
+        const uint32_t lo = __funnelshift_r(w0, w1, sh), hi = __funnelshift_r(w1, w2, sh);
+        const uint32_t e = __byte_perm(lo, 0u, 0x4240), o = __byte_perm(lo, 0u, 0x4341);   /* bytes 0, 2; 1, 3 */
+        const uint32_t m = __byte_perm(e, hi, 0x1412), n = __byte_perm(o, hi, 0x1512);     /* bytes 2, 4; 3, 5 */
+        const uint32_t he = e + 2u * o + m, ho = o + 2u * m + n;
+        const uint32_t ve = __shfl_sync(FULL, he, up) + 2u * he + __shfl_sync(FULL, he, down) + 0x00080008u;
+        const uint32_t vo = __shfl_sync(FULL, ho, up) + 2u * ho + __shfl_sync(FULL, ho, down) + 0x00080008u;
+        p[h] = o | 0x64006400u;
+        p[h + 2] = m | 0x64006400u;
+        f[h] = (p[h] & ~even_in) | ((ve >> 4) & even_in);
+        f[h + 2] = (p[h + 2] & ~odd_in) | ((vo >> 4) & odd_in);
+    }
 #pragma unroll
     for (int i = 0; i < 4; i++) {
-        const int32_t a1 = d[4 * i] + d[4 * i + 1], a2 = d[4 * i] - d[4 * i + 1];
-        const int32_t a3 = d[4 * i + 2] + d[4 * i + 3], a4 = d[4 * i + 2] - d[4 * i + 3];
-        t[4 * i + 0] = a1 + a3;
-        t[4 * i + 1] = a2 + a4;
-        t[4 * i + 2] = a1 - a3;
-        t[4 * i + 3] = a2 - a4;
+        p[i] = half_sub(c[i], p[i]);
+        f[i] = half_sub(c[i], f[i]);
     }
-    int32_t satd = 0;
-#pragma unroll
-    for (int i = 0; i < 4; i++) {
-        const int32_t a1 = t[i] + t[4 + i], a2 = t[i] - t[4 + i];
-        const int32_t a3 = t[8 + i] + t[12 + i], a4 = t[8 + i] - t[12 + i];
-        satd += abs(a1 + a3) + abs(a2 + a4) + abs(a1 - a3) + abs(a2 - a4);
-    }
-    return satd;
+    res.i_16x16_cost = satd16x16(p, 0.0f, lane);
+    res.i_16x16_filter_cost = satd16x16(f, 0.0f, lane);
 }
 
 /* ---------------------------------------------- exact float/double math */
@@ -706,7 +805,7 @@ __device__ __forceinline__ void stage_mb(uint32_t *wbuf, int k, const h261b_sess
     }
 }
 
-/* motion search + SATD costs; results are warp-uniform.  FULL: the
+/* motion search + inter SATD costs; results are warp-uniform.  FULL: the
  * exhaustive search, else the reference's grid and refinement (a launch
  * compiles only the one it runs: a smaller body misses the instruction
  * cache less) */
@@ -737,49 +836,7 @@ __device__ __forceinline__ void motion_estimate(const StageBuf s, const h261b_se
         vy = v1y + (int)compact8(best >> 1) - 3;
     }
 
-    /* costs at the final vector: lanes 0-15 inter, 16-31 filtered inter,
-     * one 4x4 sub-block each; then intra on lanes 0-15.  Each lane reads
-     * six window rows around its sub-block (clamped to the window: a
-     * clamped row is one the sub-block never needs) from one column left of
-     * it, so pixel (iy, ix) is byte ix + 1 of row iy + 1 */
-    const int sb = lane & 15, sx = sb & 3, sy = sb >> 2;
-    const bool filt = lane >= 16;
-    const int wr0 = 15 + vy + sy * 4, wc0 = 16 + vx + sx * 4;
-    uint2 rr[6];
-#pragma unroll
-    for (int k = 0; k < 6; k++)
-        rr[k] = win8(s, min(max(wr0 - 1 + k, 0), WIN_ROWS - 1), wc0 - 1);
-    /* the 3x3 filter, separable: horizontal [1 2 1] sums of rows R = 0..5
-     * at columns C = 1..4, then vertical [1 2 1] over them.  Pixel (ix, iy)
-     * of the sub-block sits at (lx, ly) = ((sx & 1) * 4 + ix, (sy & 1) * 4
-     * + iy) of its 8x8 block; only the block's interior (1..6) is filtered */
-    int32_t hs[6][4];
-#pragma unroll
-    for (int R = 0; R < 6; R++) {
-#pragma unroll
-        for (int C = 1; C <= 4; C++)
-            hs[R][C - 1] = byte8(rr[R], C - 1) + 2 * byte8(rr[R], C) + byte8(rr[R], C + 1);
-    }
-    const uint32_t xin = (sx & 1) ? 0x7u : 0xEu, yin = (sy & 1) ? 0x7u : 0xEu; /* interior ix / iy bits */
-    int32_t d[16], di[16];
-#pragma unroll
-    for (int iy = 0; iy < 4; iy++) {
-        const uint32_t cw = *s.cur(sy * 4 + iy, sx);
-#pragma unroll
-        for (int ix = 0; ix < 4; ix++) {
-            const int c = (int)((cw >> (8 * ix)) & 0xFFu);
-            const int f = (hs[iy][ix] + 2 * hs[iy + 1][ix] + hs[iy + 2][ix] + 8) >> 4;
-            const bool use_f = filt && ((xin >> ix) & (yin >> iy) & 1u);
-            const int p = use_f ? f : byte8(rr[iy + 1], ix + 1);
-            d[iy * 4 + ix] = c - p;
-            di[iy * 4 + ix] = c;
-        }
-    }
-    const int32_t satd = satd4x4(d), satd_i = satd4x4(di);
-    res.i_16x16_cost = (int32_t)__reduce_add_sync(FULL, filt ? 0u : (uint32_t)satd);
-    res.i_16x16_filter_cost = (int32_t)__reduce_add_sync(FULL, filt ? (uint32_t)satd : 0u);
-    res.i_intra_cost = (int32_t)__reduce_add_sync(FULL, filt ? 0u : (uint32_t)satd_i);
-    res.i_zero_cost = 0;
+    inter_costs(s, vx, vy, lane, res);
     res.s_16x16_mv.i8_mx = (int8_t)vx;
     res.s_16x16_mv.i8_my = (int8_t)vy;
 }
@@ -1321,6 +1378,8 @@ __global__ void __launch_bounds__(256, KIND == KIND_SEARCH ? H261B_SEARCH_MIN_BL
         me.i_intra_cost = me.i_zero_cost = me.i_16x16_cost = me.i_16x16_filter_cost = 0;
         me.s_16x16_mv.i8_mx = me.s_16x16_mv.i8_my = 0;
         int8_t s1x = 0, s1y = 0;
+        if (do_me || (phases & H261B_PHASE_MD))
+            me.i_intra_cost = intra_cost(b, lane);   /* all that an intra picture needs */
         if (do_me) {
             /* the launch's search mode is the session's (checking build) */
             (void)H261B_CHECK(S.me_mode == (FULL_SEARCH ? 1 : 0), CHK_WORK_ITEM, S.me_mode);
@@ -1337,20 +1396,6 @@ __global__ void __launch_bounds__(256, KIND == KIND_SEARCH ? H261B_SEARCH_MIN_BL
 
         MbDecision m;
         if (phases & H261B_PHASE_MD) {
-            if (!do_me) {
-                /* intra picture without search: only the intra cost matters */
-                int32_t d[16];
-                const int sb = lane & 15;
-#pragma unroll
-                for (int iy = 0; iy < 4; iy++) {
-                    const uint32_t cw = *b.cur((sb >> 2) * 4 + iy, sb & 3);
-#pragma unroll
-                    for (int ix = 0; ix < 4; ix++)
-                        d[iy * 4 + ix] = (int32_t)((cw >> (8 * ix)) & 0xFFu);
-                }
-                const int32_t v = satd4x4(d);
-                me.i_intra_cost = (int32_t)__reduce_add_sync(FULL, lane < 16 ? (uint32_t)v : 0u);
-            }
             m = mode_decide(me, S.frame_type);
             if (lane == 0 && S.rc)
                 atomicAdd(&S.rc->cost_sum, m.cost);   /* the rate control's picture cost */
