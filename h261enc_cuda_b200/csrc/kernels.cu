@@ -61,16 +61,17 @@ constexpr int WIN_ROWS = 46;        /* rows mb_y-15 .. mb_y+30; columns mb_x-16 
 constexpr int WIN_PITCH_W = 36;
 constexpr int SRC_COL_W = 12;
 constexpr uint32_t FULL = 0xffffffffu;
+/* transpose buffer: rows of 12 words, blocks of 104, so that a row moves as
+ * two 16-byte accesses and neither the rows of a block (banks 12 r) nor the
+ * columns of the four blocks (banks 8 slot + c) conflict */
+constexpr int TB_ROW = 12, TB_BLOCK = 104;
 
 struct __align__(16) WarpSmem {
     uint32_t buf[WIN_ROWS * WIN_PITCH_W]; /* both buffers, interleaved      */
     uint64_t bar[2];                      /* per buffer: the barrier its bulk
                                              row copies complete on (bulk
                                              staging only)                   */
-    float t[4][72];                       /* transpose buffer: row stride 9,
-                                             block stride 72 words, so both
-                                             row and column accesses of the
-                                             four blocks are conflict-free   */
+    float t[4][TB_BLOCK];                 /* transpose buffer               */
 };
 
 /* one MB's staged inputs: buffer k of the warp's shared memory */
@@ -199,11 +200,6 @@ __device__ __forceinline__ uint2 glob8(const uint8_t *ptr)
     const uint32_t sh = (uint32_t)((uintptr_t)ptr & 3) * 8u;
     const uint32_t a = p[0], b = p[1], c = sh ? p[2] : 0u;
     return make_uint2(__funnelshift_r(a, b, sh), __funnelshift_r(b, c, sh));
-}
-
-__device__ __forceinline__ int byte8(uint2 v, int i)
-{
-    return (int)(((i < 4 ? v.x : v.y) >> (8 * (i & 3))) & 0xFFu);
 }
 
 /* asynchronous global -> shared copies; a 16-byte window chunk outside the
@@ -640,6 +636,20 @@ __device__ __forceinline__ float dmulf(float x, double k)
     return __double2float_rn(__dmul_rn((double)x, k));
 }
 
+/* `float *= k` for a double constant k = hi + lo, in float: the fused
+ * multiply-add rounds x * hi plus a term accurate to 2^-49 of the product,
+ * which is the double product rounded to float for every float x whose
+ * product is a normal number (tests/rounding_check_mul.c checks every
+ * mantissa): with k = 0.382683 and 1.84776 for all of them, with k =
+ * 0.707107 for all but three, of more than 18 significant bits each, so
+ * there for integers.  Two instructions at full rate (1.1 cycles a warp on
+ * an SM quarter each) where the conversions to and from double take 8 each. */
+__device__ __forceinline__ float mul_hilo(float x, double k)
+{
+    const float hi = (float)k, lo = (float)(k - (double)hi);
+    return __fmaf_rn(x, hi, __fmul_rn(x, lo));
+}
+
 /* `float = float * double + float`: fused (one rounding) or not */
 template <int FMAD>
 __device__ __forceinline__ float dmadf(float a, double k, float c)
@@ -649,30 +659,39 @@ __device__ __forceinline__ float dmadf(float a, double k, float c)
     return __double2float_rn(__dadd_rn(__dmul_rn((double)a, k), (double)c));
 }
 
-/* the AAN forward butterfly shared by both passes (mbgpu_kernels.cuh:359-388) */
-template <int FMAD>
+/* the AAN forward butterfly shared by both passes (mbgpu_kernels.cuh:359-388);
+ * INTS: its inputs are integers (the first pass) */
+template <int FMAD, bool INTS>
 __device__ __forceinline__ void fdct_butterfly(float tmp0, float tmp1, float tmp2, float tmp3, float tmp4,
                                                float tmp5, float tmp6, float tmp7, float o[8])
 {
     const float tmp10 = tmp0 + tmp3, tmp13 = tmp0 - tmp3, tmp11 = tmp1 + tmp2, tmp12 = tmp1 - tmp2;
     o[0] = tmp10 + tmp11;
     o[4] = tmp10 - tmp11;
-    const float z1 = dmulf(tmp12 + tmp13, 0.707107);
+    const float z1 = INTS ? mul_hilo(tmp12 + tmp13, 0.707107) : dmulf(tmp12 + tmp13, 0.707107);
     o[2] = tmp13 + z1;
     o[6] = tmp13 - z1;
     tmp4 = tmp4 + tmp5;
     tmp5 = tmp5 + tmp6;
     tmp6 = tmp6 + tmp7;
-    const float z5 = dmulf(tmp4 - tmp6, 0.382683);
+    const float z5 = mul_hilo(tmp4 - tmp6, 0.382683);
     const float z2 = dmadf<FMAD>(tmp4, 0.541196, z5);
     const float z4 = dmadf<FMAD>(tmp6, 1.306563, z5);
-    const float z3 = dmulf(tmp5, 0.707107);
+    const float z3 = INTS ? mul_hilo(tmp5, 0.707107) : dmulf(tmp5, 0.707107);
     const float z11 = tmp7 + z3, z13 = tmp7 - z3;
     o[5] = z13 + z2;
     o[3] = z13 - z2;
     o[1] = z11 + z4;
     o[7] = z11 - z4;
 }
+
+/* 1.5 * 2^23: a float of that magnitude has a unit of one, so a sum with it
+ * rounds to an integer, the way the addition rounds, and the integer is in
+ * its low bits (two's complement).  An addition runs at full rate; the
+ * conversions between float and integer take 8 cycles a warp. */
+constexpr float kBias = 12582912.0f;
+/* kBias + floor(x), |x| < 2^22 */
+__device__ __forceinline__ float floor_biased(float x) { return __fadd_rd(x, kBias); }
 
 /* floorf( cs * post * v + 0.49999 ) as the reference writes it
  * (mbgpu_kernels.cuh:413-437): a float product, the sum with the double
@@ -681,12 +700,11 @@ __device__ __forceinline__ void fdct_butterfly(float tmp0, float tmp1, float tmp
  * floorf(p + 0.49999f) with the float literal (the float nearest to
  * 0.49999) -- checked for all 2.5e9 floats of magnitude below 2^24 by
  * tests/rounding_check.c; above it both leave p unchanged -- so the sum is
- * taken in float and floored by the conversion itself: no conversion to or
- * from double. */
-__device__ __forceinline__ int32_t fdct_round(float cs, float post, float v)
+ * taken in float and floored by a sum that rounds down: no conversion. */
+__device__ __forceinline__ float fdct_round(float cs, float post, float v)
 {
     const float prod = __fmul_rn(__fmul_rn(cs, post), v);
-    return __float2int_rd(__fadd_rn(prod, 0.49999f));
+    return __fadd_rn(floor_biased(__fadd_rn(prod, 0.49999f)), -kBias);
 }
 
 /* the AAN inverse butterfly after its first level of adds (mbgpu_kernels.cuh
@@ -702,7 +720,7 @@ __device__ __forceinline__ void idct_rest(float tmp12, float tmp13, float tmp10,
     const float tmp0 = tmp10 + tmp13, tmp1 = tmp11 + tmp12, tmp2 = tmp11 - tmp12, tmp3 = tmp10 - tmp13;
     tmp13 = z11 + z13;
     tmp11 = dmulf(z11 - z13, 1.414214);
-    const float z5 = dmulf(z12 + z10, 1.84776);
+    const float z5 = mul_hilo(z12 + z10, 1.84776);
     tmp10 = dmadf<FMAD>(z12, 1.082392, -z5);
     tmp12 = dmadf<FMAD>(z10, -2.613126, z5);
     tmp12 = tmp12 - tmp13;
@@ -732,11 +750,16 @@ __device__ __forceinline__ float first_sub(float Pa, float csa, float ta, float 
     return FMAD ? __fmaf_rn(Pa, csa, -tb) : __fsub_rn(ta, tb);
 }
 
-/* CLAMP_255( (Int32) floor( v + 0.49999 ) ) with v widened to double */
-__device__ __forceinline__ int32_t idct_round(float v)
+/* floor( v + 0.49999 ) with v widened to double (mbgpu_kernels.cuh:924-931),
+ * in float: the sum rounded down to float has the exact sum's floor, as
+ * every integer of this range is a float, and the float literal next to
+ * 0.49999 separates the same floats (tests/rounding_check_mul.c checks every
+ * float of magnitude below 2^18).  The reference clamps the result to
+ * [-256, 255] before it adds the prediction and clamps to [0, 255], which
+ * gives the same pixel without the first clamp. */
+__device__ __forceinline__ float idct_round(float v)
 {
-    const int32_t r = (int32_t)floor(__dadd_rn((double)v, 0.49999));
-    return min(255, max(-256, r));
+    return __fadd_rn(floor_biased(__fadd_rd(v, 0.49999f)), -kBias);
 }
 
 /* ---------------------------------------------------------- per MB */
@@ -868,155 +891,132 @@ __device__ __forceinline__ MbDecision mode_decide(const me_gpu_mb_t &g, int fram
     return m;
 }
 
-/* H.261 loop-filter tap pair, horizontal [1 2 1] with x4 edge columns
- * (mbgpu_kernels.cuh:88-103) on one 8-pixel row */
-__device__ __forceinline__ int hfilt(uint2 v, int c)
+/* byte i of a row of eight, as the float 2^23 + x */
+__device__ __forceinline__ float pixel_biased(uint2 v, int i)
 {
-    if (c == 0)
-        return byte8(v, 0) * 4;
-    if (c == 7)
-        return byte8(v, 7) * 4;
-    return byte8(v, c - 1) + byte8(v, c) * 2 + byte8(v, c + 1);
+    return __uint_as_float(__byte_perm(i < 4 ? v.x : v.y, 0x4B000000u, 0x7650u + (uint32_t)(i & 3)));
 }
 
-/* one pass over up to four blocks of the MB: lane = slot * 8 + row (then
- * column).  Adds the block-summed |coefficient| of column (lane & 7) to
- * colsum[v] and returns this pass's CBP bits. */
-template <int FMAD, bool ABI>
-__device__ __forceinline__ uint32_t encdec_pass(float (*tb)[72], const StageBuf s, const h261b_session_dev_t &S,
-                                                int mb, int mbx, int mby, const MbDecision &m, int quant,
-                                                bool luma_pass, int lane, int32_t colsum[8], uint32_t &ssd)
+/* the low bytes of four words */
+__device__ __forceinline__ uint32_t pack4(float a, float b, float c, float d)
 {
-    const bool active = luma_pass || lane < 16;
-    const int slot = lane >> 3, r = lane & 7;
-    const int b = luma_pass ? slot : 4 + (slot & 1);
-    const bool intra = m.type == H261B_MB_TYPE_INTRA;
-    const bool filter = (m.flags & H261B_MB_FILTER) != 0;
-    const int t = intra ? 0 : 1;
+    return __byte_perm(__byte_perm(__float_as_uint(a), __float_as_uint(b), 0x0040),
+                       __byte_perm(__float_as_uint(c), __float_as_uint(d), 0x0040), 0x5410);
+}
 
-    /* ---- prediction and residual of row r (mbgpu_kernels.cuh:59-166):
-     * the source row and up to three reference rows as 8-byte vectors */
-    const int bx8 = luma_pass ? (b & 1) * 8 : 0, by8 = luma_pass ? (b >> 1) * 8 : 0;
-    int32_t res[8];
-    uint32_t pred_lo = 0, pred_hi = 0;   /* the row's prediction, one byte a pixel */
-    if (active) {
-        const uint2 cw = luma_pass ? *reinterpret_cast<const uint2 *>(s.cur(by8 + r, bx8 >> 2))
-                                   : *reinterpret_cast<const uint2 *>(s.curc(8 * (b - 4) + r));
-        if (intra) {
+/* H.261 loop filter of one row of an 8x8 block per lane (mbgpu_kernels.cuh
+ * :88-166): [1 2 1] across and down, x4 at the block's edge columns and
+ * rows.  Sums of four pixels at a time in 16-bit fields (4,088 at most), the
+ * rows above and below from the neighbouring lanes; an edge row takes itself
+ * for both, which gives (4 h + 8) >> 4 = (h + 2) >> 2. */
+__device__ __forceinline__ uint2 loop_filter(uint2 v, int lane)
+{
+    const uint32_t e0 = __byte_perm(v.x, 0u, 0x4240), o0 = __byte_perm(v.x, 0u, 0x4341);   /* 0, 2; 1, 3 */
+    const uint32_t e1 = __byte_perm(v.y, 0u, 0x4240), o1 = __byte_perm(v.y, 0u, 0x4341);   /* 4, 6; 5, 7 */
+    uint32_t h[4];
+    h[0] = ((2u * e0 + o0 + (o0 << 16)) & 0xFFFF0000u) | ((4u * e0) & 0xFFFFu);            /* 0, 2 */
+    h[1] = 2u * o0 + e0 + __byte_perm(e0, e1, 0x5432);                                     /* 1, 3 */
+    h[2] = 2u * e1 + o1 + __byte_perm(o0, o1, 0x5432);                                     /* 4, 6 */
+    h[3] = ((2u * o1 + e1 + (e1 >> 16)) & 0xFFFFu) | ((4u * o1) & 0xFFFF0000u);            /* 5, 7 */
+    const int r = lane & 7;
+    const bool edge = r == 0 || r == 7;
+    const int up = edge ? lane : lane - 1, down = edge ? lane : lane + 1;
 #pragma unroll
-            for (int i = 0; i < 8; i++)
-                res[i] = byte8(cw, i);
-        } else {
-            /* rows r-1, r, r+1 of the prediction block, clamped inside it
-             * (the edge rows of the loop filter use row r only) */
-            const int ra_i = max(r - 1, 0), rc_i = min(r + 1, 7);
-            uint2 ra, rb, rc;
-            if (luma_pass) {
-                int wr = 15 + m.mvy + by8, wc = 16 + m.mvx + bx8;
-                /* rows wr..wr+7 of the 46-row window, byte columns wc..wc+7
-                 * with win8's three words inside the 12-word row */
-                if (!H261B_CHECK(wr >= 0 && wr + 7 < WIN_ROWS && wc >= 0 && wc <= 40, CHK_MC_WINDOW,
-                                 wr * 64 + wc)) {
-                    wr = min(max(wr, 0), WIN_ROWS - 8);
-                    wc = min(max(wc, 0), 40);
-                }
-                rb = win8(s, wr + r, wc);
-                ra = filter ? win8(s, wr + ra_i, wc) : rb;
-                rc = filter ? win8(s, wr + rc_i, wc) : rb;
-            } else {
-                int cmx = m.mvx / 2, cmy = m.mvy / 2; /* truncation toward zero */
-#ifdef H261B_DEBUG_CHECKS
-                /* rows inside the chroma plane; glob8's words (12 bytes from
-                 * the word boundary when unaligned) inside the row */
-                {
-                    const int cx = mbx * 8 + cmx, cy = mby * 8 + cmy, wc8 = S.mbw * 8;
-                    if (!H261B_CHECK(cy >= 0 && cy + 8 <= S.mbh * 8 && cx >= 0 &&
-                                         (cx & ~3) + ((cx & 3) ? 12 : 8) <= wc8,
-                                     CHK_MC_CHROMA, cy * 4096 + cx))
-                        cmx = cmy = 0;
-                }
-#endif
-                const uint8_t *g = ((b == 4) ? S.ref_cb : S.ref_cr) + (size_t)(mby * 8 + cmy) * S.pitch_c +
-                                   (mbx * 8 + cmx);
-                rb = glob8(g + (size_t)r * S.pitch_c);
-                ra = filter ? glob8(g + (size_t)ra_i * S.pitch_c) : rb;
-                rc = filter ? glob8(g + (size_t)rc_i * S.pitch_c) : rb;
-            }
+    for (int i = 0; i < 4; i++) {
+        const uint32_t t = __shfl_sync(FULL, h[i], up) + 2u * h[i] + __shfl_sync(FULL, h[i], down) + 0x00080008u;
+        h[i] = (t >> 4) & 0x00FF00FFu;
+    }
+    return make_uint2(h[0] + (h[1] << 8), h[2] + (h[3] << 8));
+}
+
+/* what a lane needs of its block for one pass: the row lane & 7 of its
+ * pixels, then the column lane & 7 of its coefficients */
+struct BlockRow {
+    uint2 cur, pred;       /* the source row and its prediction (0 for intra)  */
+    uint8_t *rec;          /* where the reconstructed row goes                 */
+    bool active;
+};
+
+/* one pass over up to four blocks of the MB: lane = slot * 8 + row (then
+ * column).  Adds |coefficient| before the denoise to noise[v] (a float:
+ * integers below 2^24), and returns this pass's CBP bits.
+ *
+ * Everything between the pixels and the packed bytes is held in floats that
+ * are integers or the reference's own floats: sums with 2^23 or 1.5 * 2^23
+ * take the place of conversions, which run on a pipe of an eighth of the
+ * rate, and the statistics stay with their lane until a run is published.
+ * With the packed loop filter, 16-byte rows in the transpose buffer and no
+ * inverse transform for a pass without a coded block: 98.9 -> 83.4 us for
+ * the encode launch of 13,464 macroblocks of mixed streams, 716 -> 554 us for
+ * 1024 QCIF streams, 43.9 -> 40.7 us for 16 intra CIF pictures. */
+template <int FMAD, bool ABI>
+__device__ __forceinline__ uint32_t encdec_pass(float (*tb)[TB_BLOCK], const BlockRow &row,
+                                                const h261b_session_dev_t &S, int mb, const MbDecision &m, int quant,
+                                                uint4 offw, bool luma_pass, int lane, float fwd_c, float inv_c,
+                                                float noise[8], uint32_t &ssd)
+{
+    const int slot = lane >> 3, c = lane & 7;
+    const int b = luma_pass ? slot : 4 + (slot & 1);
+    const bool intra = m.type == H261B_MB_TYPE_INTRA, active = row.active;
+    float *const t = tb[slot];
+    /* ---- residual and FDCT pass 1 on row c (mbgpu_kernels.cuh:59-166, :359-388) */
+    {
+        float res[8], o[8];
 #pragma unroll
-            for (int i = 0; i < 8; i++) {
-                int p;
-                if (filter) {
-                    if (r == 0 || r == 7)
-                        p = (hfilt(rb, i) + 2) >> 2;
-                    else
-                        p = (hfilt(ra, i) + hfilt(rb, i) * 2 + hfilt(rc, i) + 8) >> 4;
-                } else {
-                    p = byte8(rb, i);
-                }
-                if (i < 4)
-                    pred_lo |= (uint32_t)p << (8 * i);
-                else
-                    pred_hi |= (uint32_t)p << (8 * (i - 4));
-                res[i] = byte8(cw, i) - p;
-            }
-        }
-        /* ---- FDCT pass 1 on row r */
-        float o[8];
-        fdct_butterfly<FMAD>((float)(res[0] + res[7]), (float)(res[1] + res[6]), (float)(res[2] + res[5]),
-                             (float)(res[3] + res[4]), (float)(res[3] - res[4]), (float)(res[2] - res[5]),
-                             (float)(res[1] - res[6]), (float)(res[0] - res[7]), o);
-#pragma unroll
-        for (int k = 0; k < 8; k++)
-            tb[slot][r * 9 + k] = o[k];
+        for (int i = 0; i < 8; i++)
+            res[i] = __fsub_rn(pixel_biased(row.cur, i), pixel_biased(row.pred, i));
+        fdct_butterfly<FMAD, true>(res[0] + res[7], res[1] + res[6], res[2] + res[5], res[3] + res[4],
+                                   res[3] - res[4], res[2] - res[5], res[1] - res[6], res[0] - res[7], o);
+        *reinterpret_cast<float4 *>(t + c * TB_ROW) = make_float4(o[0], o[1], o[2], o[3]);
+        *reinterpret_cast<float4 *>(t + c * TB_ROW + 4) = make_float4(o[4], o[5], o[6], o[7]);
     }
     __syncwarp();
 
-    /* ---- FDCT pass 2 on column c = r: coefficients (v, c), v = 0..7 */
-    const int c = r;
-    int32_t lev[8], nz[8];
-    int32_t acc = 0;
-#pragma unroll
-    for (int v = 0; v < 8; v++) {
-        lev[v] = 0;
-        nz[v] = 0;
-    }
-    if (active) {
+    /* ---- FDCT pass 2 on column c: coefficients (v, c), v = 0..7 */
+    float lev[8];   /* the levels, signed */
+    uint32_t lo, hi;
+    int32_t acc;
+    {
         float q[8], o[8];
 #pragma unroll
         for (int k = 0; k < 8; k++)
-            q[k] = tb[slot][k * 9 + c];
-        fdct_butterfly<FMAD>(q[0] + q[7], q[1] + q[6], q[2] + q[5], q[3] + q[4], q[3] - q[4], q[2] - q[5],
-                             q[1] - q[6], q[0] - q[7], o);
-        const float cs = __fmul_rn(c_fwd_post[c], 0.125f); /* = dmulf(.., 0.125): a power-of-two scaling is exact */
+            q[k] = t[k * TB_ROW + c];
+        fdct_butterfly<FMAD, false>(q[0] + q[7], q[1] + q[6], q[2] + q[5], q[3] + q[4], q[3] - q[4], q[2] - q[5],
+                                    q[1] - q[6], q[0] - q[7], o);
         const float inv = c_inv_quant[quant];
-        /* this column's eight offsets, UInt16, one 16-byte load */
-        const uint4 ow = *reinterpret_cast<const uint4 *>(&S.dn->offset[t][c][0]);
-        const uint32_t offw[4] = { ow.x, ow.y, ow.z, ow.w };
+        const uint32_t ow[4] = { offw.x, offw.y, offw.z, offw.w };
+        float mag[8];
+        int32_t dc = 0;
 #pragma unroll
         for (int v = 0; v < 8; v++) {
-            int32_t lv = fdct_round(cs, c_fwd_post[v], o[v]);
-            /* denoise (mbgpu_kernels.cuh:586-604) */
-            const int32_t sign = lv >> 31;
-            lv = (lv ^ sign) - sign;
-            nz[v] = lv;
-            const int32_t off = (int32_t)((offw[v >> 1] >> (16 * (v & 1))) & 0xFFFFu);
-            lv = max(lv - off, 0);
-            lv = (lv ^ sign) - sign;
-            /* quant (mbgpu_kernels.cuh:689-716) */
-            if (intra && v == 0 && c == 0) {
-                int32_t dc = lv / 8;
-                dc = max(dc, 1);
-                dc = min(dc, 254);
-                if (dc == 128)
-                    dc = 255;
-                lev[0] = dc;
-                acc += 100;
-            } else {
-                const int32_t l = min(127, max(-127, __float2int_rz(__fmul_rn(__int2float_rn(lv), inv))));
-                lev[v] = l;
-                const int32_t al = abs(l);
-                acc += al > 1 ? 100 : al;
+            const float lv = fdct_round(fwd_c, c_fwd_post[v], o[v]);
+            noise[v] += active ? fabsf(lv) : 0.0f;
+            /* denoise (mbgpu_kernels.cuh:586-604) on the magnitude, quant
+             * (:689-716): the product truncated, which is the same on the
+             * magnitude, at most 127 */
+            const float off = (float)((ow[v >> 1] >> (16 * (v & 1))) & 0xFFFFu);
+            const float shrunk = fmaxf(fabsf(lv) - off, 0.0f);
+            mag[v] = __fadd_rz(fminf(__fmul_rn(shrunk, inv), 127.0f), 8388608.0f);
+            lev[v] = copysignf(__fadd_rn(mag[v], -8388608.0f), lv);
+            if (v == 0) {
+                /* intra DC: the denoised coefficient / 8 as 1 .. 254, 128 as 255 */
+                dc = (int32_t)copysignf(shrunk, lv) / 8;
+                dc = min(max(dc, 1), 254);
+                dc = dc == 128 ? 255 : dc;
             }
+        }
+        /* the coded-block rule: 100 for a level beyond +-1 (and an intra DC),
+         * 1 for +-1 */
+        const uint32_t m0 = pack4(mag[0], mag[1], mag[2], mag[3]), m1 = pack4(mag[4], mag[5], mag[6], mag[7]);
+        lo = pack4(__fadd_rn(lev[0], kBias), __fadd_rn(lev[1], kBias), __fadd_rn(lev[2], kBias),
+                   __fadd_rn(lev[3], kBias));
+        hi = pack4(__fadd_rn(lev[4], kBias), __fadd_rn(lev[5], kBias), __fadd_rn(lev[6], kBias),
+                   __fadd_rn(lev[7], kBias));
+        acc = __popc((m0 & 0x01010101u) | ((m1 & 0x01010101u) << 1));
+        acc = ((m0 | m1) & 0xFEFEFEFEu) || (intra && c == 0) ? 100 : acc;
+        if (intra && c == 0) {
+            lo = (lo & 0xFFFFFF00u) | (uint32_t)dc;
+            lev[0] = dc == 255 ? 128.0f : (float)dc;
         }
     }
     /* block sums over the 8 lanes of a block */
@@ -1026,131 +1026,129 @@ __device__ __forceinline__ uint32_t encdec_pass(float (*tb)[72], const StageBuf 
     const bool coded = active && acc > 2;
     const uint32_t cbp = __reduce_or_sync(FULL, coded ? (uint32_t)H261B_CBP_BIT(b) : 0u);
 
-    /* denoise statistics: sum the same coefficient position over blocks */
-#pragma unroll
-    for (int v = 0; v < 8; v++) {
-        int32_t x = nz[v];
-        x += __shfl_xor_sync(FULL, x, 8);
-        x += __shfl_xor_sync(FULL, x, 16);
-        colsum[v] += x;
-    }
-
-    /* ---- levels out */
+    /* ---- levels out: column-major, this lane's eight are contiguous */
     if (active) {
         if (ABI && S.abi_out) {
             int32_t *tc = S.abi_out[mb].rgi_tcoeff[b];
 #pragma unroll
-            for (int v = 0; v < 8; v++)
-                tc[v * 8 + c] = lev[v];
-        }
-        if (S.level_out) {
-            /* column-major: this lane's eight levels are contiguous */
-            uint32_t lo = 0, hi = 0;
-#pragma unroll
-            for (int v = 0; v < 4; v++) {
-                lo |= ((uint32_t)lev[v] & 0xFFu) << (8 * v);
-                hi |= ((uint32_t)lev[v + 4] & 0xFFu) << (8 * v);
+            for (int v = 0; v < 8; v++) {
+                const uint32_t x = (v < 4 ? lo : hi) >> (8 * (v & 3));
+                tc[v * 8 + c] = v == 0 && c == 0 && intra ? (int32_t)(x & 0xFFu) : (int32_t)(int8_t)x;
             }
-            *reinterpret_cast<uint2 *>(S.level_out + (size_t)mb * 384 + b * 64 + c * 8) = make_uint2(lo, hi);
         }
+        if (S.level_out)
+            *reinterpret_cast<uint2 *>(S.level_out + (size_t)mb * 384 + b * 64 + c * 8) = make_uint2(lo, hi);
     }
 
-    /* ---- dequant (mbgpu_kernels.cuh:763-814) and IDCT pass 1 on column c */
-    __syncwarp(); /* pass-2 reads of the transpose buffer are done */
-    if (active) {
-        const int32_t qa = coded ? ((quant - 1) | 1) : 0, qm = coded ? quant * 2 : 0;
-        float col[8];
+    /* ---- dequant (mbgpu_kernels.cuh:763-814) and IDCT pass 1 on column c;
+     * a block that is not coded has coefficients of zero, and a pass without
+     * a coded block is its prediction */
+    uint2 out = row.pred;
+    if (cbp) {
+        const float qa = coded ? (float)((quant - 1) | 1) : 0.0f, qm = coded ? (float)(2 * quant) : 0.0f;
+        float P[8], cs[8], tt[8], o[8];
 #pragma unroll
         for (int k = 0; k < 8; k++) {
-            int32_t dq;
-            if (intra && k == 0 && c == 0) {
-                dq = lev[0] == 255 ? 1024 : lev[0] * 8;
-            } else {
-                int32_t l = lev[k] * qm;
-                if (l > 0)
-                    l += qa;
-                else if (l < 0)
-                    l -= qa;
-                dq = min(2047, max(-2048, l));
-            }
-            col[k] = (float)dq;
-        }
-        if (coded) {
+            /* level * 2 QUANT, plus its sign times QUANT rounded down to odd */
+            const float sign = fminf(fmaxf(lev[k], -1.0f), 1.0f);
+            float dq = __fmaf_rn(lev[k], qm, __fmul_rn(sign, qa));
+            dq = fminf(fmaxf(dq, -2048.0f), 2047.0f);
+            if (k == 0 && intra && c == 0)
+                dq = lev[0] * 8.0f;
             /* prescale: t = (coef * pre[col]) * (pre[row] * 0.125) */
-            float P[8], cs[8], tt[8], o[8];
-#pragma unroll
-            for (int k = 0; k < 8; k++) {
-                cs[k] = __fmul_rn(c_inv_pre[k], 0.125f); /* exact, as dmulf(.., 0.125) */
-                P[k] = __fmul_rn(col[k], c_inv_pre[c]);
-                tt[k] = __fmul_rn(P[k], cs[k]);
-            }
-            idct_rest<FMAD>(first_sub<FMAD>(P[2], cs[2], tt[2], tt[6]), first_add<FMAD>(P[2], cs[2], tt[2], tt[6]),
-                            first_add<FMAD>(P[0], cs[0], tt[0], tt[4]), first_sub<FMAD>(P[0], cs[0], tt[0], tt[4]),
-                            first_add<FMAD>(P[1], cs[1], tt[1], tt[7]), first_sub<FMAD>(P[1], cs[1], tt[1], tt[7]),
-                            first_add<FMAD>(P[5], cs[5], tt[5], tt[3]), first_sub<FMAD>(P[5], cs[5], tt[5], tt[3]), o);
-#pragma unroll
-            for (int k = 0; k < 8; k++)
-                tb[slot][k * 9 + c] = o[k];
-        } else {
-#pragma unroll
-            for (int k = 0; k < 8; k++)
-                tb[slot][k * 9 + c] = col[k];
+            cs[k] = __fmul_rn(c_inv_pre[k], 0.125f); /* exact, as dmulf(.., 0.125) */
+            P[k] = __fmul_rn(dq, inv_c);
+            tt[k] = __fmul_rn(P[k], cs[k]);
         }
-    }
-    __syncwarp();
+        idct_rest<FMAD>(first_sub<FMAD>(P[2], cs[2], tt[2], tt[6]), first_add<FMAD>(P[2], cs[2], tt[2], tt[6]),
+                        first_add<FMAD>(P[0], cs[0], tt[0], tt[4]), first_sub<FMAD>(P[0], cs[0], tt[0], tt[4]),
+                        first_add<FMAD>(P[1], cs[1], tt[1], tt[7]), first_sub<FMAD>(P[1], cs[1], tt[1], tt[7]),
+                        first_add<FMAD>(P[5], cs[5], tt[5], tt[3]), first_sub<FMAD>(P[5], cs[5], tt[5], tt[3]), o);
+        __syncwarp(); /* pass-2 reads of the transpose buffer are done */
+#pragma unroll
+        for (int k = 0; k < 8; k++)
+            t[k * TB_ROW + c] = o[k];
+        __syncwarp();
 
-    /* ---- IDCT pass 2 on row r and reconstruction (mbgpu_kernels.cuh:988-1096) */
+        /* ---- IDCT pass 2 on row c and reconstruction (mbgpu_kernels.cuh:988-1096) */
+        const float4 p0 = *reinterpret_cast<const float4 *>(t + c * TB_ROW);
+        const float4 p1 = *reinterpret_cast<const float4 *>(t + c * TB_ROW + 4);
+        idct_rest<FMAD>(p0.z - p1.z, p0.z + p1.z, p0.x + p1.x, p0.x - p1.x, p0.y + p1.w, p0.y - p1.w, p1.y + p0.w,
+                        p1.y - p0.w, o);
+#pragma unroll
+        for (int i = 0; i < 8; i++)
+            o[i] = fminf(fmaxf(idct_round(o[i]) + pixel_biased(row.pred, i), 8388608.0f), 8388608.0f + 255.0f);
+        out = make_uint2(pack4(o[0], o[1], o[2], o[3]), pack4(o[4], o[5], o[6], o[7]));
+    }
     if (active) {
-        const float *p = tb[slot] + r * 9;
-        int32_t out[8];
-        if (coded) {
-            float o[8];
-            idct_rest<FMAD>(p[2] - p[6], p[2] + p[6], p[0] + p[4], p[0] - p[4], p[1] + p[7], p[1] - p[7],
-                            p[5] + p[3], p[5] - p[3], o);
-#pragma unroll
-            for (int i = 0; i < 8; i++)
-                out[i] = idct_round(o[i]);
-        } else {
-#pragma unroll
-            for (int i = 0; i < 8; i++)
-                out[i] = (int32_t)p[i];
-        }
-        uint32_t lo = 0, hi = 0;
-#pragma unroll
-        for (int i = 0; i < 8; i++) {
-            const int32_t pi = (int32_t)(((i < 4 ? pred_lo : pred_hi) >> (8 * (i & 3))) & 0xFFu);
-            const int32_t v = min(255, max(0, out[i] + pi));
-            if (i < 4)
-                lo |= (uint32_t)v << (8 * i);
-            else
-                hi |= (uint32_t)v << (8 * (i - 4));
-        }
-        uint8_t *dst;
-        if (luma_pass)
-            dst = S.rec_y + (size_t)(mby * 16 + by8 + r) * S.pitch_y + mbx * 16 + bx8;
-        else
-            dst = ((b == 4) ? S.rec_cb : S.rec_cr) + (size_t)(mby * 8 + r) * S.pitch_c + mbx * 8;
-        if (H261B_CHECK(luma_pass ? (mby * 16 + by8 + r < S.mbh * 16 && mbx * 16 + bx8 + 8 <= S.mbw * 16)
-                                  : (mby * 8 + r < S.mbh * 8 && mbx * 8 + 8 <= S.mbw * 8),
-                        CHK_RECON, mby * 4096 + mbx))
-            *reinterpret_cast<uint2 *>(dst) = make_uint2(lo, hi);
+        *reinterpret_cast<uint2 *>(row.rec) = out;
         if (S.ssd_out) {
             /* squared error of this row against the source, for the
              * picture's PSNR (h261_main.c:38-91) */
-            const uint2 cw = luma_pass ? *reinterpret_cast<const uint2 *>(s.cur(by8 + r, bx8 >> 2))
-                                       : *reinterpret_cast<const uint2 *>(s.curc(8 * (b - 4) + r));
-            const uint2 rw = make_uint2(lo, hi);
-            uint32_t e = 0;
-#pragma unroll
-            for (int i = 0; i < 8; i++) {
-                const int d = byte8(cw, i) - byte8(rw, i);
-                e += (uint32_t)(d * d);
-            }
-            ssd = e;
+            const uint32_t d0 = __vabsdiffu4(row.cur.x, out.x), d1 = __vabsdiffu4(row.cur.y, out.y);
+            ssd = __dp4a(d0, d0, __dp4a(d1, d1, 0u));
         }
     }
     __syncwarp();
     return cbp;
+}
+
+/* the lane's row of the luma pass: block slot = lane / 8 */
+__device__ __forceinline__ BlockRow luma_row(const StageBuf s, const h261b_session_dev_t &S, int mbx, int mby,
+                                             const MbDecision &m, int lane)
+{
+    const int b = lane >> 3, r = lane & 7, bx8 = (b & 1) * 8, by8 = (b >> 1) * 8;
+    BlockRow o;
+    o.cur = *reinterpret_cast<const uint2 *>(s.cur(by8 + r, bx8 >> 2));
+    o.pred = make_uint2(0u, 0u);
+    if (m.type != H261B_MB_TYPE_INTRA) {
+        int wr = 15 + m.mvy + by8, wc = 16 + m.mvx + bx8;
+        /* rows wr..wr+7 of the 46-row window, byte columns wc..wc+7 with
+         * win8's three words inside the 12-word row */
+        if (!H261B_CHECK(wr >= 0 && wr + 7 < WIN_ROWS && wc >= 0 && wc <= 40, CHK_MC_WINDOW, wr * 64 + wc)) {
+            wr = min(max(wr, 0), WIN_ROWS - 8);
+            wc = min(max(wc, 0), 40);
+        }
+        o.pred = win8(s, wr + r, wc);
+        if (m.flags & H261B_MB_FILTER)
+            o.pred = loop_filter(o.pred, lane);
+    }
+    o.rec = S.rec_y + (size_t)(mby * 16 + by8 + r) * S.pitch_y + mbx * 16 + bx8;
+    o.active = H261B_CHECK(mby * 16 + by8 + r < S.mbh * 16 && mbx * 16 + bx8 + 8 <= S.mbw * 16, CHK_RECON,
+                           mby * 4096 + mbx);
+    return o;
+}
+
+/* the lane's row of the chroma pass: lanes 0-7 Cb, 8-15 Cr; lanes 16-31
+ * repeat them and write nothing */
+__device__ __forceinline__ BlockRow chroma_row(const StageBuf s, const h261b_session_dev_t &S, int mbx, int mby,
+                                               const MbDecision &m, int lane)
+{
+    const int pl = (lane >> 3) & 1, r = lane & 7;
+    BlockRow o;
+    o.cur = *reinterpret_cast<const uint2 *>(s.curc(8 * pl + r));
+    o.pred = make_uint2(0u, 0u);
+    if (m.type != H261B_MB_TYPE_INTRA) {
+        int cmx = m.mvx / 2, cmy = m.mvy / 2; /* truncation toward zero */
+#ifdef H261B_DEBUG_CHECKS
+        /* rows inside the chroma plane; glob8's words (12 bytes from the
+         * word boundary when unaligned) inside the row */
+        {
+            const int cx = mbx * 8 + cmx, cy = mby * 8 + cmy, wc8 = S.mbw * 8;
+            if (!H261B_CHECK(cy >= 0 && cy + 8 <= S.mbh * 8 && cx >= 0 &&
+                                 (cx & ~3) + ((cx & 3) ? 12 : 8) <= wc8,
+                             CHK_MC_CHROMA, cy * 4096 + cx))
+                cmx = cmy = 0;
+        }
+#endif
+        o.pred = glob8((pl ? S.ref_cr : S.ref_cb) + (size_t)(mby * 8 + cmy + r) * S.pitch_c + (mbx * 8 + cmx));
+        if (m.flags & H261B_MB_FILTER)
+            o.pred = loop_filter(o.pred, lane);
+    }
+    o.rec = (pl ? S.rec_cr : S.rec_cb) + (size_t)(mby * 8 + r) * S.pitch_c + mbx * 8;
+    o.active = lane < 16 && H261B_CHECK(mby * 8 + r < S.mbh * 8 && mbx * 8 + 8 <= S.mbw * 8, CHK_RECON,
+                                        mby * 4096 + mbx);
+    return o;
 }
 
 /* frame-end denoise update by the session's last warp (mbgpu_kernels.cuh:478-503) */
@@ -1176,17 +1174,21 @@ __device__ __forceinline__ void denoise_frame_end(h261b_denoise_dev_t *dn, int l
         atomicExch(&dn->ticket, 0u);
 }
 
-/* publish a warp's statistics for a run of n MBs of one session and type;
- * the publication that completes the session's frame updates the offsets */
-__device__ __forceinline__ void publish_run(const h261b_session_dev_t &S, int t, int n, const int32_t colsum[8],
-                                            int lane)
+/* publish a warp's statistics for a run of n MBs of one session and type,
+ * and clear them; the publication that completes the session's frame updates
+ * the offsets.  noise[v] holds the lane's own blocks' sum for coefficient
+ * (v, lane & 7). */
+__device__ __forceinline__ void publish_run(const h261b_session_dev_t &S, int t, int n, float noise[8], int lane)
 {
     h261b_denoise_dev_t *dn = S.dn;
-    if (lane < 8) {
 #pragma unroll
-        for (int v = 0; v < 8; v++)
-            if (colsum[v])
-                atomicAdd(&dn->noise[t][v * 8 + lane], colsum[v]);
+    for (int v = 0; v < 8; v++) {
+        int32_t x = (int32_t)noise[v];
+        noise[v] = 0.0f;
+        x += __shfl_xor_sync(FULL, x, 8);
+        x += __shfl_xor_sync(FULL, x, 16);
+        if (lane < 8 && x)
+            atomicAdd(&dn->noise[t][v * 8 + lane], x);
     }
     if (lane == 0)
         atomicAdd(&dn->count[t], 6 * n);
@@ -1254,7 +1256,10 @@ __global__ void __launch_bounds__(256, KIND == KIND_SEARCH ? H261B_SEARCH_MIN_BL
     const size_t warp_bytes = KIND == KIND_SEARCH ? kSearchWarpBytes : sizeof(WarpSmem);
     unsigned char *mine = smem_raw + warp * warp_bytes;
     uint32_t *wbuf = reinterpret_cast<uint32_t *>(mine);
-    float(*tb)[72] = reinterpret_cast<WarpSmem *>(mine)->t;   /* not used by KIND_SEARCH */
+    float(*tb)[TB_BLOCK] = reinterpret_cast<WarpSmem *>(mine)->t;   /* not used by KIND_SEARCH */
+    /* this lane's column factors: forward post-scale (times 0.125, exact)
+     * and inverse pre-scale */
+    const float fwd_c = __fmul_rn(c_fwd_post[lane & 7], 0.125f), inv_c = c_inv_pre[lane & 7];
     /* bulk staging: the two buffers' barriers; per buffer, the parity of
      * its next phase, whether its current staging used the barrier, and
      * whether a wait on it gave up.  A barrier whose wait gave up is not
@@ -1333,10 +1338,10 @@ __global__ void __launch_bounds__(256, KIND == KIND_SEARCH ? H261B_SEARCH_MIN_BL
     uint32_t nitem = gn < n_work ? work[gn] : 0u;
 
     int run_s = -1, run_t = 0, run_n = 0;
-    int32_t colsum[8];
+    float noise[8];
 #pragma unroll
     for (int v = 0; v < 8; v++)
-        colsum[v] = 0;
+        noise[v] = 0.0f;
 
     for (int cur = 0; g < n_work; cur ^= 1) {
         const int gnn = gn < n_work ? next_item() : n_work;
@@ -1425,12 +1430,10 @@ __global__ void __launch_bounds__(256, KIND == KIND_SEARCH ? H261B_SEARCH_MIN_BL
          * picture QUANT is known */
         if (want_enc && !(S.rc && (phases & H261B_PHASE_MD))) {
             const int t = m.type == H261B_MB_TYPE_INTRA ? 0 : 1;
-            if (run_n > 0 && (sidx != run_s || t != run_t)) {
-                publish_run(sessions[run_s], run_t, run_n, colsum, lane);
+            /* (the noise sums are exact below 2^24: 4,000 MBs of 2,041) */
+            if (run_n > 0 && (sidx != run_s || t != run_t || run_n >= 2048)) {
+                publish_run(sessions[run_s], run_t, run_n, noise, lane);
                 run_n = 0;
-#pragma unroll
-                for (int v = 0; v < 8; v++)
-                    colsum[v] = 0;
             }
             run_s = sidx;
             run_t = t;
@@ -1442,10 +1445,15 @@ __global__ void __launch_bounds__(256, KIND == KIND_SEARCH ? H261B_SEARCH_MIN_BL
              * code run twice (two inlined copies miss the instruction cache
              * more) */
             uint32_t ssd_l = 0, ssd_c = 0, cbp = 0;
+            /* this column's eight denoise offsets, UInt16, one 16-byte load */
+            const uint4 offw = *reinterpret_cast<const uint4 *>(&S.dn->offset[t][lane & 7][0]);
 #pragma unroll 1
             for (int pass = 0; pass < 2; pass++) {
                 uint32_t e = 0;
-                cbp |= encdec_pass<FMAD, ABI>(tb, b, S, mb, mbx, mby, m, quant, pass == 0, lane, colsum, e);
+                const BlockRow row = pass == 0 ? luma_row(b, S, mbx, mby, m, lane)
+                                               : chroma_row(b, S, mbx, mby, m, lane);
+                cbp |= encdec_pass<FMAD, ABI>(tb, row, S, mb, m, quant, offw, pass == 0, lane, fwd_c, inv_c, noise,
+                                              e);
                 if (pass == 0)
                     ssd_l = e;
                 else
@@ -1498,7 +1506,7 @@ __global__ void __launch_bounds__(256, KIND == KIND_SEARCH ? H261B_SEARCH_MIN_BL
         nitem = nnitem;
     }
     if (want_enc && run_n > 0)
-        publish_run(sessions[run_s], run_t, run_n, colsum, lane);
+        publish_run(sessions[run_s], run_t, run_n, noise, lane);
     if (bars) {
         for (int k = 0; k < 2; k++) {
             /* the copies of a phase whose wait gave up may still be landing:
