@@ -192,16 +192,6 @@ __device__ __forceinline__ uint2 win8(const StageBuf s, int row, int col)
     return make_uint2(__funnelshift_r(a, b, sh), __funnelshift_r(b, c, sh));
 }
 
-/* eight bytes from global memory at any alignment; reads only the words
- * that hold one of those bytes */
-__device__ __forceinline__ uint2 glob8(const uint8_t *ptr)
-{
-    const uint32_t *p = reinterpret_cast<const uint32_t *>((uintptr_t)ptr & ~(uintptr_t)3);
-    const uint32_t sh = (uint32_t)((uintptr_t)ptr & 3) * 8u;
-    const uint32_t a = p[0], b = p[1], c = sh ? p[2] : 0u;
-    return make_uint2(__funnelshift_r(a, b, sh), __funnelshift_r(b, c, sh));
-}
-
 /* asynchronous global -> shared copies; a 16-byte window chunk outside the
  * picture is not read (src-size 0) and its bytes are zero-filled.  Window
  * chunks are cached in L1 too: neighbouring MBs of a warp share two thirds
@@ -764,6 +754,11 @@ __device__ __forceinline__ float idct_round(float v)
 
 /* ---------------------------------------------------------- per MB */
 
+/* mb / mbw for mb < 4096: half a step above the quotient's lower end, which
+ * is at least 0.5 / mbw away from an integer, where the approximate
+ * reciprocal is off by less than 2^-10 / mbw */
+__device__ __forceinline__ int mb_row(int mb, int mbw) { return (int)__fdividef((float)mb + 0.5f, (float)mbw); }
+
 struct MbDecision {
     int32_t type, flags, mvx, mvy, cost;
 };
@@ -1119,32 +1114,53 @@ __device__ __forceinline__ BlockRow luma_row(const StageBuf s, const h261b_sessi
     return o;
 }
 
+/* the words of the lane's chroma prediction row: loaded before the luma
+ * pass, so that their latency passes behind it */
+struct ChromaRef {
+    uint32_t a, b, c, sh;
+};
+
+__device__ __forceinline__ ChromaRef chroma_ref(const h261b_session_dev_t &S, int mbx, int mby, const MbDecision &m,
+                                                int lane)
+{
+    ChromaRef o = { 0u, 0u, 0u, 0u };
+    if (m.type == H261B_MB_TYPE_INTRA)
+        return o;
+    const int pl = (lane >> 3) & 1, r = lane & 7;
+    int cmx = m.mvx / 2, cmy = m.mvy / 2; /* truncation toward zero */
+#ifdef H261B_DEBUG_CHECKS
+    /* rows inside the chroma plane; the words (12 bytes from the word
+     * boundary when unaligned) inside the row */
+    {
+        const int cx = mbx * 8 + cmx, cy = mby * 8 + cmy, wc8 = S.mbw * 8;
+        if (!H261B_CHECK(cy >= 0 && cy + 8 <= S.mbh * 8 && cx >= 0 && (cx & ~3) + ((cx & 3) ? 12 : 8) <= wc8,
+                         CHK_MC_CHROMA, cy * 4096 + cx))
+            cmx = cmy = 0;
+    }
+#endif
+    const uint8_t *g = (pl ? S.ref_cr : S.ref_cb) + (size_t)(mby * 8 + cmy + r) * S.pitch_c + (mbx * 8 + cmx);
+    /* only the words that hold one of the row's bytes */
+    const uint32_t *p = reinterpret_cast<const uint32_t *>((uintptr_t)g & ~(uintptr_t)3);
+    o.sh = (uint32_t)((uintptr_t)g & 3) * 8u;
+    if (lane < 16) {
+        o.a = p[0];
+        o.b = p[1];
+        o.c = o.sh ? p[2] : 0u;
+    }
+    return o;
+}
+
 /* the lane's row of the chroma pass: lanes 0-7 Cb, 8-15 Cr; lanes 16-31
- * repeat them and write nothing */
+ * write nothing */
 __device__ __forceinline__ BlockRow chroma_row(const StageBuf s, const h261b_session_dev_t &S, int mbx, int mby,
-                                               const MbDecision &m, int lane)
+                                               const MbDecision &m, const ChromaRef &f, int lane)
 {
     const int pl = (lane >> 3) & 1, r = lane & 7;
     BlockRow o;
     o.cur = *reinterpret_cast<const uint2 *>(s.curc(8 * pl + r));
-    o.pred = make_uint2(0u, 0u);
-    if (m.type != H261B_MB_TYPE_INTRA) {
-        int cmx = m.mvx / 2, cmy = m.mvy / 2; /* truncation toward zero */
-#ifdef H261B_DEBUG_CHECKS
-        /* rows inside the chroma plane; glob8's words (12 bytes from the
-         * word boundary when unaligned) inside the row */
-        {
-            const int cx = mbx * 8 + cmx, cy = mby * 8 + cmy, wc8 = S.mbw * 8;
-            if (!H261B_CHECK(cy >= 0 && cy + 8 <= S.mbh * 8 && cx >= 0 &&
-                                 (cx & ~3) + ((cx & 3) ? 12 : 8) <= wc8,
-                             CHK_MC_CHROMA, cy * 4096 + cx))
-                cmx = cmy = 0;
-        }
-#endif
-        o.pred = glob8((pl ? S.ref_cr : S.ref_cb) + (size_t)(mby * 8 + cmy + r) * S.pitch_c + (mbx * 8 + cmx));
-        if (m.flags & H261B_MB_FILTER)
-            o.pred = loop_filter(o.pred, lane);
-    }
+    o.pred = make_uint2(__funnelshift_r(f.a, f.b, f.sh), __funnelshift_r(f.b, f.c, f.sh));
+    if (m.type != H261B_MB_TYPE_INTRA && (m.flags & H261B_MB_FILTER))
+        o.pred = loop_filter(o.pred, lane);
     o.rec = (pl ? S.rec_cr : S.rec_cb) + (size_t)(mby * 8 + r) * S.pitch_c + mbx * 8;
     o.active = lane < 16 && H261B_CHECK(mby * 8 + r < S.mbh * 8 && mbx * 8 + 8 <= S.mbw * 8, CHK_RECON,
                                         mby * 4096 + mbx);
@@ -1231,9 +1247,13 @@ __device__ __forceinline__ void publish_run(const h261b_session_dev_t &S, int t,
  * launch does per MB; FULL_SEARCH: the exhaustive search instead of the
  * reference's; ABI: the launch may write the reference-layout outputs
  * (h261_macroblock_t records, ME results, stage-1 vectors) that only the
- * gpu_device.h boundary asks for.  Each launch runs the instantiation for
- * its flags (h261b_launch_step), so no launch carries code it never runs. */
-template <int FMAD, int KIND, bool FULL_SEARCH, bool ABI>
+ * gpu_device.h boundary asks for; BULK: the search window comes by bulk row
+ * copies.  Each launch runs the instantiation for its flags
+ * (h261b_launch_step), so no launch carries code it never runs: instruction
+ * fetch is a seventh of the kernel's stalls, and leaving the bulk staging's
+ * code out of the cp.async kernel alone took its launch of 13,464
+ * macroblocks from 83.0 to 79.4 us. */
+template <int FMAD, int KIND, bool FULL_SEARCH, bool ABI, bool BULK>
 __global__ void __launch_bounds__(256, KIND == KIND_SEARCH ? H261B_SEARCH_MIN_BLOCKS : H261B_STEP_MIN_BLOCKS)
     step_kernel(const h261b_session_dev_t *__restrict__ sessions, const uint32_t *__restrict__ work, int32_t n_work,
                 int32_t chunk, int32_t phases_arg, int32_t *sched)
@@ -1266,7 +1286,7 @@ __global__ void __launch_bounds__(256, KIND == KIND_SEARCH ? H261B_SEARCH_MIN_BL
      * armed again (its phase may never complete): that buffer falls back to
      * cp.async staging, and at the end the warp waits once more, bounded,
      * for the copies of the phase that gave up. */
-    uint64_t *bars = (phases_arg & H261B_STAGE_BULK) ? reinterpret_cast<WarpSmem *>(mine)->bar : nullptr;
+    uint64_t *bars = BULK ? reinterpret_cast<WarpSmem *>(mine)->bar : nullptr;
     uint32_t parity = 0, bulk_used = 0, stuck = 0;
 #ifdef H261B_DEBUG_CHECKS
     /* checking build only: the warp's first bulk staging announces 16 bytes
@@ -1307,7 +1327,7 @@ __global__ void __launch_bounds__(256, KIND == KIND_SEARCH ? H261B_SEARCH_MIN_BL
      * prediction block covers (none for an intra MB) */
     auto stage_item = [&](int k, uint32_t it) {
         const h261b_session_dev_t &N = sessions[it >> 12];
-        const int nmb = (int)(it & 0xFFFu), nmby = nmb / N.mbw;
+        const int nmb = (int)(it & 0xFFFu), nmby = mb_row(nmb, N.mbw), nmbx = nmb - nmby * N.mbw;
         uint64_t *bar = (bars && !((stuck >> k) & 1u)) ? &bars[k] : nullptr;
         const uint32_t extra = bar ? short_first : 0u;
         if (bar) {
@@ -1321,9 +1341,9 @@ __global__ void __launch_bounds__(256, KIND == KIND_SEARCH ? H261B_SEARCH_MIN_BL
         if (KIND == KIND_ENCODE) {
             const h261_mb_mode_decision_t &d = N.md_in[nmb];
             const bool inter = d.i_mb_type != H261B_MB_TYPE_INTRA;
-            stage_mb(wbuf, k, N, nmb - nmby * N.mbw, nmby, lane, 15 + d.i_mv_y, inter ? 16 : 0, bar, extra);
+            stage_mb(wbuf, k, N, nmbx, nmby, lane, 15 + d.i_mv_y, inter ? 16 : 0, bar, extra);
         } else {
-            stage_mb(wbuf, k, N, nmb - nmby * N.mbw, nmby, lane, 0, WIN_ROWS, bar, extra);
+            stage_mb(wbuf, k, N, nmbx, nmby, lane, 0, WIN_ROWS, bar, extra);
         }
     };
 
@@ -1375,7 +1395,7 @@ __global__ void __launch_bounds__(256, KIND == KIND_SEARCH ? H261B_SEARCH_MIN_BL
             nitem = nnitem;
             continue;
         }
-        const int mby = mb / S.mbw, mbx = mb - mby * S.mbw;
+        const int mby = mb_row(mb, S.mbw), mbx = mb - mby * S.mbw;
         const StageBuf b = stage_view(wbuf, cur);
         const bool do_me = (phases & H261B_PHASE_ME) && !S.skip_search;
 
@@ -1441,24 +1461,19 @@ __global__ void __launch_bounds__(256, KIND == KIND_SEARCH ? H261B_SEARCH_MIN_BL
             if (S.md_in && !(phases & H261B_PHASE_MD))
                 quant += S.md_in[mb].i_quantiser_adjust;
             quant = min(31, max(1, quant)); /* gpu_device.cu:625-627 */
-            /* the luma pass, then the chroma pass: one copy of the pass's
-             * code run twice (two inlined copies miss the instruction cache
-             * more) */
+            /* the luma pass, then the chroma pass, each its own copy of the
+             * pass's code: straight code fetches ahead, and with the pass at
+             * half its former size two copies run faster than a loop (79.5
+             * -> 78.2 us for 13,464 macroblocks of mixed streams, 519 -> 504
+             * us for 1024 QCIF streams) */
             uint32_t ssd_l = 0, ssd_c = 0, cbp = 0;
             /* this column's eight denoise offsets, UInt16, one 16-byte load */
             const uint4 offw = *reinterpret_cast<const uint4 *>(&S.dn->offset[t][lane & 7][0]);
-#pragma unroll 1
-            for (int pass = 0; pass < 2; pass++) {
-                uint32_t e = 0;
-                const BlockRow row = pass == 0 ? luma_row(b, S, mbx, mby, m, lane)
-                                               : chroma_row(b, S, mbx, mby, m, lane);
-                cbp |= encdec_pass<FMAD, ABI>(tb, row, S, mb, m, quant, offw, pass == 0, lane, fwd_c, inv_c, noise,
-                                              e);
-                if (pass == 0)
-                    ssd_l = e;
-                else
-                    ssd_c = e;
-            }
+            const ChromaRef ref = chroma_ref(S, mbx, mby, m, lane);
+            cbp = encdec_pass<FMAD, ABI>(tb, luma_row(b, S, mbx, mby, m, lane), S, mb, m, quant, offw, true, lane,
+                                         fwd_c, inv_c, noise, ssd_l);
+            cbp |= encdec_pass<FMAD, ABI>(tb, chroma_row(b, S, mbx, mby, m, ref, lane), S, mb, m, quant, offw, false,
+                                          lane, fwd_c, inv_c, noise, ssd_c);
             if (S.ssd_out) {
                 const uint32_t ey = __reduce_add_sync(FULL, ssd_l);
                 const uint32_t ecb = __reduce_add_sync(FULL, lane < 8 ? ssd_c : 0u);
@@ -1585,23 +1600,30 @@ using StepFn = void (*)(const h261b_session_dev_t *, const uint32_t *, int32_t, 
 
 /* the instantiation of a launch's flags: the encode kind has no search and
  * writes no reference-layout output, the search kind no encode output */
-template <int FMAD>
-StepFn step_fn_of(int kind, int full, int abi)
+template <int FMAD, bool BULK>
+StepFn step_fn_of(int kind, int full)
 {
     if (kind == KIND_ENCODE)
-        return step_kernel<FMAD, KIND_ENCODE, false, false>;
+        return step_kernel<FMAD, KIND_ENCODE, false, false, BULK>;
     if (kind == KIND_SEARCH)
-        return full ? step_kernel<FMAD, KIND_SEARCH, true, false> : step_kernel<FMAD, KIND_SEARCH, false, false>;
-    if (abi)
-        return full ? step_kernel<FMAD, KIND_FUSED, true, true> : step_kernel<FMAD, KIND_FUSED, false, true>;
+        return full ? step_kernel<FMAD, KIND_SEARCH, true, false, BULK>
+                    : step_kernel<FMAD, KIND_SEARCH, false, false, BULK>;
     if (kind == KIND_FULL)
-        return full ? step_kernel<FMAD, KIND_FULL, true, false> : step_kernel<FMAD, KIND_FULL, false, false>;
-    return full ? step_kernel<FMAD, KIND_FUSED, true, false> : step_kernel<FMAD, KIND_FUSED, false, false>;
+        return full ? step_kernel<FMAD, KIND_FULL, true, false, BULK> : step_kernel<FMAD, KIND_FULL, false, false, BULK>;
+    return full ? step_kernel<FMAD, KIND_FUSED, true, false, BULK> : step_kernel<FMAD, KIND_FUSED, false, false, BULK>;
 }
 
-StepFn step_fn(int fmad, int kind, int full, int abi)
+template <int FMAD>
+StepFn step_fn_of(int kind, int full, int abi, int bulk)
 {
-    return fmad ? step_fn_of<1>(kind, full, abi) : step_fn_of<0>(kind, full, abi);
+    if (abi && kind != KIND_ENCODE && kind != KIND_SEARCH)
+        return full ? step_kernel<FMAD, KIND_FUSED, true, true, false> : step_kernel<FMAD, KIND_FUSED, false, true, false>;
+    return bulk ? step_fn_of<FMAD, true>(kind, full) : step_fn_of<FMAD, false>(kind, full);
+}
+
+StepFn step_fn(int fmad, int kind, int full, int abi, int bulk)
+{
+    return fmad ? step_fn_of<1>(kind, full, abi, bulk) : step_fn_of<0>(kind, full, abi, bulk);
 }
 
 } // namespace
@@ -1621,17 +1643,18 @@ extern "C" int h261b_launch_step(const h261b_session_dev_t *sessions_dev, const 
     if (kind == KIND_FUSED && (phases & all_phases) == all_phases)
         kind = KIND_FULL;
     const int full = (phases & H261B_LAUNCH_ME_FULL) ? 1 : 0, abi = (phases & H261B_ABI_OUT) ? 1 : 0;
+    const int bulk = (phases & H261B_STAGE_BULK) ? 1 : 0;
     const bool pdl = (phases & H261B_LAUNCH_PDL) != 0;
     const int tail_code = (phases >> H261B_TAIL_SHIFT) & 15;
     if (kind > KIND_FULL)
         return (int)cudaErrorInvalidValue;
-    const int ph = phases & (0xFF | H261B_STAGE_BULK | H261B_STAGE_SHORT);
+    const int ph = phases & (0xFF | H261B_STAGE_SHORT);
     const int threads = warps_per_cta * 32;
     const size_t warp_bytes = kind == KIND_SEARCH ? kSearchWarpBytes : sizeof(WarpSmem);
     const size_t smem = warp_bytes * (size_t)warps_per_cta;
-    const StepFn fn = step_fn(fmad, kind, full, abi);
+    const StepFn fn = step_fn(fmad, kind, full, abi, bulk);
     static std::mutex mu;
-    static int sms[64], resident[64][2][4][2][2][9];
+    static int sms[64], resident[64][2][4][2][2][2][9];
     int dev = 0;
     cudaError_t err = cudaGetDevice(&dev);
     if (err != cudaSuccess || dev < 0 || dev >= 64)
@@ -1645,13 +1668,13 @@ extern "C" int h261b_launch_step(const h261b_session_dev_t *sessions_dev, const 
             const int max_smem = (int)(sizeof(WarpSmem) * 8);
             for (int f = 0; f < 2; f++)
                 for (int k = 0; k < 4; k++)
-                    for (int x = 0; x < 4; x++)
-                        if ((err = cudaFuncSetAttribute(step_fn(f, k, x & 1, x >> 1),
+                    for (int x = 0; x < 8; x++)
+                        if ((err = cudaFuncSetAttribute(step_fn(f, k, x & 1, (x >> 1) & 1, x >> 2),
                                                         cudaFuncAttributeMaxDynamicSharedMemorySize, max_smem)) !=
                             cudaSuccess)
                             return (int)err;
         }
-        int &r = resident[dev][fmad][kind][full][abi][warps_per_cta];
+        int &r = resident[dev][fmad][kind][full][abi][bulk][warps_per_cta];
         if (!r) {
             err = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&r, fn, threads, smem);
             if (err != cudaSuccess)
