@@ -441,8 +441,9 @@ __global__ void __launch_bounds__(LAYOUT_THREADS) layout_kernel(const h261b_sess
  * that finishes a picture's last MB then copies it into the host arena */
 constexpr int PACK_DONE_MAX = 64;   /* pictures a CTA copies together at its end */
 
-/* a finished picture into the host arena by threads t0, t0 + nt, ..., and
- * its record (bytes, offset, status, QUANT) by thread t0 */
+/* a finished picture into the host arena by threads t0, t0 + nt, ..., with
+ * its MB records and squared errors where the step wants them on the host,
+ * and its picture record (bytes, offset, status, QUANT) by thread t0 */
 __device__ __forceinline__ void copy_picture(const h261b_session_dev_t &S, uint8_t *host_arena, int t0, int nt)
 {
     const int total = S.vlc_total[0];
@@ -450,16 +451,60 @@ __device__ __forceinline__ void copy_picture(const h261b_session_dev_t &S, uint8
     const int st = (total < 0 || words * 4 > S.bits_cap) ? H261B_BITS_OVERFLOW : S.vlc_total[1];
     const int off = st == 0 ? S.vlc_total[2] : -1;
     const int bytes = (total + 7) >> 3;
-    const int units = ((bytes + 15) & ~15) / 16;
-    if (t0 == 0)
+    if (t0 == 0) {
         *S.pic_out = h261b_pic_info_t{ st == 0 ? bytes : 0, off, st, S.rc ? S.rc->picture_quant : S.quant };
-    if (off < 0 || !host_arena)
-        return;
-    /* other SMs wrote the words: read them from L2 */
+        if (S.host_ssd)
+            for (int c = 0; c < 3; c++)
+                S.host_ssd[c] = __ldcg(S.ssd_out + c);
+    }
+    /* other SMs wrote the words and records: read them from L2 */
+    const int units = off < 0 || !host_arena ? 0 : ((bytes + 15) & ~15) / 16;
     const uint4 *s4 = reinterpret_cast<const uint4 *>(S.bits_out);
     uint4 *d4 = reinterpret_cast<uint4 *>(host_arena + off);
     for (int i = t0; i < units; i += nt)
         d4[i] = __ldcg(s4 + i);
+    if (S.host_info) {
+        const uint4 *r4 = reinterpret_cast<const uint4 *>(S.info_out);
+        uint4 *h4 = reinterpret_cast<uint4 *>(S.host_info);
+        const int nmb = S.mbw * S.mbh;
+        for (int i = t0; i < nmb; i += nt)
+            h4[i] = __ldcg(r4 + i);
+    }
+}
+
+/* ---- fetch: a small step's uploads, read from pinned host memory.  Each
+ * 16-byte load waits about a microsecond for the bus, so a thread keeps four
+ * in flight and the grid is wide enough for one or two rounds.  A live QCIF
+ * step (40 KB up, 1.6 KB of records down by the pack kernel) went from 77 to
+ * 55 us on the device with this, the records and fewer event nodes. */
+constexpr int FETCH_THREADS = 256, FETCH_LOADS = 4;
+
+__global__ void __launch_bounds__(FETCH_THREADS) fetch_kernel(uint4 *dst0, const uint4 *src0, int n0, uint4 *dst1,
+                                                              const uint4 *src1, int n1, uint4 *zero, int nz)
+{
+    const int stride = gridDim.x * FETCH_THREADS;
+    for (int i = blockIdx.x * FETCH_THREADS + threadIdx.x; i < n0 + n1 + nz; i += FETCH_LOADS * stride) {
+        uint4 v[FETCH_LOADS];
+#pragma unroll
+        for (int k = 0; k < FETCH_LOADS; k++) {
+            const int j = i + k * stride;
+            v[k] = make_uint4(0u, 0u, 0u, 0u);
+            if (j < n0)
+                v[k] = src0[j];
+            else if (j < n0 + n1)
+                v[k] = src1[j - n0];
+        }
+#pragma unroll
+        for (int k = 0; k < FETCH_LOADS; k++) {
+            const int j = i + k * stride;
+            if (j < n0)
+                dst0[j] = v[k];
+            else if (j < n0 + n1)
+                dst1[j - n0] = v[k];
+            else if (j < n0 + n1 + nz)
+                zero[j - n0 - n1] = v[k];
+        }
+    }
 }
 
 __global__ void __launch_bounds__(VLC_THREADS) pack_kernel(const h261b_session_dev_t *sessions,
@@ -621,6 +666,20 @@ extern "C" h261b_bits_layout_t h261b_bits_layout(int32_t w, int32_t h)
     l.total = l.plan + al(nmb * 4);
     l.bytes = l.total + 256;
     return l;
+}
+
+extern "C" int h261b_launch_fetch(void *dst0, const void *src0, int64_t bytes0, void *dst1, const void *src1,
+                                  int64_t bytes1, void *zero, int64_t zero_bytes, int32_t sm_count, void *stream)
+{
+    const int64_t n = (bytes0 + bytes1 + zero_bytes) / 16;
+    if (n <= 0)
+        return 0;
+    const int ctas = (int)std::min<int64_t>((n + FETCH_THREADS - 1) / FETCH_THREADS, sm_count);
+    fetch_kernel<<<ctas, FETCH_THREADS, 0, (cudaStream_t)stream>>>((uint4 *)dst0, (const uint4 *)src0,
+                                                                   (int)(bytes0 / 16), (uint4 *)dst1,
+                                                                   (const uint4 *)src1, (int)(bytes1 / 16),
+                                                                   (uint4 *)zero, (int)(zero_bytes / 16));
+    return (int)cudaGetLastError();
 }
 
 extern "C" int64_t h261b_bits_slot_bytes(int32_t w, int32_t h) { return h261b_bits_layout(w, h).bytes; }

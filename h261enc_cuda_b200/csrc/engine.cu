@@ -330,16 +330,15 @@ struct h261b_engine_s {
     bool upload_checked = false;
     int64_t next_step = 0;     /* id of the next step; slot = id % NSLOT    */
     int64_t done_step = -1;    /* every step up to this one has completed   */
-    cudaEvent_t h2d_done[NSLOT] = {};
-    cudaEvent_t kernel_done[NSLOT] = {};
-    cudaEvent_t step_done[NSLOT] = {};
-    cudaEvent_t k_start[NSLOT] = {}, k_end[NSLOT] = {};
+    /* a step's timeline, one event a boundary, which the host and the other
+     * streams also wait on (each event is a node of the step's graph, about a
+     * microsecond of its chain): begin, uploads done, kernels may start (the
+     * previous step's encode is done), the encode kernel's end, results on
+     * the host */
+    cudaEvent_t t_begin[NSLOT] = {}, t_h2d[NSLOT] = {};
+    cudaEvent_t k_start[NSLOT] = {}, k_end[NSLOT] = {}, t_end[NSLOT] = {};
     cudaEvent_t b_end[NSLOT] = {};         /* after the bitstream kernel */
     cudaEvent_t layout_done[NSLOT] = {};   /* rate control inputs written */
-    /* timing of each phase of a step: begin, uploads done, kernels may
-     * start (the previous step's encode is done), results downloaded */
-    cudaEvent_t t_begin[NSLOT] = {}, t_h2d[NSLOT] = {};
-    cudaEvent_t t_ready[NSLOT] = {}, t_end[NSLOT] = {};
     /* step arena bytes asked for by h261b_engine_reserve_step */
     size_t reserved_upload = 0, reserved_results = 0, reserved_desc = 0;
     /* the encode launches' work counters, two per stream (h261b_launch_step) */
@@ -587,13 +586,10 @@ extern "C" int h261b_engine_create(const h261b_engine_config_t *cfg, h261b_engin
              cudaStreamCreateWithFlags(&e->side[p], cudaStreamNonBlocking) == cudaSuccess &&
              cudaEventCreateWithFlags(&e->fork_ev[p], cudaEventDisableTiming) == cudaSuccess &&
              cudaEventCreateWithFlags(&e->join_ev[p], cudaEventDisableTiming) == cudaSuccess &&
-             cudaEventCreateWithFlags(&e->h2d_done[p], cudaEventDisableTiming) == cudaSuccess &&
-             cudaEventCreateWithFlags(&e->kernel_done[p], cudaEventDisableTiming) == cudaSuccess &&
-             cudaEventCreateWithFlags(&e->step_done[p], cudaEventDisableTiming) == cudaSuccess &&
              cudaEventCreate(&e->k_start[p]) == cudaSuccess && cudaEventCreate(&e->k_end[p]) == cudaSuccess &&
              cudaEventCreate(&e->b_end[p]) == cudaSuccess && cudaEventCreate(&e->t_begin[p]) == cudaSuccess &&
              cudaEventCreateWithFlags(&e->layout_done[p], cudaEventDisableTiming) == cudaSuccess &&
-             cudaEventCreate(&e->t_h2d[p]) == cudaSuccess && cudaEventCreate(&e->t_ready[p]) == cudaSuccess &&
+             cudaEventCreate(&e->t_h2d[p]) == cudaSuccess &&
              cudaEventCreate(&e->t_end[p]) == cudaSuccess;
     }
     ok = ok && cudaMalloc(&e->sched_dev, 2 * NSLOT * sizeof(int32_t)) == cudaSuccess &&
@@ -678,16 +674,12 @@ extern "C" int h261b_engine_destroy(h261b_engine_t *e)
         e->results[p].release();
         e->desc[p].release();
         e->bits[p].release();
-        cudaEventDestroy(e->h2d_done[p]);
-        cudaEventDestroy(e->kernel_done[p]);
-        cudaEventDestroy(e->step_done[p]);
         cudaEventDestroy(e->k_start[p]);
         cudaEventDestroy(e->k_end[p]);
         cudaEventDestroy(e->b_end[p]);
         cudaEventDestroy(e->layout_done[p]);
         cudaEventDestroy(e->t_begin[p]);
         cudaEventDestroy(e->t_h2d[p]);
-        cudaEventDestroy(e->t_ready[p]);
         cudaEventDestroy(e->t_end[p]);
         if (e->stream[p])
             cudaStreamDestroy(e->stream[p]);
@@ -904,7 +896,7 @@ static int reserve_input(h261b_engine_t *e, Session *s, int32_t id, int32_t quan
         /* the copy that last read this pinned arena (NSLOT steps ago) must be
          * complete before the host writes into it */
         if (e->in_flight[p])
-            H261B_CUDA_TRY(cudaEventSynchronize(e->h2d_done[p]));
+            H261B_CUDA_TRY(cudaEventSynchronize(e->t_h2d[p]));
         e->upload_checked = true;
         e->upload_used = 0;
     }
@@ -963,7 +955,7 @@ extern "C" int h261b_engine_inputs(h261b_engine_t *e, int32_t n, const int32_t *
         const int p = (int)(e->next_step % NSLOT);
         if (!e->upload_checked) {
             if (e->in_flight[p])
-                H261B_CUDA_TRY(cudaEventSynchronize(e->h2d_done[p]));
+                H261B_CUDA_TRY(cudaEventSynchronize(e->t_h2d[p]));
             e->upload_checked = true;
             e->upload_used = 0;
         }
@@ -1203,7 +1195,7 @@ extern "C" int h261b_engine_step(h261b_engine_t *e)
                                     256) +
                            levels + align_up((size_t)mbs * sizeof(h261_mb_mode_decision_t), 256);
         const size_t desc = sizeof(h261b_step_dev_t) + align_up(n_list * sizeof(h261b_session_dev_t), 256) +
-                            (size_t)mbs * sizeof(uint32_t);
+                            align_up((size_t)mbs * sizeof(uint32_t), 16);
         int rc = grow_arenas(e, p, 0, 0, res, desc);
         if (rc)
             return rc;
@@ -1211,7 +1203,7 @@ extern "C" int h261b_engine_step(h261b_engine_t *e)
     int rc;
     /* arenas of this slot were last used by step id - NSLOT */
     if (e->in_flight[p] && id - NSLOT > e->done_step) {
-        H261B_CUDA_TRY(cudaEventSynchronize(e->step_done[p]));
+        H261B_CUDA_TRY(cudaEventSynchronize(e->t_end[p]));
         e->done_step = id - NSLOT;
         reclaim(e);
     }
@@ -1338,7 +1330,7 @@ extern "C" int h261b_engine_step(h261b_engine_t *e)
         }
     }
     cudaStream_t st = e->stream[p];
-    const size_t desc_bytes = work_off + (size_t)n_work * sizeof(uint32_t);
+    const size_t desc_bytes = align_up(work_off + (size_t)n_work * sizeof(uint32_t), 16);
     e->copier->join();   /* pictures of h261b_engine_submit_batch_async */
     LaunchPlan plan;
     const int tuning = next_plan(e, 2 * inter_mbs >= total_mb, &plan);
@@ -1362,6 +1354,25 @@ extern "C" int h261b_engine_step(h261b_engine_t *e)
     const size_t d2h = e->cfg.levels_to_host ? res_off : levels_base;
     if (n_bits && (rc = e->bits[p].reserve(e->bits_want)))
         return rc;
+    /* When every picture of the step is written as a bitstream and no levels
+     * are wanted, the pack kernel stores each picture's records straight into
+     * the host's results (pinned, so the device can address them) beside its
+     * bytes, and no copy follows it: a copy of 1.6 KB behind the kernels took
+     * about 10 us. */
+    const bool direct = n_bits == (int32_t)n && !e->cfg.levels_to_host;
+    if (direct)
+        for (size_t k = 0; k < n; k++) {
+            const Result &r = e->sessions[(size_t)list[k]].res[p];
+            desc[k].pic_out = (h261b_pic_info_t *)(rm.host + r.pic_off);
+            desc[k].host_info = (h261b_mb_info_t *)(rm.host + r.info_off);
+            desc[k].host_ssd = r.has_ssd ? (unsigned long long *)(rm.host + r.ssd_off) : nullptr;
+        }
+    /* A small step's descriptors and pictures come up by a kernel that reads
+     * them from the pinned arenas: the two copies it replaces take 13 us on
+     * the copy engine, however few bytes they move (12 -> 4 us for the
+     * descriptors of 64 streams).  Larger uploads stay with the copy engine,
+     * which runs beside the previous step's kernels. */
+    const bool fetch = desc_bytes + upload_bytes <= H261B_FETCH_MAX;
 
     /* the step's device work: uploads, encode (and rate control), the
      * bitstream kernels, the download, and the events the host and the
@@ -1371,17 +1382,25 @@ extern "C" int h261b_engine_step(h261b_engine_t *e)
         const unsigned rf = capturing ? cudaEventRecordExternal : cudaEventRecordDefault;
         const unsigned wf = capturing ? cudaEventWaitExternal : cudaEventWaitDefault;
         H261B_CUDA_TRY(cudaEventRecordWithFlags(e->t_begin[p], st, rf));
-        if (n_ssd)
-            H261B_CUDA_TRY(cudaMemsetAsync(rm.dev + ssd_base, 0, n * 32, st));
-        H261B_CUDA_TRY(cudaMemcpyAsync(dm.dev, dm.host, desc_bytes, cudaMemcpyHostToDevice, st));
-        if (upload_bytes)
-            H261B_CUDA_TRY(cudaMemcpyAsync(um.dev, um.host, upload_bytes, cudaMemcpyHostToDevice, st));
-        H261B_CUDA_TRY(cudaEventRecordWithFlags(e->h2d_done[p], st, rf));
+        if (fetch) {
+            const int fr = h261b_launch_fetch(dm.dev, dm.host, (int64_t)desc_bytes, um.dev, um.host,
+                                              (int64_t)upload_bytes, rm.dev + ssd_base, n_ssd ? (int64_t)n * 32 : 0,
+                                              e->sm_count, st);
+            if (fr != 0) {
+                set_error("upload launch failed: %s", cudaGetErrorString((cudaError_t)fr));
+                return H261B_ERR_CUDA;
+            }
+        } else {
+            if (n_ssd)
+                H261B_CUDA_TRY(cudaMemsetAsync(rm.dev + ssd_base, 0, n * 32, st));
+            H261B_CUDA_TRY(cudaMemcpyAsync(dm.dev, dm.host, desc_bytes, cudaMemcpyHostToDevice, st));
+            if (upload_bytes)
+                H261B_CUDA_TRY(cudaMemcpyAsync(um.dev, um.host, upload_bytes, cudaMemcpyHostToDevice, st));
+        }
         H261B_CUDA_TRY(cudaEventRecordWithFlags(e->t_h2d[p], st, rf));
         /* the previous step's reconstructions are this step's references */
         if (id > 0)
-            H261B_CUDA_TRY(cudaStreamWaitEvent(st, e->kernel_done[prev], wf));
-        H261B_CUDA_TRY(cudaEventRecordWithFlags(e->t_ready[p], st, rf));
+            H261B_CUDA_TRY(cudaStreamWaitEvent(st, e->k_end[prev], wf));
         H261B_CUDA_TRY(cudaEventRecordWithFlags(e->k_start[p], st, rf));
         int32_t *sched = e->sched_dev + 2 * p;
         /* fused: one launch encodes the fixed-QUANT sessions and searches
@@ -1418,7 +1437,6 @@ extern "C" int h261b_engine_step(h261b_engine_t *e)
         H261B_CUDA_TRY(cudaEventRecord(e->fork_ev[p], st));
         H261B_CUDA_TRY(cudaStreamWaitEvent(e->side[p], e->fork_ev[p], 0));
         H261B_CUDA_TRY(cudaEventRecordWithFlags(e->k_end[p], e->side[p], rf));
-        H261B_CUDA_TRY(cudaEventRecordWithFlags(e->kernel_done[p], e->side[p], rf));
         H261B_CUDA_TRY(cudaEventRecord(e->join_ev[p], e->side[p]));
         if (n_bits) {
             lr = h261b_launch_bitstream(desc_dev, (int32_t)n, work_dev, n_work, (h261b_step_dev_t *)dm.dev,
@@ -1430,13 +1448,13 @@ extern "C" int h261b_engine_step(h261b_engine_t *e)
             }
             H261B_CUDA_TRY(cudaEventRecordWithFlags(e->b_end[p], st, rf));
         }
-        /* the records download waits for the encode kernel's end: the
-         * bitstream kernels may finish first (the codes kernel waits only
-         * for the pictures that write a bitstream) */
+        /* the step's end, and a records download, wait for the encode
+         * kernel's end: the bitstream kernels may finish first (the codes
+         * kernel waits only for the pictures that write a bitstream) */
         H261B_CUDA_TRY(cudaStreamWaitEvent(st, e->join_ev[p], 0));
-        H261B_CUDA_TRY(cudaMemcpyAsync(rm.host, rm.dev, d2h, cudaMemcpyDeviceToHost, st));
+        if (!direct)
+            H261B_CUDA_TRY(cudaMemcpyAsync(rm.host, rm.dev, d2h, cudaMemcpyDeviceToHost, st));
         H261B_CUDA_TRY(cudaEventRecordWithFlags(e->t_end[p], st, rf));
-        H261B_CUDA_TRY(cudaEventRecordWithFlags(e->step_done[p], st, rf));
         return H261B_OK;
     };
 
@@ -1448,7 +1466,7 @@ extern "C" int h261b_engine_step(h261b_engine_t *e)
      * with use_graphs = 0 launch directly. */
     const StepKey key = { dm.host, dm.dev, um.host, um.dev, rm.host, rm.dev, bits_dev_or_null(e, p, n_bits),
                           n_bits ? e->bits[p].cap : 0, desc_off, work_off, desc_bytes, upload_bytes, ssd_base,
-                          d2h, (int64_t)n, n_work, rc_begin, n_rc, n_ssd ? 1 : 0, warps, ctas, phases,
+                          d2h, (int64_t)n, n_work, rc_begin, n_rc, (n_ssd ? 1 : 0) | (direct ? 2 : 0), warps, ctas, phases,
                           (int32_t)std::min<int64_t>(id, NSLOT - 1) };
     StepGraph &gr = e->graph[p];
     const bool repeated = gr.has_last_direct && gr.last_direct == key;
@@ -1529,7 +1547,7 @@ static int wait_step(h261b_engine_t *e, int64_t id)
         return H261B_OK;
     NvtxRange range("h261b wait step %lld", (long long)id);
     for (int64_t k = std::max(e->done_step + 1, id - NSLOT + 1); k <= id; k++)
-        H261B_CUDA_TRY(cudaEventSynchronize(e->step_done[k % NSLOT]));
+        H261B_CUDA_TRY(cudaEventSynchronize(e->t_end[k % NSLOT]));
     e->done_step = id;
     reclaim(e);
     return H261B_OK;
@@ -1747,7 +1765,7 @@ extern "C" int h261b_engine_step_timing(h261b_engine_t *e, h261b_step_timing_t *
     const int p = (int)(e->done_step % NSLOT);
     float a = 0, b = 0, c = 0, d = 0, f = 0;
     H261B_CUDA_TRY(cudaEventElapsedTime(&a, e->t_begin[p], e->t_h2d[p]));
-    H261B_CUDA_TRY(cudaEventElapsedTime(&b, e->t_h2d[p], e->t_ready[p]));
+    H261B_CUDA_TRY(cudaEventElapsedTime(&b, e->t_h2d[p], e->k_start[p]));
     H261B_CUDA_TRY(cudaEventElapsedTime(&c, e->k_start[p], e->k_end[p]));
     if (e->step_bits_ran[p])
         H261B_CUDA_TRY(cudaEventElapsedTime(&d, e->k_end[p], e->b_end[p]));

@@ -134,6 +134,10 @@ typedef struct {
      * picture as soon as its count is complete, while the encode launch
      * still works on other pictures */
     int32_t mbs_done;
+    /* where the pack kernel copies the picture's records and squared-error
+     * sums when it finishes the picture (pinned host memory), or NULL */
+    h261b_mb_info_t *host_info;
+    unsigned long long *host_ssd;
 } h261b_session_dev_t;
 
 /* coefficient bits of one MB at most: six blocks of an 8-bit DC or a first
@@ -185,6 +189,11 @@ int h261b_launch_step(const h261b_session_dev_t *sessions_dev, const uint32_t *w
                       int32_t n_work, int32_t phases, int32_t warps_per_cta, int32_t max_ctas,
                       int32_t *sched_dev, void *stream);
 int h261b_set_quant_table(void);
+/* copy two spans from pinned host memory into device memory and zero a third
+ * by a kernel (all 16-byte aligned, sizes in bytes, multiples of 16) */
+#define H261B_FETCH_MAX (256 * 1024)   /* bytes up to which a step uses it */
+int h261b_launch_fetch(void *dst0, const void *src0, int64_t bytes0, void *dst1, const void *src1, int64_t bytes1,
+                       void *zero, int64_t zero_bytes, int32_t sm_count, void *stream);
 /* the picture QUANT of every session with rc (one thread per session) */
 int h261b_launch_ratectrl(h261b_session_dev_t *sessions_dev, int32_t n_sessions, void *stream);
 
