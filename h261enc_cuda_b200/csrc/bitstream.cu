@@ -7,43 +7,38 @@
  * QCIF / CIF order, macroblocks with MBA, MTYPE, MQUANT, MVD, CBP, TCOEFF
  * and EOB, the last byte zero-padded (src/h261_bitstream.c:64-76).
  *
- * Three launches; the macroblock-parallel ones take contiguous ranges of the
- * step's work list, one warp per macroblock, so that every SM takes part
- * whatever the mix of picture sizes.  Kernel boundaries order layout and
- * pack; codes starts on a picture as soon as the encode launch has counted
- * all of its MBs done:
+ * Two or three launches; the macroblock-parallel ones go over the step's
+ * work list, so that every SM takes part whatever the mix of picture sizes:
  *
- *   codes   the macroblock's coded blocks, four at a time with eight lanes
- *           per block (lane j holds positions 8j..8j+7 of the transmission
- *           order): runs from the block's nonzero mask, TCOEFF / escape /
- *           DC / EOB codes, a scan for their offsets, assembled in shared
- *           memory and stored as the MB's coefficient bit string.
+ *   codes   (large steps; the encode kernel of a small step does it itself,
+ *           H261B_CODE_INLINE) a warp per macroblock: its coefficient bit
+ *           string (vlc_coder.h).
  *   layout  one CTA per picture, a warp per GOB with a lane per macroblock:
  *           the address increments, quantiser in force and vector
  *           predictors come from ballots over the GOB's coded / COEFF / MC
  *           flags; MB sizes, a scan over the GOB and one over the GOBs give
  *           every macroblock's position; the picture is cleared and gets its
  *           picture and GOB headers.
- *   pack    every coded macroblock (one per half-warp) writes its header and
- *           shifts its bit string into place; a macroblock's first and last
- *           word can be shared with its neighbours and are ORed in with
- *           atomics.  Half-warps count the MBs they finish per picture; the
- *           CTA whose count completes a picture copies it into the host
- *           arena (mapped pinned memory) at the offset layout drew with one
- *           atomic, and writes its record.
+ *   pack    every coded macroblock (one per half-warp, contiguous ranges)
+ *           writes its header and shifts its bit string into place; a
+ *           macroblock's first and last word can be shared with its
+ *           neighbours and are ORed in with atomics.  Half-warps count the
+ *           MBs they finish per picture; the CTA whose count completes a
+ *           picture copies it into the host arena (mapped pinned memory) at
+ *           the offset layout drew with one atomic, and writes its record.
  *
- * All three are programmatic dependent launches: the kernel before each
- * one (the encode kernel, codes, layout) lets it launch as soon as its own
- * CTAs are running, so each launch's latency overlaps the kernel before it.
- * Layout and pack wait (griddepcontrol.wait) for the whole previous grid
- * and its memory before they read what it wrote.  Codes instead waits per
- * picture, bounded, on the count the encode warps release after their
- * writes (session_dev_t.mbs_done), so that it codes the pictures finished
- * early while the encode launch's last MBs still run on other SMs; it
- * starts only once every encode CTA is running, and no encode CTA waits on
- * it.  The events that mark the
- * encode kernel's end are recorded on a side stream, so that nothing sits
- * between the encode kernel and codes in the stream.
+ * All are programmatic dependent launches: the kernel before each one lets
+ * it launch as soon as its own CTAs are running, so each launch's latency
+ * overlaps the kernel before it.  Pack, and layout after codes, wait
+ * (griddepcontrol.wait) for the whole previous grid and its memory before
+ * they read what it wrote.  The first kernel after the encode launch instead
+ * waits per picture, bounded, on the count the encode warps release after
+ * their writes (session_dev_t.mbs_done), so that it takes up the pictures
+ * finished early while the encode launch's last MBs still run on other SMs;
+ * it starts only once every encode CTA is running, and no encode CTA waits
+ * on it.  The events that mark the encode kernel's end are recorded on a
+ * side stream, so that nothing sits between the encode kernel and the first
+ * of these in the stream.
  */
 #include <cuda_runtime.h>
 #include <stddef.h>
@@ -67,6 +62,7 @@ __device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;"
 } // namespace
 #include "ratectrl_dev.h"
 #include "vlc_coder.h"
+#include "vlc_tables.h"
 
 namespace h261b {
 namespace {
@@ -78,12 +74,6 @@ constexpr int MB_WORDS = H261B_VLC_MB_WORDS;
 /* header bits of one macroblock at most: MBA 11, MTYPE 10, MQUANT 5,
  * MVD 2 x 11, CBP 9 */
 constexpr int MB_HDR_MAX = 57;
-
-struct CodesSmem {
-    alignas(16) int8_t blk[VLC_WARPS][4][64];   /* column-major levels of the blocks in flight */
-    alignas(16) uint32_t stage[VLC_WARPS][MB_WORDS];
-    uint16_t tc[27][16];
-};
 
 __device__ __forceinline__ uint32_t bswap(uint32_t x) { return __byte_perm(x, 0, 0x0123); }
 
@@ -190,18 +180,23 @@ __device__ __forceinline__ void warp_range(int32_t n_work, int &lo, int &hi)
 
 /* Waits (lane 0) until an encoding launch has finished every MB of a
  * picture: an acquire load of the count the encode warps add to after
- * fencing their levels and records.  The codes kernel is a programmatic
- * dependent of that launch, so it starts once every encode CTA is running,
+ * fencing their levels or strings and records.  The kernel that calls this is
+ * a programmatic dependent of that launch, so it starts once every encode CTA is running,
  * and no encode CTA waits on it: the count completes.  The wait is bounded
  * all the same (bound_ns of globaltimer, or 2^22 polls); false when it
  * gives up. */
+__device__ __forceinline__ bool picture_encoded(const int32_t *done, int32_t nmb)
+{
+    int32_t v;
+    asm volatile("ld.acquire.gpu.global.s32 %0, [%1];" : "=r"(v) : "l"(done) : "memory");
+    return v >= nmb;
+}
+
 __device__ __forceinline__ bool wait_picture_encoded(const int32_t *done, int32_t nmb, uint64_t bound_ns)
 {
     uint64_t t0 = 0;
     for (int it = 0; it < (1 << 22); it++) {
-        int32_t v;
-        asm volatile("ld.acquire.gpu.global.s32 %0, [%1];" : "=r"(v) : "l"(done) : "memory");
-        if (v >= nmb)
+        if (picture_encoded(done, nmb))
             return true;
         uint64_t t;
         asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(t));
@@ -214,11 +209,23 @@ __device__ __forceinline__ bool wait_picture_encoded(const int32_t *done, int32_
     return false;
 }
 
-/* work items a codes warp takes per draw: an intra MB codes six blocks, a
- * skipped inter MB none, so a static split leaves SMs idle at the end */
-constexpr int CODES_DRAW = 2;
+/* what a codes warp needs of one MB, loaded while it codes the one before */
+struct CodesItem {
+    int sidx, mb;          /* sidx < 0: none                                  */
+    bool ready;            /* its picture is encoded, the rest is loaded      */
+    uint2 rec;             /* type, flags, quant, cbp, vector                 */
+    uint32_t lev[3];       /* its levels' words lane, lane + 32, lane + 64    */
+};
 
-/* ---- codes: each macroblock's coefficient bit string */
+struct CodesSmem {
+    VlcScratch warp[VLC_WARPS];
+    VlcTables tables;
+};
+
+/* ---- codes: each macroblock's coefficient bit string.  A MB takes a chain of
+ * dependent loads (work item, descriptor, its picture's count, record and
+ * levels) of some 600 cycles each before it can be coded, so each warp draws
+ * and loads the next one before it codes the one at hand. */
 /* extra > 0 (the checking build's test of the bounded wait): wait for
  * that many MBs more than a picture has, for 2 ms at most */
 __global__ void __launch_bounds__(VLC_THREADS) codes_kernel(const h261b_session_dev_t *sessions,
@@ -228,92 +235,117 @@ __global__ void __launch_bounds__(VLC_THREADS) codes_kernel(const h261b_session_
     __shared__ CodesSmem sm;
     pdl_launch_dependents();
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-    load_tcoeff_table(sm.tc, tid, VLC_THREADS);
-    uint32_t zz0, zz1;
-    zigzag_lane(lane, zz0, zz1);
-    uint32_t *stage = sm.stage[warp];
+    load_vlc_tables(sm.tables, tid, VLC_THREADS);
+    VlcScratch &sc = sm.warp[warp];
     for (int i = lane; i < MB_WORDS; i += 32)
-        stage[i] = 0u;
-    /* no wait for the whole encode grid: each picture is coded once its
-     * MBs are (the encode launch's tail overlaps this kernel) */
+        sc.stage[i] = 0u;
     __syncthreads();
-
-    const int slot = lane >> 3, j = lane & 7;
-    /* the warp draws CODES_DRAW items at a time from the step's counter
-     * (zeroed by the step's descriptor upload) until the list is done */
-    int lo = 0, hi = 0;
-    int ready = -1;         /* the last session seen complete             */
-    bool failed = false;    /* a wait gave up: code nothing more          */
-    for (int w = 0;; w++) {
-        if (w >= hi) {
-            int d = 0;
-            if (lane == 0)
-                d = (int)atomicAdd(&step->codes_next, (uint32_t)CODES_DRAW);
-            lo = __shfl_sync(FULL, d, 0);
-            if (lo >= n_work)
-                break;
-            hi = min(lo + CODES_DRAW, n_work);
-            w = lo;
+    int ready = -1;         /* the last session seen complete                 */
+    bool failed = false;    /* a wait gave up: code nothing more              */
+    /* the record and levels of an item whose picture is encoded; `block`:
+     * wait for it */
+    auto load = [&](CodesItem &c, bool block) {
+        if (c.sidx < 0 || c.ready)
+            return;
+        const h261b_session_dev_t &S = sessions[c.sidx];
+        if (!S.bits_out) {
+            c.sidx = -1;
+            return;
         }
-        const uint32_t item = work[w];
-        const int sidx = (int)(item >> 12);
-        const h261b_session_dev_t &S = sessions[sidx];
-        if (!S.bits_out || failed)
-            continue;
-        if (sidx != ready) {
+        const uint2 *rp = reinterpret_cast<const uint2 *>(S.info_out + c.mb);
+        const uint32_t *lp = reinterpret_cast<const uint32_t *>(S.level_out + (size_t)c.mb * 384) + lane;
+        if (c.sidx != ready) {
             int ok = 0;
+            const int32_t nmb = S.mbw * S.mbh + extra;
             if (lane == 0)
-                ok = wait_picture_encoded(&S.mbs_done, S.mbw * S.mbh + extra,
-                                          extra ? 2000000ull : 200000000ull) ? 1 : 0;
+                ok = block ? wait_picture_encoded(&S.mbs_done, nmb, extra ? 2000000ull : 200000000ull)
+                           : picture_encoded(&S.mbs_done, nmb);
             __syncwarp();   /* orders lane 0's acquire before every lane's reads */
             if (!__shfl_sync(FULL, ok, 0)) {
-                if (lane == 0)
-                    atomicExch(&step->codes_failed, 1u);
-                failed = true;
-                continue;
+                if (block) {
+                    if (lane == 0)
+                        atomicExch(&step->codes_failed, 1u);
+                    failed = true;
+                    c.sidx = -1;
+                }
+                return;
             }
-            ready = sidx;
+            ready = c.sidx;
         }
-        const int mb = (int)(item & 4095u);
-        h261b_mb_info_t &rec = S.info_out[mb];
-        const int cbp = coded_blocks(rec);
-        const bool intra = rec.type == H261B_MB_TYPE_INTRA;
-        /* block b is coded when bit b of `order` is set */
-        const uint32_t order = __brev((uint32_t)cbp) >> 26;
-        const int nb = __popc(order);
-
-        int pos = 0, oob = 0;
-        const int8_t *lv = S.level_out + (size_t)mb * 384;
-        for (int r0 = 0; r0 < nb; r0 += 4) {
-            const bool here = r0 + slot < nb;
-            const int b = here ? (int)__fns(order, 0, r0 + slot + 1) : 0;
-            if (here)
-                *reinterpret_cast<uint2 *>(&sm.blk[warp][slot][j * 8]) =
-                    *reinterpret_cast<const uint2 *>(lv + b * 64 + j * 8);
-            __syncwarp();
-            pos += code_block_group(sm.blk[warp][slot], here, intra, zz0, zz1, sm.tc, stage, MB_WORDS, pos, lane,
-                                    oob);
-            __syncwarp();
+        c.ready = true;
+        c.rec = __ldcg(rp);
+#pragma unroll
+        for (int k = 0; k < 3; k++)
+            c.lev[k] = __ldcg(lp + 32 * k);
+    };
+    /* the first item is the warp's own, the others are drawn from the step's
+     * counter (zeroed by the step's descriptor upload): an intra MB codes six
+     * blocks, a skipped inter MB none */
+    const int total = (int)gridDim.x * VLC_WARPS;
+    int at = (int)blockIdx.x * VLC_WARPS + warp;
+    auto take = [&](int w) {
+        CodesItem c;
+        c.ready = false;
+        c.sidx = -1;
+        if (w < n_work) {
+            const uint32_t item = work[w];
+            c.sidx = (int)(item >> 12);
+            c.mb = (int)(item & 4095u);
         }
-        const int bits = store_mb_string(stage, S.vlc_scratch + (size_t)mb * MB_WORDS, pos, oob, lane);
+        return c;
+    };
+    CodesItem cur = take(at);
+    while (at < n_work) {
+        int next = 0;
         if (lane == 0)
-            rec.coef_bits = bits;
+            next = total + (int)atomicAdd(&step->codes_next, 1u);
+        load(cur, true);
+        if (failed)
+            break;
+        next = __shfl_sync(FULL, next, 0);
+        CodesItem after = take(next);
+        load(after, false);
+        if (cur.sidx >= 0) {
+            const h261b_session_dev_t &S = sessions[cur.sidx];
+            h261b_mb_info_t r;
+            memcpy(&r, &cur.rec, sizeof(cur.rec));
+            /* block b is coded when bit b is set */
+            const uint32_t blocks = __brev((uint32_t)coded_blocks(r)) >> 26;
+            int bits = 0;
+            if (blocks) {
+                int oob = 0;
+#pragma unroll
+                for (int k = 0; k < 3; k++)
+                    sc.cm[lane + 32 * k] = cur.lev[k];
+                __syncwarp();
+                const int pos = code_mb(blocks, r.type == H261B_MB_TYPE_INTRA, sm.tables, sc, lane, oob);
+                bits = store_mb_string(sc.stage, S.vlc_scratch + (size_t)cur.mb * MB_WORDS, pos, oob, lane);
+            }
+            if (lane == 0)
+                S.info_out[cur.mb].coef_bits = bits;
+        }
+        cur = after;
+        at = next;
     }
 }
 
 /* ---- layout: one CTA per picture, a warp per GOB (12 warps: all of a CIF
  * picture's GOBs at once); it also draws the picture's place in the host
- * arena, so that whichever CTA finishes the picture can copy it */
+ * arena, so that whichever CTA finishes the picture can copy it.
+ * extra > 0 (the checking build's test of the bounded wait): wait for that
+ * many MBs more than a picture has, for 2 ms at most */
 constexpr int LAYOUT_THREADS = 12 * 32;
 
 __global__ void __launch_bounds__(LAYOUT_THREADS) layout_kernel(const h261b_session_dev_t *sessions,
-                                                                h261b_step_dev_t *step, int64_t host_cap)
+                                                                h261b_step_dev_t *step, int64_t host_cap,
+                                                                int32_t after_codes, int32_t extra)
 {
     pdl_launch_dependents();
     const h261b_session_dev_t &S = sessions[blockIdx.x];
     if (!S.bits_out)
         return;
-    pdl_wait();   /* the codes kernel's MB sizes */
+    if (after_codes)
+        pdl_wait();   /* the codes kernel's MB sizes */
     __shared__ int32_t rel[396];       /* MB position within its GOB */
     __shared__ int32_t gob_bits[12];
     __shared__ int64_t gob_start[13];
@@ -323,8 +355,13 @@ __global__ void __launch_bounds__(LAYOUT_THREADS) layout_kernel(const h261b_sess
     const int ngob = cif ? 12 : 3, nmb = S.mbw * S.mbh;
     const int gq = S.rc ? S.rc->picture_quant : S.quant;
     const h261b_mb_info_t *info = S.info_out;
-    if (tid == 0)
+    /* right after the encode launch: the picture is laid out once its MBs
+     * are coded, and refused when the wait gives up.  The barrier orders
+     * thread 0's acquire before every thread's reads */
+    if (tid == 0 && after_codes)
         bad = step->codes_failed ? 1 : 0;   /* some picture's strings are missing */
+    else if (tid == 0)
+        bad = wait_picture_encoded(&S.mbs_done, nmb + extra, extra ? 2000000ull : 200000000ull) ? 0 : 1;
     __syncthreads();
 
     const int nwarps = blockDim.x >> 5;
@@ -729,8 +766,8 @@ static cudaError_t launch_dependent(void (*kernel)(Params...), dim3 grid, dim3 b
 
 extern "C" int h261b_launch_bitstream(h261b_session_dev_t *sessions_dev, int32_t n_sessions, const uint32_t *work_dev,
                                       int32_t n_work, h261b_step_dev_t *step, uint8_t *host_arena_dev,
-                                      int64_t host_cap, int32_t sm_count, void *stream, void *layout_done_event,
-                                      int32_t test_extra_wait)
+                                      int64_t host_cap, int32_t sm_count, int32_t coded, void *stream,
+                                      void *layout_done_event, int32_t test_extra_wait)
 {
     if (n_work <= 0 || n_sessions <= 0)
         return 0;
@@ -742,16 +779,18 @@ extern "C" int h261b_launch_bitstream(h261b_session_dev_t *sessions_dev, int32_t
     if (err != cudaSuccess)
         return (int)err;
     const int64_t want = (n_work + 2 * VLC_WARPS - 1) / (2 * VLC_WARPS);
-    const int codes_ctas = (int)std::min<int64_t>(want, (int64_t)sm_count * codes_res);
+    const int codes_ctas = (int)std::min<int64_t>((n_work + VLC_WARPS - 1) / VLC_WARPS, (int64_t)sm_count * codes_res);
     const int ctas = (int)std::min<int64_t>(want, (int64_t)sm_count * pack_res);
     cudaStream_t st = (cudaStream_t)stream;
-    err = launch_dependent(codes_kernel, dim3(codes_ctas), dim3(VLC_THREADS), st,
-                           (const h261b_session_dev_t *)sessions_dev, work_dev, n_work, step, test_extra_wait);
-    if (err != cudaSuccess)
-        return (int)err;
+    if (!coded) {
+        err = launch_dependent(codes_kernel, dim3(codes_ctas), dim3(VLC_THREADS), st,
+                               (const h261b_session_dev_t *)sessions_dev, work_dev, n_work, step, test_extra_wait);
+        if (err != cudaSuccess)
+            return (int)err;
+    }
     err = launch_dependent(layout_kernel, dim3(n_sessions), dim3(LAYOUT_THREADS), st,
-                                       (const h261b_session_dev_t *)sessions_dev, step,
-                                       (int64_t)(host_arena_dev ? host_cap : 0));
+                           (const h261b_session_dev_t *)sessions_dev, step, (int64_t)(host_arena_dev ? host_cap : 0),
+                           (int32_t)(coded ? 0 : 1), test_extra_wait);
     if (err != cudaSuccess)
         return (int)err;
     if (layout_done_event) {

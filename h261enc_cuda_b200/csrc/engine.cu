@@ -367,7 +367,7 @@ struct h261b_engine_s {
 
     /* phases-word bits the checking build adds for its tests (0 otherwise) */
     int32_t test_bits = 0;
-    int32_t test_codes_extra = 0;   /* checking build: the codes wait's test */
+    int32_t test_codes_extra = 0;   /* checking build: the test of the wait for a picture's MBs */
     /* the encode kernel's launch plan, and its tuning */
     LaunchPlan plan;
     Tuner tuner;
@@ -650,7 +650,7 @@ extern "C" int h261b_engine_create(const h261b_engine_config_t *cfg, h261b_engin
      * first bulk staging announces more bytes than it copies */
     if (getenv("H261B_TEST_STAGE_SHORT"))
         e->test_bits |= H261B_STAGE_SHORT;
-    /* and of the codes kernel's bounded wait for a picture's MBs */
+    /* and of the bounded wait for a picture's MBs after the encode launch */
     if (getenv("H261B_TEST_CODES_WAIT"))
         e->test_codes_extra = 1;
 #endif
@@ -1234,6 +1234,14 @@ extern "C" int h261b_engine_step(h261b_engine_t *e)
      * kernels; device only, after the levels) */
     const size_t md_base = levels_base + levels_total;
     size_t md_off = md_base;
+    /* Small steps, of at most a MB a resident warp, code each MB in the warp
+     * that encodes it: a kernel less in a chain of latencies.  In larger ones
+     * the coding's dependent shuffles and look-ups would hold up the warp's
+     * next MB, and a kernel with 2.5 times the warps hides them better.
+     * Device time of a step, inline against the codes kernel: one QCIF picture
+     * 49 / 52 us, ten pictures (1,881 MBs) 74 / 83, 6,336 MBs 118 / 114,
+     * 13,464 MBs 130 / 116, 101,376 MBs 830 / 689. */
+    const bool coded = total_mb <= (int64_t)e->sm_count * 16;
     int64_t inter_mbs = 0;
     int32_t n_work = 0, n_bits = 0, n_rc = 0, rc_begin = 0, n_ssd = 0;
     for (size_t k = 0; k < n; k++) {
@@ -1279,7 +1287,8 @@ extern "C" int h261b_engine_step(h261b_engine_t *e)
         d.info_out = (h261b_mb_info_t *)(rm.dev + info_off);
         info_off += (size_t)s.nmb * sizeof(h261b_mb_info_t);
         r.level_off = res_off;
-        d.level_out = (int8_t *)(rm.dev + res_off);
+        /* (a step that codes its MBs as they are encoded needs no levels) */
+        d.level_out = !coded || e->cfg.levels_to_host ? (int8_t *)(rm.dev + res_off) : nullptr;
         res_off += align_up((size_t)s.nmb * 384, 256);
         r.has_bits = s.bitstream;
         r.pic_off = pic_base + k * sizeof(h261b_pic_info_t);
@@ -1338,8 +1347,9 @@ extern "C" int h261b_engine_step(h261b_engine_t *e)
     /* the arithmetic and the search mode are the engine's, for every launch */
     const int fmad_bit =
         (e->cfg.fmad ? H261B_FMAD_BIT : 0) | (e->cfg.me_mode == H261B_ME_FULL ? H261B_LAUNCH_ME_FULL : 0);
+    const int code_bit = n_bits && coded ? H261B_CODE_INLINE : 0;
     const int phases = H261B_PHASE_ME | H261B_PHASE_MD | H261B_PHASE_ENCDEC | fmad_bit | plan.bits() |
-                       e->test_bits | (plan.split ? H261B_KIND_SEARCH : 0);
+                       e->test_bits | (plan.split ? H261B_KIND_SEARCH : 0) | code_bit;
     if (!plan.split)
         for (size_t k = 0; k < n; k++)
             if (!desc[k].rc)
@@ -1421,12 +1431,13 @@ extern "C" int h261b_engine_step(h261b_engine_t *e)
             /* the encode launch over every MB, right after the search launch
              * (a programmatic dependent launch) or after the rate control */
             lr = h261b_launch_step(desc_dev, work_dev, n_work,
-                                   H261B_PHASE_ENCDEC | fmad_bit | plan.bits() | e->test_bits | H261B_KIND_ENCODE |
+                                   H261B_PHASE_ENCDEC | fmad_bit | plan.bits() | e->test_bits | H261B_KIND_ENCODE | code_bit |
                                        (n_rc ? 0 : H261B_LAUNCH_PDL),
                                    warps, ctas, sched, st);
         } else if (lr == 0 && n_rc) {
             lr = h261b_launch_step(desc_dev, work_dev + rc_begin, n_work - rc_begin,
-                                   H261B_PHASE_ENCDEC | fmad_bit | plan.bits() | e->test_bits, warps, ctas, sched, st);
+                                   H261B_PHASE_ENCDEC | fmad_bit | plan.bits() | e->test_bits | code_bit, warps, ctas,
+                                   sched, st);
         }
         if (lr != 0) {
             set_error("step launch failed: %s", cudaGetErrorString((cudaError_t)lr));
@@ -1440,7 +1451,7 @@ extern "C" int h261b_engine_step(h261b_engine_t *e)
         H261B_CUDA_TRY(cudaEventRecord(e->join_ev[p], e->side[p]));
         if (n_bits) {
             lr = h261b_launch_bitstream(desc_dev, (int32_t)n, work_dev, n_work, (h261b_step_dev_t *)dm.dev,
-                                        e->bits[p].dev, (int64_t)e->bits[p].cap, e->sm_count, st,
+                                        e->bits[p].dev, (int64_t)e->bits[p].cap, e->sm_count, coded ? 1 : 0, st,
                                         n_rc ? (void *)e->layout_done[p] : nullptr, e->test_codes_extra);
             if (lr != 0) {
                 set_error("bitstream launch failed: %s", cudaGetErrorString((cudaError_t)lr));
@@ -1449,8 +1460,8 @@ extern "C" int h261b_engine_step(h261b_engine_t *e)
             H261B_CUDA_TRY(cudaEventRecordWithFlags(e->b_end[p], st, rf));
         }
         /* the step's end, and a records download, wait for the encode
-         * kernel's end: the bitstream kernels may finish first (the codes
-         * kernel waits only for the pictures that write a bitstream) */
+         * kernel's end: the bitstream kernels may finish first (the first of
+         * them waits only for the pictures that write a bitstream) */
         H261B_CUDA_TRY(cudaStreamWaitEvent(st, e->join_ev[p], 0));
         if (!direct)
             H261B_CUDA_TRY(cudaMemcpyAsync(rm.host, rm.dev, d2h, cudaMemcpyDeviceToHost, st));

@@ -79,7 +79,8 @@ typedef struct {
  * descriptor upload zeroes it every step) */
 typedef struct {
     uint32_t host_used;       /* bytes of the host arena handed out          */
-    uint32_t codes_next;      /* work items the codes kernel has handed out  */
+    uint32_t codes_next;      /* work items the codes kernel has handed out,
+                                 beyond the first of each warp               */
     uint32_t codes_failed;    /* nonzero: a codes warp gave up waiting for a
                                  picture's MBs (the layout refuses every
                                  picture of the step)                        */
@@ -130,8 +131,8 @@ typedef struct {
     unsigned long long *ssd_out;
     /* MBs of the picture an encoding launch has finished, zero before the
      * step: each warp adds a run's MBs after a fence, so that the codes
-     * kernel (a programmatic dependent of the encode launch) may code a
-     * picture as soon as its count is complete, while the encode launch
+     * or layout kernel (the programmatic dependent of the encode launch) may
+     * take up a picture as soon as its count is complete, while the encode launch
      * still works on other pictures */
     int32_t mbs_done;
     /* where the pack kernel copies the picture's records and squared-error
@@ -175,6 +176,9 @@ typedef struct {
 /*   bit 18       the exhaustive +-15 search (the sessions' me_mode 1)
  *   bit 19       the launch may write the reference-layout outputs
  *                (abi_out, me_out, stage1_out: the gpu_device.h boundary) */
+/*   bit 20       sessions with bits_out: each MB's coefficient bit string is
+ *                made by the warp that encodes it */
+#define H261B_CODE_INLINE   0x100000
 #define H261B_LAUNCH_ME_FULL 0x40000
 #define H261B_ABI_OUT       0x80000
 
@@ -197,17 +201,19 @@ int h261b_launch_fetch(void *dst0, const void *src0, int64_t bytes0, void *dst1,
 /* the picture QUANT of every session with rc (one thread per session) */
 int h261b_launch_ratectrl(h261b_session_dev_t *sessions_dev, int32_t n_sessions, void *stream);
 
-/* the bitstream of every work item's session that has bits_out: three
- * launches (coefficient codes and packing over the step's work list, the
- * layout per session; the CTA that packs a picture's last MBs copies it);
- * the picture ends in bits_out and in the host arena (device-mapped pinned
- * memory, host_cap bytes) at an offset drawn from step->host_used.
- * test_extra_wait > 0 (tests of the checking build only): the codes kernel
- * waits for that many MBs more than each picture has, for 2 ms, so that its
- * bounded wait runs out and the step's pictures are refused */
+/* the bitstream of every work item's session that has bits_out: the MBs'
+ * coefficient strings (unless `coded`: the encode launch left them,
+ * H261B_CODE_INLINE), the layout per session, and packing (the CTA that packs
+ * a picture's last MBs copies it); the picture ends in bits_out and in the
+ * host arena (device-mapped pinned memory, host_cap bytes) at an offset drawn
+ * from step->host_used.  test_extra_wait > 0 (tests of the checking build
+ * only): the first launch waits for that many MBs more than each picture has,
+ * for 2 ms, so that its bounded wait runs out and the step's pictures are
+ * refused */
 int h261b_launch_bitstream(h261b_session_dev_t *sessions_dev, int32_t n_sessions, const uint32_t *work_dev,
                            int32_t n_work, h261b_step_dev_t *step, uint8_t *host_arena_dev, int64_t host_cap,
-                           int32_t sm_count, void *stream, void *layout_done_event, int32_t test_extra_wait);
+                           int32_t sm_count, int32_t coded, void *stream, void *layout_done_event,
+                           int32_t test_extra_wait);
 /* device bytes per step slot a w x h session's bitstream needs: picture
  * bytes, MB scratch and offsets (0: no bitstream for this size), and where
  * each part starts in that block */

@@ -45,8 +45,12 @@
 #include <mutex>
 
 #include "h261b_device.h"
+#include "vlc_coder.h"
 
 namespace {
+
+using namespace h261b;
+
 
 constexpr int WIN_ROWS = 46;        /* rows mb_y-15 .. mb_y+30; columns mb_x-16 .. mb_x+31 */
 /* A warp's two buffers (this MB, next MB) share 46 rows of 36 words.
@@ -72,6 +76,7 @@ struct __align__(16) WarpSmem {
                                              row copies complete on (bulk
                                              staging only)                   */
     float t[4][TB_BLOCK];                 /* transpose buffer               */
+    VlcScratch vlc;                       /* the MB's levels and codes      */
 };
 
 /* one MB's staged inputs: buffer k of the warp's shared memory */
@@ -88,8 +93,12 @@ struct StageBuf {
 __device__ __forceinline__ StageBuf stage_view(const uint32_t *wbuf, int k) { return StageBuf{ wbuf + 16 * k }; }
 
 /* shared memory of one warp: both staging buffers, plus the transpose
- * buffer for kernels that encode (the search-only kernel has none) */
+ * buffer for kernels that encode (the search-only kernel has none), plus the
+ * coder's memory for those that also code; theirs ends with the coder's
+ * tables, one per CTA */
 constexpr size_t kSearchWarpBytes = sizeof(uint32_t) * WIN_ROWS * WIN_PITCH_W + 2 * sizeof(uint64_t);
+constexpr size_t kEncodeWarpBytes = offsetof(WarpSmem, vlc);
+static_assert(kEncodeWarpBytes % 16 == 0 && sizeof(WarpSmem) % 16 == 0, "warp shared layout");
 static_assert(kSearchWarpBytes % 16 == 0 && offsetof(WarpSmem, t) == kSearchWarpBytes, "warp shared layout");
 
 /* what a launch of the step kernel does per MB */
@@ -944,8 +953,8 @@ struct BlockRow {
  * inverse transform for a pass without a coded block: 98.9 -> 83.4 us for
  * the encode launch of 13,464 macroblocks of mixed streams, 716 -> 554 us for
  * 1024 QCIF streams, 43.9 -> 40.7 us for 16 intra CIF pictures. */
-template <int FMAD, bool ABI>
-__device__ __forceinline__ uint32_t encdec_pass(float (*tb)[TB_BLOCK], const BlockRow &row,
+template <int FMAD, bool ABI, bool CODE>
+__device__ __forceinline__ uint32_t encdec_pass(float (*tb)[TB_BLOCK], uint32_t *cm, const BlockRow &row,
                                                 const h261b_session_dev_t &S, int mb, const MbDecision &m, int quant,
                                                 uint4 offw, bool luma_pass, int lane, float fwd_c, float inv_c,
                                                 float noise[8], uint32_t &ssd)
@@ -1033,6 +1042,8 @@ __device__ __forceinline__ uint32_t encdec_pass(float (*tb)[TB_BLOCK], const Blo
         }
         if (S.level_out)
             *reinterpret_cast<uint2 *>(S.level_out + (size_t)mb * 384 + b * 64 + c * 8) = make_uint2(lo, hi);
+        if (CODE)
+            *reinterpret_cast<uint2 *>(cm + b * 16 + c * 2) = make_uint2(lo, hi);
     }
 
     /* ---- dequant (mbgpu_kernels.cuh:763-814) and IDCT pass 1 on column c;
@@ -1213,8 +1224,8 @@ __device__ __forceinline__ void publish_run(const h261b_session_dev_t &S, int t,
     uint32_t last = 0;
     if (lane == 0) {
         last = atomicAdd(&dn->ticket, (uint32_t)n) + (uint32_t)n == (uint32_t)(S.mbw * S.mbh) ? 1u : 0u;
-        /* the run's levels and records are written and fenced: count its
-         * MBs for the codes kernel */
+        /* the run's levels, strings and records are written and fenced: count
+         * its MBs for the kernel after this launch */
         atomicAdd(const_cast<int32_t *>(&S.mbs_done), n);
     }
     last = __shfl_sync(FULL, last, 0);
@@ -1248,12 +1259,12 @@ __device__ __forceinline__ void publish_run(const h261b_session_dev_t &S, int t,
  * reference's; ABI: the launch may write the reference-layout outputs
  * (h261_macroblock_t records, ME results, stage-1 vectors) that only the
  * gpu_device.h boundary asks for; BULK: the search window comes by bulk row
- * copies.  Each launch runs the instantiation for its flags
+ * copies; CODE: the launch makes the MBs' coefficient bit strings.  Each launch runs the instantiation for its flags
  * (h261b_launch_step), so no launch carries code it never runs: instruction
  * fetch is a seventh of the kernel's stalls, and leaving the bulk staging's
  * code out of the cp.async kernel alone took its launch of 13,464
  * macroblocks from 83.0 to 79.4 us. */
-template <int FMAD, int KIND, bool FULL_SEARCH, bool ABI, bool BULK>
+template <int FMAD, int KIND, bool FULL_SEARCH, bool ABI, bool BULK, bool CODE>
 __global__ void __launch_bounds__(256, KIND == KIND_SEARCH ? H261B_SEARCH_MIN_BLOCKS : H261B_STEP_MIN_BLOCKS)
     step_kernel(const h261b_session_dev_t *__restrict__ sessions, const uint32_t *__restrict__ work, int32_t n_work,
                 int32_t chunk, int32_t phases_arg, int32_t *sched)
@@ -1273,10 +1284,12 @@ __global__ void __launch_bounds__(256, KIND == KIND_SEARCH ? H261B_SEARCH_MIN_BL
                        : KIND == KIND_FULL   ? (H261B_PHASE_ME | H261B_PHASE_MD | H261B_PHASE_ENCDEC)
                                              : phases_arg;
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    const size_t warp_bytes = KIND == KIND_SEARCH ? kSearchWarpBytes : sizeof(WarpSmem);
+    const size_t warp_bytes = KIND == KIND_SEARCH ? kSearchWarpBytes : CODE ? sizeof(WarpSmem) : kEncodeWarpBytes;
     unsigned char *mine = smem_raw + warp * warp_bytes;
     uint32_t *wbuf = reinterpret_cast<uint32_t *>(mine);
     float(*tb)[TB_BLOCK] = reinterpret_cast<WarpSmem *>(mine)->t;   /* not used by KIND_SEARCH */
+    VlcScratch &vlc = reinterpret_cast<WarpSmem *>(mine)->vlc;      /* nor this */
+    VlcTables &tables = *reinterpret_cast<VlcTables *>(smem_raw + (blockDim.x >> 5) * warp_bytes);
     /* this lane's column factors: forward post-scale (times 0.125, exact)
      * and inverse pre-scale */
     const float fwd_c = __fmul_rn(c_fwd_post[lane & 7], 0.125f), inv_c = c_inv_pre[lane & 7];
@@ -1303,6 +1316,12 @@ __global__ void __launch_bounds__(256, KIND == KIND_SEARCH ? H261B_SEARCH_MIN_BL
             asm volatile("fence.mbarrier_init.release.cluster;\n" ::: "memory");
         }
         __syncwarp();
+    }
+    if (CODE) {
+        load_vlc_tables(tables, (int)threadIdx.x, (int)blockDim.x);
+        for (int i = lane; i < VLC_MB_WORDS; i += 32)
+            vlc.stage[i] = 0u;
+        __syncthreads();
     }
     const int warps = blockDim.x >> 5;
     const int total_warps = gridDim.x * warps;
@@ -1470,9 +1489,9 @@ __global__ void __launch_bounds__(256, KIND == KIND_SEARCH ? H261B_SEARCH_MIN_BL
             /* this column's eight denoise offsets, UInt16, one 16-byte load */
             const uint4 offw = *reinterpret_cast<const uint4 *>(&S.dn->offset[t][lane & 7][0]);
             const ChromaRef ref = chroma_ref(S, mbx, mby, m, lane);
-            cbp = encdec_pass<FMAD, ABI>(tb, luma_row(b, S, mbx, mby, m, lane), S, mb, m, quant, offw, true, lane,
+            cbp = encdec_pass<FMAD, ABI, CODE>(tb, vlc.cm, luma_row(b, S, mbx, mby, m, lane), S, mb, m, quant, offw, true, lane,
                                          fwd_c, inv_c, noise, ssd_l);
-            cbp |= encdec_pass<FMAD, ABI>(tb, chroma_row(b, S, mbx, mby, m, ref, lane), S, mb, m, quant, offw, false,
+            cbp |= encdec_pass<FMAD, ABI, CODE>(tb, vlc.cm, chroma_row(b, S, mbx, mby, m, ref, lane), S, mb, m, quant, offw, false,
                                           lane, fwd_c, inv_c, noise, ssd_c);
             if (S.ssd_out) {
                 const uint32_t ey = __reduce_add_sync(FULL, ssd_l);
@@ -1487,6 +1506,18 @@ __global__ void __launch_bounds__(256, KIND == KIND_SEARCH ? H261B_SEARCH_MIN_BL
             run_n++;
 
             const int flags = m.flags | (cbp ? H261B_MB_COEFF : 0);
+            /* the MB's coefficient bit string: all blocks of an intra MB, the
+             * coded ones of an inter MB (bit b = block b) */
+            int coef_bits = 0;
+            if (CODE && S.bits_out) {
+                const bool intra = m.type == H261B_MB_TYPE_INTRA;
+                const uint32_t blocks = intra ? 63u : __brev(cbp) >> 26;
+                if (blocks) {
+                    int oob = 0;
+                    const int pos = code_mb(blocks, intra, tables, vlc, lane, oob);
+                    coef_bits = store_mb_string(vlc.stage, S.vlc_scratch + (size_t)mb * VLC_MB_WORDS, pos, oob, lane);
+                }
+            }
             if (lane == 0) {
                 if (ABI && S.abi_out) {
                     h261_macroblock_t *o = &S.abi_out[mb];
@@ -1509,7 +1540,7 @@ __global__ void __launch_bounds__(256, KIND == KIND_SEARCH ? H261B_SEARCH_MIN_BL
                     inf.mvx = (int8_t)m.mvx;
                     inf.mvy = (int8_t)m.mvy;
                     inf.cost = m.cost;
-                    inf.coef_bits = 0;   /* the bitstream kernels fill it in */
+                    inf.coef_bits = coef_bits;
                     S.info_out[mb] = inf;
                 }
             }
@@ -1600,30 +1631,39 @@ using StepFn = void (*)(const h261b_session_dev_t *, const uint32_t *, int32_t, 
 
 /* the instantiation of a launch's flags: the encode kind has no search and
  * writes no reference-layout output, the search kind no encode output */
-template <int FMAD, bool BULK>
+template <int FMAD, bool BULK, bool CODE>
 StepFn step_fn_of(int kind, int full)
 {
     if (kind == KIND_ENCODE)
-        return step_kernel<FMAD, KIND_ENCODE, false, false, BULK>;
-    if (kind == KIND_SEARCH)
-        return full ? step_kernel<FMAD, KIND_SEARCH, true, false, BULK>
-                    : step_kernel<FMAD, KIND_SEARCH, false, false, BULK>;
+        return step_kernel<FMAD, KIND_ENCODE, false, false, BULK, CODE>;
     if (kind == KIND_FULL)
-        return full ? step_kernel<FMAD, KIND_FULL, true, false, BULK> : step_kernel<FMAD, KIND_FULL, false, false, BULK>;
-    return full ? step_kernel<FMAD, KIND_FUSED, true, false, BULK> : step_kernel<FMAD, KIND_FUSED, false, false, BULK>;
+        return full ? step_kernel<FMAD, KIND_FULL, true, false, BULK, CODE>
+                    : step_kernel<FMAD, KIND_FULL, false, false, BULK, CODE>;
+    return full ? step_kernel<FMAD, KIND_FUSED, true, false, BULK, CODE>
+                : step_kernel<FMAD, KIND_FUSED, false, false, BULK, CODE>;
+}
+
+template <int FMAD, bool BULK>
+StepFn step_fn_of(int kind, int full, int code)
+{
+    if (kind == KIND_SEARCH)
+        return full ? step_kernel<FMAD, KIND_SEARCH, true, false, BULK, false>
+                    : step_kernel<FMAD, KIND_SEARCH, false, false, BULK, false>;
+    return code ? step_fn_of<FMAD, BULK, true>(kind, full) : step_fn_of<FMAD, BULK, false>(kind, full);
 }
 
 template <int FMAD>
-StepFn step_fn_of(int kind, int full, int abi, int bulk)
+StepFn step_fn_of(int kind, int full, int abi, int bulk, int code)
 {
     if (abi && kind != KIND_ENCODE && kind != KIND_SEARCH)
-        return full ? step_kernel<FMAD, KIND_FUSED, true, true, false> : step_kernel<FMAD, KIND_FUSED, false, true, false>;
-    return bulk ? step_fn_of<FMAD, true>(kind, full) : step_fn_of<FMAD, false>(kind, full);
+        return full ? step_kernel<FMAD, KIND_FUSED, true, true, false, false>
+                    : step_kernel<FMAD, KIND_FUSED, false, true, false, false>;
+    return bulk ? step_fn_of<FMAD, true>(kind, full, code) : step_fn_of<FMAD, false>(kind, full, code);
 }
 
-StepFn step_fn(int fmad, int kind, int full, int abi, int bulk)
+StepFn step_fn(int fmad, int kind, int full, int abi, int bulk, int code)
 {
-    return fmad ? step_fn_of<1>(kind, full, abi, bulk) : step_fn_of<0>(kind, full, abi, bulk);
+    return fmad ? step_fn_of<1>(kind, full, abi, bulk, code) : step_fn_of<0>(kind, full, abi, bulk, code);
 }
 
 } // namespace
@@ -1644,17 +1684,19 @@ extern "C" int h261b_launch_step(const h261b_session_dev_t *sessions_dev, const 
         kind = KIND_FULL;
     const int full = (phases & H261B_LAUNCH_ME_FULL) ? 1 : 0, abi = (phases & H261B_ABI_OUT) ? 1 : 0;
     const int bulk = (phases & H261B_STAGE_BULK) ? 1 : 0;
+    const int code = (phases & H261B_CODE_INLINE) ? 1 : 0;
     const bool pdl = (phases & H261B_LAUNCH_PDL) != 0;
     const int tail_code = (phases >> H261B_TAIL_SHIFT) & 15;
     if (kind > KIND_FULL)
         return (int)cudaErrorInvalidValue;
     const int ph = phases & (0xFF | H261B_STAGE_SHORT);
     const int threads = warps_per_cta * 32;
-    const size_t warp_bytes = kind == KIND_SEARCH ? kSearchWarpBytes : sizeof(WarpSmem);
-    const size_t smem = warp_bytes * (size_t)warps_per_cta;
-    const StepFn fn = step_fn(fmad, kind, full, abi, bulk);
+    const bool codes = code && kind != KIND_SEARCH && !abi;
+    const size_t warp_bytes = kind == KIND_SEARCH ? kSearchWarpBytes : codes ? sizeof(WarpSmem) : kEncodeWarpBytes;
+    const size_t smem = warp_bytes * (size_t)warps_per_cta + (codes ? sizeof(VlcTables) : 0);
+    const StepFn fn = step_fn(fmad, kind, full, abi, bulk, code);
     static std::mutex mu;
-    static int sms[64], resident[64][2][4][2][2][2][9];
+    static int sms[64], resident[64][2][4][2][2][2][2][9];
     int dev = 0;
     cudaError_t err = cudaGetDevice(&dev);
     if (err != cudaSuccess || dev < 0 || dev >= 64)
@@ -1665,16 +1707,16 @@ extern "C" int h261b_launch_step(const h261b_session_dev_t *sessions_dev, const 
         if (!sms[dev]) {
             if ((err = cudaDeviceGetAttribute(&sms[dev], cudaDevAttrMultiProcessorCount, dev)) != cudaSuccess)
                 return (int)err;
-            const int max_smem = (int)(sizeof(WarpSmem) * 8);
+            const int max_smem = (int)(sizeof(WarpSmem) * 8 + sizeof(VlcTables));
             for (int f = 0; f < 2; f++)
                 for (int k = 0; k < 4; k++)
-                    for (int x = 0; x < 8; x++)
-                        if ((err = cudaFuncSetAttribute(step_fn(f, k, x & 1, (x >> 1) & 1, x >> 2),
+                    for (int x = 0; x < 16; x++)
+                        if ((err = cudaFuncSetAttribute(step_fn(f, k, x & 1, (x >> 1) & 1, (x >> 2) & 1, x >> 3),
                                                         cudaFuncAttributeMaxDynamicSharedMemorySize, max_smem)) !=
                             cudaSuccess)
                             return (int)err;
         }
-        int &r = resident[dev][fmad][kind][full][abi][bulk][warps_per_cta];
+        int &r = resident[dev][fmad][kind][full][abi][bulk][code][warps_per_cta];
         if (!r) {
             err = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&r, fn, threads, smem);
             if (err != cudaSuccess)

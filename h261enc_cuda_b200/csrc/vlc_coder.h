@@ -10,21 +10,91 @@
  *     the table has no entry;
  *   - EOB (10) after the block.
  *
- * A warp codes up to four blocks at once: lane (slot, j), slot = lane / 8,
- * holds transmission positions 8j .. 8j+7 of its slot's block.  The codes
- * are ORed into a zeroed word buffer, MSB first.  The bitstream's codes
- * kernel runs them on each MB's levels after the encode kernel. */
+ * The encode kernel's warp codes each macroblock as soon as it has its
+ * levels, from shared memory: the levels are put into transmission order,
+ * each block gets a mask of its nonzero positions, and then every code of the
+ * macroblock -- the levels of all of its blocks and an EOB after each -- has
+ * a lane of its own.  The codes are ORed into a zeroed word buffer, MSB
+ * first. */
 #pragma once
 
 #include <cstdint>
 
-#include "vlc_tables.h"
+#include "h261b_device.h"
 
 namespace h261b {
 
 /* MB string words: six blocks of an 8-bit DC or a first code, 63 escapes of
  * 20 bits and an EOB */
 constexpr int VLC_MB_WORDS = H261B_VLC_MB_WORDS;
+
+/* zig-zag index of coefficient (vertical frequency v, horizontal u): the
+ * diagonal d = u + v starts at d(d+1)/2 (or 64 - (15-d)(16-d)/2 past the
+ * main anti-diagonal); odd diagonals run with increasing v, even ones with
+ * decreasing v -- the transmission order of H.261 */
+__host__ __device__ constexpr int zigzag_index(int v, int u)
+{
+    return (u + v < 8 ? ((u + v) * (u + v + 1)) >> 1 : 64 - (((15 - u - v) * (16 - u - v)) >> 1)) +
+           (((u + v) & 1) ? v - (u + v < 8 ? 0 : u + v - 7) : (u + v < 8 ? u + v : 7) - v);
+}
+
+/* the coder's tables (the codes are the standard's, ITU-T H.261 Table 5, the
+ * same values the reference's src/h261_tables.c holds), in device memory so
+ * that a CTA loads them with one coalesced access a thread; lanes look them
+ * up at different places, which constant memory would serve one by one */
+struct VlcTables {
+    /* TCOEFF without the sign bit, run 0..26 x level 0..15 (level 0 unused):
+     * length << 8 | code; 0 = send with the 20-bit escape */
+    uint16_t tc[27][16];
+    /* column-major index (u * 8 + v) of the k-th coefficient sent */
+    uint8_t cm[64];
+};
+static_assert(sizeof(VlcTables) % 16 == 0, "loaded as 16-byte words");
+
+#define VLC(code, len) (uint16_t)(((len) << 8) | (code))
+constexpr VlcTables make_vlc_tables()
+{
+    VlcTables t = { {
+    { 0, VLC(3, 2), VLC(4, 4), VLC(5, 5), VLC(6, 7), VLC(38, 8), VLC(33, 8), VLC(10, 10), VLC(29, 12),
+      VLC(24, 12), VLC(19, 12), VLC(16, 12), VLC(26, 13), VLC(25, 13), VLC(24, 13), VLC(23, 13) },
+    { 0, VLC(3, 3), VLC(6, 6), VLC(37, 8), VLC(12, 10), VLC(27, 12), VLC(22, 13), VLC(21, 13) },
+    { 0, VLC(5, 4), VLC(4, 7), VLC(11, 10), VLC(20, 12), VLC(20, 13) },
+    { 0, VLC(7, 5), VLC(36, 8), VLC(28, 12), VLC(19, 13) },
+    { 0, VLC(6, 5), VLC(15, 10), VLC(18, 12) },
+    { 0, VLC(7, 6), VLC(9, 10), VLC(18, 13) },
+    { 0, VLC(5, 6), VLC(30, 12) },
+    { 0, VLC(4, 6), VLC(21, 12) },
+    { 0, VLC(7, 7), VLC(17, 12) },
+    { 0, VLC(5, 7), VLC(17, 13) },
+    { 0, VLC(39, 8), VLC(16, 13) },
+    { 0, VLC(35, 8) }, { 0, VLC(34, 8) }, { 0, VLC(32, 8) }, { 0, VLC(14, 10) }, { 0, VLC(13, 10) },
+    { 0, VLC(8, 10) }, { 0, VLC(31, 12) }, { 0, VLC(26, 12) }, { 0, VLC(25, 12) }, { 0, VLC(23, 12) },
+    { 0, VLC(22, 12) }, { 0, VLC(31, 13) }, { 0, VLC(30, 13) }, { 0, VLC(29, 13) }, { 0, VLC(28, 13) },
+    { 0, VLC(27, 13) },
+}, {} };
+    for (int v = 0; v < 8; v++)
+        for (int u = 0; u < 8; u++)
+            t.cm[zigzag_index(v, u)] = (uint8_t)(u * 8 + v);
+    return t;
+}
+#undef VLC
+static __device__ const VlcTables g_vlc_tables = make_vlc_tables();
+
+/* by the threads of a CTA; the caller synchronises before the first lookup */
+__device__ __forceinline__ void load_vlc_tables(VlcTables &t, int tid, int nthreads)
+{
+    for (int i = tid; i < (int)(sizeof(VlcTables) / 16); i += nthreads)
+        reinterpret_cast<uint4 *>(&t)[i] = reinterpret_cast<const uint4 *>(&g_vlc_tables)[i];
+}
+
+/* a warp's working memory */
+struct alignas(16) VlcScratch {
+    uint32_t stage[VLC_MB_WORDS];   /* the MB's codes; zero between MBs       */
+    uint32_t cm[96];                /* the MB's levels, six blocks of 64 bytes,
+                                       column-major, an intra DC as uint8     */
+    uint32_t level[96];             /* the same in transmission order         */
+    uint32_t mask[6][2];            /* per block: its nonzero positions       */
+};
 
 /* OR a code of len <= 32 bits into MSB-first words at bit position pos of
  * a buffer of `words` words; a position outside it is not written and
@@ -46,121 +116,143 @@ __device__ __forceinline__ void put_bits(uint32_t *w, int words, int pos, uint32
     }
 }
 
-/* this lane's eight column-major indices of transmission positions
- * 8j .. 8j+7 (j = lane % 8), packed one byte each into two words */
-__device__ __forceinline__ void zigzag_lane(int lane, uint32_t &zz0, uint32_t &zz1)
+/* one bit per nonzero byte of a word */
+__device__ __forceinline__ uint32_t nonzero_bytes(uint32_t w)
 {
-    const int j = lane & 7;
-    zz0 = zz1 = 0u;
-#pragma unroll
-    for (int i = 0; i < 4; i++) {
-        zz0 |= (uint32_t)c_zigzag_cm.cm[8 * j + i] << (8 * i);
-        zz1 |= (uint32_t)c_zigzag_cm.cm[8 * j + 4 + i] << (8 * i);
+    const uint32_t f = ((((w & 0x7F7F7F7Fu) + 0x7F7F7F7Fu) | w) >> 7) & 0x01010101u;
+    return (f * 0x10204080u) >> 28;
+}
+
+/* the k-th set bit (from 0) of a mask that has it */
+__device__ __forceinline__ int select_bit(uint32_t lo, uint32_t hi, int k)
+{
+    int p = 0, c = __popc(lo);
+    uint32_t m = lo;
+    if (k >= c) {
+        k -= c;
+        p = 32;
+        m = hi;
     }
+#pragma unroll
+    for (int h = 16; h >= 1; h >>= 1) {
+        c = __popc(m & ((1u << h) - 1u));
+        if (k >= c) {
+            k -= c;
+            p += h;
+            m >>= h;
+        }
+    }
+    return p;
 }
 
-/* the TCOEFF table into shared memory (27 x 16 entries), by the threads of
- * a CTA; the caller synchronises before the first lookup */
-__device__ __forceinline__ void load_tcoeff_table(uint16_t (*tc)[16], int tid, int nthreads)
-{
-    for (int i = tid; i < 27 * 16; i += nthreads)
-        (&tc[0][0])[i] = (&c_vlc_tcoeff[0][0])[i];
-}
-
-/* One group of up to four coded blocks.  Lane (slot, j) codes positions
- * 8j .. 8j+7 of `blk` (the slot's block: 64 levels, column-major, an intra
- * DC stored as uint8) when `here`.  The group's codes go into `stage` from
- * bit `pos` on, the blocks one after another in slot order; returns the
- * group's bits (the same on every lane).  Every lane of the warp calls it. */
-__device__ __forceinline__ int code_block_group(const int8_t *blk, bool here, bool intra, uint32_t zz0, uint32_t zz1,
-                                                const uint16_t (*tc)[16], uint32_t *stage, int words, int pos,
-                                                int lane, int &oob)
+/* The codes of an MB's coded blocks (bit b of `blocks`) from its levels in
+ * sc.cm.  They go into sc.stage from bit 0 on; returns their bits (the same
+ * on every lane).  Every lane of the warp calls it; the caller's warp has
+ * synchronised after writing the levels.
+ *
+ * Blocks hold a few nonzero levels each, so a lane a code does in one round
+ * of about a hundred instructions what a kernel of its own, with eight
+ * positions a lane and four blocks at a time, took two rounds of 280 for. */
+__device__ __forceinline__ int code_mb(uint32_t blocks, bool intra, const VlcTables &tab, VlcScratch &sc, int lane,
+                                       int &oob)
 {
     constexpr unsigned FULLMASK = 0xFFFFFFFFu;
-    const int slot = lane >> 3, j = lane & 7;
-    int c[8];
-    uint32_t m8 = 0;
+    /* transmission order: the lane's positions 4j .. 4j + 3 of block
+     * lane / 16 + 2 i, for i = 0, 1, 2 */
+    {
+        const int j = lane & 15, half = lane >> 4;
+        const uint32_t c4 = *reinterpret_cast<const uint32_t *>(&tab.cm[4 * j]);
+        const uint8_t *base = reinterpret_cast<const uint8_t *>(sc.cm) + 64 * half;
+        const uint8_t *a0 = base + (c4 & 0xFFu), *a1 = base + ((c4 >> 8) & 0xFFu);
+        const uint8_t *a2 = base + ((c4 >> 16) & 0xFFu), *a3 = base + (c4 >> 24);
 #pragma unroll
-    for (int i = 0; i < 8; i++) {
-        const int idx = (int)(((i < 4 ? zz0 : zz1) >> (8 * (i & 3))) & 0xFFu);
-        const int8_t x = here ? blk[idx] : (int8_t)0;
-        c[i] = (intra && j == 0 && i == 0) ? (int)(uint8_t)x : (int)x;
-        m8 |= (c[i] != 0) ? (1u << i) : 0u;
-    }
-    /* the block's nonzero mask in transmission order */
-    uint32_t mlo = j < 4 ? m8 << (8 * j) : 0u, mhi = j >= 4 ? m8 << (8 * (j - 4)) : 0u;
-#pragma unroll
-    for (int o = 1; o < 8; o <<= 1) {
-        mlo |= __shfl_xor_sync(FULLMASK, mlo, o);
-        mhi |= __shfl_xor_sync(FULLMASK, mhi, o);
-    }
-    const uint64_t mask = ((uint64_t)mhi << 32) | mlo;
-    const uint64_t bl = j ? mask & ((1ull << (8 * j)) - 1ull) : 0ull;
-    int prev = bl ? 63 - __clzll((long long)bl) : -1;
-    uint32_t code[8];
-    int clen[8], mine = 0;
-#pragma unroll
-    for (int i = 0; i < 8; i++) {
-        const int k = 8 * j + i;
-        clen[i] = 0;
-        code[i] = 0;
-        if (!((m8 >> i) & 1u))
-            continue;
-        const int v = c[i];
-        if (k == 0 && intra) {
-            code[i] = (uint32_t)v & 0xFFu;       /* the DC level as it is */
-            clen[i] = 8;
-        } else if (k == 0 && (v == 1 || v == -1)) {
-            code[i] = v < 0 ? 3u : 2u;            /* first inter coefficient +-1 */
-            clen[i] = 2;
-        } else {
-            const int run = k - prev - 1;
-            const int a = v < 0 ? -v : v;
-            const uint16_t e = (run <= 26 && a <= 15) ? tc[run][a] : (uint16_t)0;
-            if (e) {
-                code[i] = ((uint32_t)(e & 0xFF) << 1) | (v < 0 ? 1u : 0u);
-                clen[i] = (e >> 8) + 1;
-            } else {
-                /* escape 0000 01, 6-bit run, 8-bit level */
-                code[i] = (1u << 14) | ((uint32_t)run << 8) | ((uint32_t)v & 0xFFu);
-                clen[i] = 20;
-            }
+        for (int i = 0; i < 3; i++) {
+            const int b = half + 2 * i;
+            const uint32_t w = __byte_perm((uint32_t)a0[128 * i] | ((uint32_t)a1[128 * i] << 8),
+                                           (uint32_t)a2[128 * i] | ((uint32_t)a3[128 * i] << 8), 0x5410);
+            const uint32_t nz = ((blocks >> b) & 1u) ? nonzero_bytes(w) : 0u;
+            const uint32_t next = __shfl_down_sync(FULLMASK, nz, 1);
+            sc.level[16 * b + j] = w;
+            if (!(lane & 1))
+                reinterpret_cast<uint8_t *>(sc.mask[b])[j >> 1] = (uint8_t)(nz | (next << 4));
         }
-        prev = k;
-        mine += clen[i];
     }
-    /* offsets of this lane's codes within its block */
-    int incl = mine;
+    __syncwarp();
+    /* codes of block `lane` (its levels and EOB) and of the blocks up to it */
+    int n = 0;
+    if (lane < 6 && ((blocks >> lane) & 1u))
+        n = __popc(sc.mask[lane][0]) + __popc(sc.mask[lane][1]) + 1;
+    int incl = n;
 #pragma unroll
     for (int o = 1; o < 8; o <<= 1) {
-        const int t = __shfl_up_sync(FULLMASK, incl, o, 8);
-        if (j >= o)
+        const int t = __shfl_up_sync(FULLMASK, incl, o);
+        if (lane >= o)
             incl += t;
     }
-    const int last = __shfl_sync(FULLMASK, incl, (slot << 3) | 7);
-    const int btotal = here ? last + 2 : 0;
-    int bstart = pos, rtotal = 0;
+    int upto[6];
 #pragma unroll
-    for (int s2 = 0; s2 < 4; s2++) {
-        const int t = __shfl_sync(FULLMASK, btotal, s2 << 3);
-        if (s2 < slot)
-            bstart += t;
-        rtotal += t;
-    }
-    if (here) {
-        int p = bstart + incl - mine;
+    for (int b = 0; b < 6; b++)
+        upto[b] = __shfl_sync(FULLMASK, incl, b);
+    int pos = 0;
+    for (int t0 = 0; t0 < upto[5]; t0 += 32) {
+        const int t = t0 + lane;
+        uint32_t code = 0;
+        int len = 0;
+        if (t < upto[5]) {
+            int b = 0, first = 0;
 #pragma unroll
-        for (int i = 0; i < 8; i++) {
-            put_bits(stage, words, p, code[i], clen[i], oob);
-            p += clen[i];
+            for (int i = 0; i < 5; i++)
+                if (t >= upto[i]) {
+                    b = i + 1;
+                    first = upto[i];
+                }
+            const uint32_t lo = sc.mask[b][0], hi = sc.mask[b][1];
+            const int k = t - first;
+            if (k == __popc(lo) + __popc(hi)) {
+                code = 2u;              /* EOB */
+                len = 2;
+            } else {
+                const int at = select_bit(lo, hi, k);
+                const int v = reinterpret_cast<const int8_t *>(sc.level)[64 * b + at], a = v < 0 ? -v : v;
+                if (at == 0 && intra) {
+                    code = (uint32_t)v & 0xFFu;       /* the DC level as it is */
+                    len = 8;
+                } else if (at == 0 && a == 1) {
+                    code = v < 0 ? 3u : 2u;           /* first inter coefficient +-1 */
+                    len = 2;
+                } else {
+                    /* zeros since the nonzero position before */
+                    const uint32_t bh = at >= 32 ? hi & ((1u << (at - 32)) - 1u) : 0u;
+                    const uint32_t bl = at >= 32 ? lo : lo & ((1u << at) - 1u);
+                    const int prev = bh ? 63 - __clz((int)bh) : 31 - __clz((int)bl);
+                    const int run = at - prev - 1;
+                    const uint16_t e = (run <= 26 && a <= 15) ? tab.tc[run][a] : (uint16_t)0;
+                    if (e) {
+                        code = ((uint32_t)(e & 0xFF) << 1) | (v < 0 ? 1u : 0u);
+                        len = (e >> 8) + 1;
+                    } else {
+                        /* escape 0000 01, 6-bit run, 8-bit level */
+                        code = (1u << 14) | ((uint32_t)run << 8) | ((uint32_t)v & 0xFFu);
+                        len = 20;
+                    }
+                }
+            }
         }
-        if (j == 7)
-            put_bits(stage, words, bstart + btotal - 2, 2u, 2, oob);   /* EOB */
+        int end = len;
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1) {
+            const int x = __shfl_up_sync(FULLMASK, end, o);
+            if (lane >= o)
+                end += x;
+        }
+        put_bits(sc.stage, VLC_MB_WORDS, pos + end - len, code, len, oob);
+        pos += __shfl_sync(FULLMASK, end, 31);
     }
-    return rtotal;
+    __syncwarp();   /* the codes are in place */
+    return pos;
 }
 
-/* after an MB's groups: its string from the staging words into dst (the
+/* after code_mb: the MB's string from the staging words into dst (the
  * MB's VLC_MB_WORDS words), the staging words cleared for the next MB;
  * returns the string's bits, or -1 if a code fell outside the words (which
  * makes the layout refuse the picture).  Every lane calls it. */

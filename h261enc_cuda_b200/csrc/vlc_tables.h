@@ -1,6 +1,7 @@
-/* H.261 variable-length code tables for the device bitstream writer.
+/* H.261 variable-length code tables for the macroblock headers of the device
+ * bitstream writer (the coefficients' are in vlc_coder.h).
  *
- * The codes are the standard's (ITU-T H.261 Tables 1-5), the same values
+ * The codes are the standard's (ITU-T H.261 Tables 1-4), the same values
  * the reference's src/h261_tables.c holds; the writer must reproduce the
  * reference's bytes, so nothing here may differ from the standard.  Layouts
  * are ours: (length << 8) | code in 16 bits, 0 = no entry. */
@@ -11,27 +12,6 @@
 namespace h261b {
 
 #define VLC(code, len) (uint16_t)(((len) << 8) | (code))
-
-/* TCOEFF without the sign bit, run 0..26 x level 0..15 (level 0 unused);
- * 0 = send with the 20-bit escape */
-static __device__ __constant__ uint16_t c_vlc_tcoeff[27][16] = {
-    { 0, VLC(3, 2), VLC(4, 4), VLC(5, 5), VLC(6, 7), VLC(38, 8), VLC(33, 8), VLC(10, 10), VLC(29, 12),
-      VLC(24, 12), VLC(19, 12), VLC(16, 12), VLC(26, 13), VLC(25, 13), VLC(24, 13), VLC(23, 13) },
-    { 0, VLC(3, 3), VLC(6, 6), VLC(37, 8), VLC(12, 10), VLC(27, 12), VLC(22, 13), VLC(21, 13) },
-    { 0, VLC(5, 4), VLC(4, 7), VLC(11, 10), VLC(20, 12), VLC(20, 13) },
-    { 0, VLC(7, 5), VLC(36, 8), VLC(28, 12), VLC(19, 13) },
-    { 0, VLC(6, 5), VLC(15, 10), VLC(18, 12) },
-    { 0, VLC(7, 6), VLC(9, 10), VLC(18, 13) },
-    { 0, VLC(5, 6), VLC(30, 12) },
-    { 0, VLC(4, 6), VLC(21, 12) },
-    { 0, VLC(7, 7), VLC(17, 12) },
-    { 0, VLC(5, 7), VLC(17, 13) },
-    { 0, VLC(39, 8), VLC(16, 13) },
-    { 0, VLC(35, 8) }, { 0, VLC(34, 8) }, { 0, VLC(32, 8) }, { 0, VLC(14, 10) }, { 0, VLC(13, 10) },
-    { 0, VLC(8, 10) }, { 0, VLC(31, 12) }, { 0, VLC(26, 12) }, { 0, VLC(25, 12) }, { 0, VLC(23, 12) },
-    { 0, VLC(22, 12) }, { 0, VLC(31, 13) }, { 0, VLC(30, 13) }, { 0, VLC(29, 13) }, { 0, VLC(28, 13) },
-    { 0, VLC(27, 13) },
-};
 
 /* MBA, address increment 1..33 */
 static __device__ __constant__ uint16_t c_vlc_mba[34] = {
@@ -71,39 +51,5 @@ enum {
     MT_MC_FIL, MT_MC_FIL_CBP, MT_MC_FIL_CBP_MQ
 };
 static __device__ __constant__ uint8_t c_vlc_mtype_len[10] = { 4, 7, 1, 5, 9, 8, 10, 3, 2, 6 };
-
-/* zig-zag index of coefficient (vertical frequency v, horizontal u): the
- * diagonal d = u + v starts at d(d+1)/2 (or 64 - (15-d)(16-d)/2 past the
- * main anti-diagonal); odd diagonals run with increasing v, even ones with
- * decreasing v -- the transmission order of H.261 */
-__host__ __device__ constexpr int zigzag_index(int v, int u)
-{
-    return (u + v < 8 ? ((u + v) * (u + v + 1)) >> 1 : 64 - (((15 - u - v) * (16 - u - v)) >> 1)) +
-           (((u + v) & 1) ? v - (u + v < 8 ? 0 : u + v - 7) : (u + v < 8 ? u + v : 7) - v);
-}
-
-/* column-major index (u * 8 + v) of the k-th coefficient sent, generated
- * from zigzag_index at compile time */
-struct ZigzagTable {
-    uint8_t cm[64];
-};
-__host__ __device__ constexpr ZigzagTable make_zigzag_table()
-{
-    ZigzagTable t{};
-    for (int v = 0; v < 8; v++)
-        for (int u = 0; u < 8; u++)
-            t.cm[zigzag_index(v, u)] = (uint8_t)(u * 8 + v);
-    return t;
-}
-static __device__ __constant__ ZigzagTable c_zigzag_cm = make_zigzag_table();
-
-/* bits of one non-DC coefficient sent after `run` zeros: table code plus
- * sign, or the escape */
-__device__ __forceinline__ int tcoeff_bits(int run, int level)
-{
-    const int a = level < 0 ? -level : level;
-    const int e = (run <= 26 && a <= 15) ? (c_vlc_tcoeff[run][a] >> 8) : 0;
-    return e ? e + 1 : 20;
-}
 
 } // namespace h261b
