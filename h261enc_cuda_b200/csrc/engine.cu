@@ -346,6 +346,21 @@ struct h261b_engine_s {
     bool step_bits_ran[NSLOT] = {};
     bool in_flight[NSLOT] = {};
     int64_t step_mbs[NSLOT] = {};   /* MB records of the step in each arena */
+    /* sessions that have queued a picture since the last step, in the order
+     * of the calls (one that was closed since is skipped), and each slot's
+     * latest step's sessions in ascending order */
+    std::vector<int32_t> queue;
+    std::vector<int32_t> step_sessions[NSLOT];
+    /* what each slot's work list holds: the sizes of its sessions in order
+     * (and whether rate-controlled), where it lies, and whether the device
+     * copy is the same.  Steps of the same sessions, a stream's usual case,
+     * write and upload it once. */
+    struct WorkList {
+        std::vector<uint32_t> sizes;
+        const void *host = nullptr, *dev = nullptr;
+        size_t off = 0;
+        bool uploaded = false;
+    } work_list[NSLOT];
     int64_t last_h2d = 0, last_d2h = 0;  /* bytes copied by the last step */
     HostArena bits[NSLOT];     /* pictures written by the bitstream kernel */
     size_t bits_want = 0;      /* capacity the arenas grow to              */
@@ -911,6 +926,7 @@ static int reserve_input(h261b_engine_t *e, Session *s, int32_t id, int32_t quan
     e->upload_used = *off + align_up(s->lay.bytes, 256);
     s->src_off = *off;
     s->queued = true;
+    e->queue.push_back(id);
     s->queued_quant = quant > 0 ? quant : 0;
     return H261B_OK;
 }
@@ -977,6 +993,7 @@ extern "C" int h261b_engine_inputs(h261b_engine_t *e, int32_t n, const int32_t *
                 Session *t = get_session(e, ids[j]);
                 t->queued = false;
                 t->queued_quant = 0;
+                e->queue.pop_back();
             }
             e->upload_used = used0;
             return rc;
@@ -1098,6 +1115,7 @@ extern "C" int h261b_session_submit_device(h261b_engine_t *e, int32_t id, const 
     s->dev_src[2] = cr;
     s->queued = true;
     s->queued_quant = quant > 0 ? quant : 0;
+    e->queue.push_back(id);
     return H261B_OK;
 }
 
@@ -1142,6 +1160,7 @@ extern "C" int h261b_engine_submit_device_batch(h261b_engine_t *e, int32_t n, co
         s.dev_src[2] = cr[i];
         s.queued = true;
         s.queued_quant = q > 0 ? q : 0;
+        e->queue.push_back(ids[i]);
     }
     return H261B_OK;
 }
@@ -1173,12 +1192,19 @@ extern "C" int h261b_engine_step(h261b_engine_t *e)
     const int64_t id = e->next_step;
     const int p = (int)(id % NSLOT);
     const int prev = (int)((id + NSLOT - 1) % NSLOT);   /* the slot of step id - 1 */
+    /* the queued sessions in ascending order: a session closed since it
+     * queued is out, one whose slot was opened and queued again is in once */
     std::vector<int32_t> list;
-    for (size_t i = 0; i < e->sessions.size(); i++)
-        if (e->sessions[i].open && e->sessions[i].queued)
-            list.push_back((int32_t)i);
-    if (list.empty())
+    list.reserve(e->queue.size());
+    for (int32_t i : e->queue)
+        if (e->sessions[(size_t)i].open && e->sessions[(size_t)i].queued)
+            list.push_back(i);
+    std::sort(list.begin(), list.end());
+    list.erase(std::unique(list.begin(), list.end()), list.end());
+    if (list.empty()) {
+        e->queue.clear();
         return 0;
+    }
     /* this step's descriptor and result bytes (the layouts below) */
     {
         int64_t mbs = 0;
@@ -1327,19 +1353,41 @@ extern "C" int h261b_engine_step(h261b_engine_t *e)
     }
     /* work list: the MBs of fixed-QUANT sessions, then those of
      * rate-controlled ones (the second encode launch takes that tail) */
-    for (int pass = 0; pass < 2; pass++) {
-        if (pass == 1)
-            rc_begin = n_work;
+    h261b_engine_s::WorkList &wl = e->work_list[p];
+    {
+        bool same = wl.host == dm.host && wl.dev == dm.dev && wl.off == work_off && wl.sizes.size() == n;
         for (size_t k = 0; k < n; k++) {
             const Session &s = e->sessions[(size_t)list[k]];
-            if ((int)s.rc != pass)
-                continue;
-            for (int32_t m = 0; m < s.nmb; m++)
-                work[n_work++] = ((uint32_t)k << 12) | (uint32_t)m;
+            const uint32_t size = (uint32_t)s.nmb | (s.rc ? 1u << 31 : 0u);
+            same = same && wl.sizes[k] == size;
+            n_work += s.nmb;
+            if (!s.rc)
+                rc_begin += s.nmb;
+        }
+        if (!same) {
+            wl.host = dm.host;
+            wl.dev = dm.dev;
+            wl.off = work_off;
+            wl.uploaded = false;
+            wl.sizes.resize(n);
+            uint32_t *w = work;
+            for (int pass = 0; pass < 2; pass++)
+                for (size_t k = 0; k < n; k++) {
+                    const Session &s = e->sessions[(size_t)list[k]];
+                    wl.sizes[k] = (uint32_t)s.nmb | (s.rc ? 1u << 31 : 0u);
+                    if ((int)s.rc != pass)
+                        continue;
+                    const uint32_t base = (uint32_t)k << 12;
+                    const int32_t nmb = s.nmb;
+                    for (int32_t m = 0; m < nmb; m++)
+                        w[m] = base | (uint32_t)m;
+                    w += nmb;
+                }
         }
     }
     cudaStream_t st = e->stream[p];
-    const size_t desc_bytes = align_up(work_off + (size_t)n_work * sizeof(uint32_t), 16);
+    const size_t desc_bytes = wl.uploaded ? work_off : align_up(work_off + (size_t)n_work * sizeof(uint32_t), 16);
+    wl.uploaded = false;   /* until this step's launches are issued */
     e->copier->join();   /* pictures of h261b_engine_submit_batch_async */
     LaunchPlan plan;
     const int tuning = next_plan(e, 2 * inter_mbs >= total_mb, &plan);
@@ -1523,6 +1571,7 @@ extern "C" int h261b_engine_step(h261b_engine_t *e)
     e->last_d2h = (int64_t)d2h;
     e->in_flight[p] = true;
     e->step_mbs[p] = total_mb;
+    wl.uploaded = true;
 
     if (tuning) {
         /* time this candidate before moving on (tuning steps are synchronous) */
@@ -1540,6 +1589,8 @@ extern "C" int h261b_engine_step(h261b_engine_t *e)
         s.rec_cur ^= 1;
         s.frame_index++;
     }
+    e->queue.clear();
+    e->step_sessions[p].swap(list);
     e->next_step = id + 1;
     e->upload_checked = false;
     e->upload_used = 0;
@@ -1670,7 +1721,8 @@ extern "C" int h261b_engine_step_bits(h261b_engine_t *e, int64_t *bytes, int32_t
         return H261B_OK;
     const int p = (int)(e->done_step % NSLOT);
     const Mirror &rm = e->results[p];
-    for (const Session &s : e->sessions) {
+    for (int32_t i : e->step_sessions[p]) {
+        const Session &s = e->sessions[(size_t)i];
         const Result &r = s.res[p];
         if (!s.open || !r.has_bits || r.step != e->done_step)
             continue;
@@ -1807,8 +1859,8 @@ extern "C" int h261b_engine_step_pictures(h261b_engine_t *e, int32_t cap, h261b_
     const Mirror &rm = e->results[p];
     int64_t span = 0;
     int32_t n = 0;
-    for (size_t i = 0; i < e->sessions.size(); i++) {
-        const Session &s = e->sessions[i];
+    for (int32_t i : e->step_sessions[p]) {
+        const Session &s = e->sessions[(size_t)i];
         const Result &r = s.res[p];
         if (!s.open || !r.has_bits || r.step != e->done_step)
             continue;
@@ -1819,7 +1871,7 @@ extern "C" int h261b_engine_step_pictures(h261b_engine_t *e, int32_t cap, h261b_
             e->bits_want = std::max(e->bits_want, 2 * e->bits[p].cap);   /* later steps fit */
         if (n < cap) {
             h261b_picture_t &o = out[n];
-            o.session_id = (int32_t)i;
+            o.session_id = i;
             o.frame_index = r.frame;
             o.bytes = pi.status == 0 ? pi.bytes : 0;
             o.status = pi.status == 0 ? (pi.host_off >= 0 ? 0 : 1) : H261B_ERR_STATE;
