@@ -1412,18 +1412,29 @@ extern "C" int h261b_engine_step(h261b_engine_t *e)
     const size_t d2h = e->cfg.levels_to_host ? res_off : levels_base;
     if (n_bits && (rc = e->bits[p].reserve(e->bits_want)))
         return rc;
-    /* When every picture of the step is written as a bitstream and no levels
-     * are wanted, the pack kernel stores each picture's records straight into
-     * the host's results (pinned, so the device can address them) beside its
-     * bytes, and no copy follows it: a copy of 1.6 KB behind the kernels took
-     * about 10 us. */
-    const bool direct = n_bits == (int32_t)n && !e->cfg.levels_to_host;
+    /* Results go straight to the host's results arena (pinned, so the device
+     * can address it) where the kernel that makes them can store them there:
+     * the records, sizes and squared errors of a bitstream's picture from the
+     * pack kernel beside its bytes, the records of pictures without bitstream
+     * or squared errors and the levels from the encode kernel.  When that is
+     * everything, no copy follows the kernels: one of 1.6 KB took about 10 us,
+     * and the levels of four 640x480 pictures (1.8 MB) 45 us, which now pass
+     * while the encode kernel runs. */
+    const bool levels_direct = e->cfg.levels_to_host && (coded || n_bits == 0);
+    const bool direct = (!e->cfg.levels_to_host || levels_direct) &&
+                        (n_bits == (int32_t)n || (n_bits == 0 && n_ssd == 0));
     if (direct)
         for (size_t k = 0; k < n; k++) {
             const Result &r = e->sessions[(size_t)list[k]].res[p];
-            desc[k].pic_out = (h261b_pic_info_t *)(rm.host + r.pic_off);
-            desc[k].host_info = (h261b_mb_info_t *)(rm.host + r.info_off);
-            desc[k].host_ssd = r.has_ssd ? (unsigned long long *)(rm.host + r.ssd_off) : nullptr;
+            if (levels_direct)
+                desc[k].level_out = (int8_t *)(rm.host + r.level_off);
+            if (n_bits) {
+                desc[k].pic_out = (h261b_pic_info_t *)(rm.host + r.pic_off);
+                desc[k].host_info = (h261b_mb_info_t *)(rm.host + r.info_off);
+                desc[k].host_ssd = r.has_ssd ? (unsigned long long *)(rm.host + r.ssd_off) : nullptr;
+            } else {
+                desc[k].info_out = (h261b_mb_info_t *)(rm.host + r.info_off);
+            }
         }
     /* A small step's descriptors and pictures come up by a kernel that reads
      * them from the pinned arenas: the two copies it replaces take 13 us on
