@@ -1390,14 +1390,23 @@ extern "C" int h261b_engine_step(h261b_engine_t *e)
     wl.uploaded = false;   /* until this step's launches are issued */
     e->copier->join();   /* pictures of h261b_engine_submit_batch_async */
     LaunchPlan plan;
-    const int tuning = next_plan(e, 2 * inter_mbs >= total_mb, &plan);
+    /* a step too small to give each resident warp slot a MB takes a team of
+     * warps for each, unless the configuration asks for a launch shape; the
+     * plan, and its trial, are for the larger ones */
+    const bool team = total_mb <= (int64_t)H261B_TEAM_PER_SM * e->sm_count && e->cfg.warps_per_cta == 0 &&
+                      e->cfg.max_ctas == 0 && e->cfg.kernel_split == 0 && e->cfg.tail_items == 0 &&
+                      e->cfg.staging == 0;
+    const int tuning = team ? 0 : next_plan(e, 2 * inter_mbs >= total_mb, &plan);
+    const int team_bit = team ? H261B_LAUNCH_TEAM : 0;
+    if (team)
+        plan = LaunchPlan();
     const int warps = plan.warps, ctas = plan.ctas;
     /* the arithmetic and the search mode are the engine's, for every launch */
     const int fmad_bit =
         (e->cfg.fmad ? H261B_FMAD_BIT : 0) | (e->cfg.me_mode == H261B_ME_FULL ? H261B_LAUNCH_ME_FULL : 0);
     const int code_bit = n_bits && coded ? H261B_CODE_INLINE : 0;
     const int phases = H261B_PHASE_ME | H261B_PHASE_MD | H261B_PHASE_ENCDEC | fmad_bit | plan.bits() |
-                       e->test_bits | (plan.split ? H261B_KIND_SEARCH : 0) | code_bit;
+                       e->test_bits | (plan.split ? H261B_KIND_SEARCH : 0) | code_bit | team_bit;
     if (!plan.split)
         for (size_t k = 0; k < n; k++)
             if (!desc[k].rc)
@@ -1495,8 +1504,8 @@ extern "C" int h261b_engine_step(h261b_engine_t *e)
                                    warps, ctas, sched, st);
         } else if (lr == 0 && n_rc) {
             lr = h261b_launch_step(desc_dev, work_dev + rc_begin, n_work - rc_begin,
-                                   H261B_PHASE_ENCDEC | fmad_bit | plan.bits() | e->test_bits | code_bit, warps, ctas,
-                                   sched, st);
+                                   H261B_PHASE_ENCDEC | fmad_bit | plan.bits() | e->test_bits | code_bit | team_bit, warps,
+                                   ctas, sched, st);
         }
         if (lr != 0) {
             set_error("step launch failed: %s", cudaGetErrorString((cudaError_t)lr));

@@ -155,7 +155,8 @@ typedef struct {
  *   bits 9-10    kernel kind: 0 fused (the phases above in one pass),
  *                1 search (ME + MD into md_out), 2 encode (ENCDEC from md_in)
  *   bit 11       programmatic dependent launch on the kernel before it in
- *                the stream (an encode launch right after its search launch)
+ *                the stream (an encode launch right after its search launch,
+ *                a launch right after the kernel that writes its descriptor)
  *   bits 12-15   tail items per warp drawn from the scheduler, plus one
  *                (0: the default, 2)
  */
@@ -179,6 +180,12 @@ typedef struct {
 /*   bit 20       sessions with bits_out: each MB's coefficient bit string is
  *                made by the warp that encodes it */
 #define H261B_CODE_INLINE   0x100000
+/*   bit 21       a CTA of four warps per MB (small launches; fused phases,
+ *                cp.async staging, no reference-layout outputs) */
+#define H261B_LAUNCH_TEAM   0x200000
+/* MBs a multiprocessor up to which that is the launch: four such CTAs are
+ * resident on each */
+#define H261B_TEAM_PER_SM   4
 #define H261B_LAUNCH_ME_FULL 0x40000
 #define H261B_ABI_OUT       0x80000
 
@@ -193,6 +200,9 @@ int h261b_launch_step(const h261b_session_dev_t *sessions_dev, const uint32_t *w
                       int32_t n_work, int32_t phases, int32_t warps_per_cta, int32_t max_ctas,
                       int32_t *sched_dev, void *stream);
 int h261b_set_quant_table(void);
+/* a team launch over one picture whose descriptor (host memory) travels with
+ * the launch; nothing is counted in its mbs_done */
+int h261b_launch_team_picture(const h261b_session_dev_t *session, int32_t phases, void *stream);
 /* copy two spans from pinned host memory into device memory and zero a third
  * by a kernel (all 16-byte aligned, sizes in bytes, multiples of 16) */
 #define H261B_FETCH_MAX (256 * 1024)   /* bytes up to which a step uses it */

