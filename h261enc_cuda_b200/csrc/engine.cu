@@ -337,7 +337,8 @@ struct h261b_engine_s {
      * the host */
     cudaEvent_t t_begin[NSLOT] = {}, t_h2d[NSLOT] = {};
     cudaEvent_t k_start[NSLOT] = {}, k_end[NSLOT] = {}, t_end[NSLOT] = {};
-    cudaEvent_t b_end[NSLOT] = {};         /* after the bitstream kernel */
+    cudaEvent_t b_end[NSLOT] = {};         /* after the bitstream kernels */
+    cudaEvent_t bits_end[NSLOT] = {};      /* b_end, or t_end where that is the same */
     cudaEvent_t layout_done[NSLOT] = {};   /* rate control inputs written */
     /* step arena bytes asked for by h261b_engine_reserve_step */
     size_t reserved_upload = 0, reserved_results = 0, reserved_desc = 0;
@@ -1390,13 +1391,13 @@ extern "C" int h261b_engine_step(h261b_engine_t *e)
     wl.uploaded = false;   /* until this step's launches are issued */
     e->copier->join();   /* pictures of h261b_engine_submit_batch_async */
     LaunchPlan plan;
+    const int tuning = next_plan(e, 2 * inter_mbs >= total_mb, &plan);
     /* a step too small to give each resident warp slot a MB takes a team of
-     * warps for each, unless the configuration asks for a launch shape; the
-     * plan, and its trial, are for the larger ones */
-    const bool team = total_mb <= (int64_t)H261B_TEAM_PER_SM * e->sm_count && e->cfg.warps_per_cta == 0 &&
+     * warps for each, unless the configuration asks for a launch shape or the
+     * step is one of the plan's trial */
+    const bool team = !tuning && total_mb <= (int64_t)H261B_TEAM_PER_SM * e->sm_count && e->cfg.warps_per_cta == 0 &&
                       e->cfg.max_ctas == 0 && e->cfg.kernel_split == 0 && e->cfg.tail_items == 0 &&
                       e->cfg.staging == 0;
-    const int tuning = team ? 0 : next_plan(e, 2 * inter_mbs >= total_mb, &plan);
     const int team_bit = team ? H261B_LAUNCH_TEAM : 0;
     if (team)
         plan = LaunchPlan();
@@ -1448,8 +1449,11 @@ extern "C" int h261b_engine_step(h261b_engine_t *e)
     /* A small step's descriptors and pictures come up by a kernel that reads
      * them from the pinned arenas: the two copies it replaces take 13 us on
      * the copy engine, however few bytes they move (12 -> 4 us for the
-     * descriptors of 64 streams).  Larger uploads stay with the copy engine,
-     * which runs beside the previous step's kernels. */
+     * descriptors of 64 streams), and the pictures are then in L2 for the
+     * encode kernel (four 640x480 pictures: upload 45.9 -> 45.1, encode 44.5
+     * -> 38.6 us; ten due pictures, 0.7 MB: 25.4 -> 22.4 us of upload).
+     * Larger uploads stay with the copy engine, which runs beside the
+     * previous step's kernels: it is as fast from some megabytes on. */
     const bool fetch = desc_bytes + upload_bytes <= H261B_FETCH_MAX;
 
     /* the step's device work: uploads, encode (and rate control), the
@@ -1459,7 +1463,18 @@ extern "C" int h261b_engine_step(h261b_engine_t *e)
     auto enqueue = [&](bool capturing) -> int {
         const unsigned rf = capturing ? cudaEventRecordExternal : cudaEventRecordDefault;
         const unsigned wf = capturing ? cudaEventWaitExternal : cudaEventWaitDefault;
-        H261B_CUDA_TRY(cudaEventRecordWithFlags(e->t_begin[p], st, rf));
+        /* A boundary's event.  In a graph an event is a node of about a
+         * microsecond, so there the side stream records it, beside the chain
+         * of copies and kernels and not in it. */
+        auto mark = [&](cudaEvent_t ev) -> cudaError_t {
+            if (!capturing)
+                return cudaEventRecord(ev, st);
+            cudaError_t err = cudaEventRecord(e->fork_ev[p], st);
+            if (err == cudaSuccess)
+                err = cudaStreamWaitEvent(e->side[p], e->fork_ev[p], 0);
+            return err == cudaSuccess ? cudaEventRecordWithFlags(ev, e->side[p], rf) : err;
+        };
+        H261B_CUDA_TRY(mark(e->t_begin[p]));
         if (fetch) {
             const int fr = h261b_launch_fetch(dm.dev, dm.host, (int64_t)desc_bytes, um.dev, um.host,
                                               (int64_t)upload_bytes, rm.dev + ssd_base, n_ssd ? (int64_t)n * 32 : 0,
@@ -1475,11 +1490,11 @@ extern "C" int h261b_engine_step(h261b_engine_t *e)
             if (upload_bytes)
                 H261B_CUDA_TRY(cudaMemcpyAsync(um.dev, um.host, upload_bytes, cudaMemcpyHostToDevice, st));
         }
-        H261B_CUDA_TRY(cudaEventRecordWithFlags(e->t_h2d[p], st, rf));
+        H261B_CUDA_TRY(mark(e->t_h2d[p]));
         /* the previous step's reconstructions are this step's references */
         if (id > 0)
             H261B_CUDA_TRY(cudaStreamWaitEvent(st, e->k_end[prev], wf));
-        H261B_CUDA_TRY(cudaEventRecordWithFlags(e->k_start[p], st, rf));
+        H261B_CUDA_TRY(mark(e->k_start[p]));
         int32_t *sched = e->sched_dev + 2 * p;
         /* fused: one launch encodes the fixed-QUANT sessions and searches
          * the rate-controlled ones; split: a search launch over every MB
@@ -1525,7 +1540,9 @@ extern "C" int h261b_engine_step(h261b_engine_t *e)
                 set_error("bitstream launch failed: %s", cudaGetErrorString((cudaError_t)lr));
                 return H261B_ERR_CUDA;
             }
-            H261B_CUDA_TRY(cudaEventRecordWithFlags(e->b_end[p], st, rf));
+            /* without a copy after them the bitstream kernels' end is the step's */
+            if (!direct)
+                H261B_CUDA_TRY(cudaEventRecordWithFlags(e->b_end[p], st, rf));
         }
         /* the step's end, and a records download, wait for the encode
          * kernel's end: the bitstream kernels may finish first (the first of
@@ -1587,6 +1604,7 @@ extern "C" int h261b_engine_step(h261b_engine_t *e)
             return rc;
     }
     e->step_bits_ran[p] = n_bits > 0;
+    e->bits_end[p] = direct ? e->t_end[p] : e->b_end[p];
     e->last_h2d = (int64_t)desc_bytes + (int64_t)upload_bytes;
     e->last_d2h = (int64_t)d2h;
     e->in_flight[p] = true;
@@ -1831,8 +1849,8 @@ extern "C" int h261b_engine_last_bits_ms(h261b_engine_t *e, float *ms)
     *ms = 0.f;
     if (!e->step_bits_ran[p])
         return H261B_OK;
-    H261B_CUDA_TRY(cudaEventSynchronize(e->b_end[p]));
-    H261B_CUDA_TRY(cudaEventElapsedTime(ms, e->k_end[p], e->b_end[p]));
+    H261B_CUDA_TRY(cudaEventSynchronize(e->bits_end[p]));
+    H261B_CUDA_TRY(cudaEventElapsedTime(ms, e->k_end[p], e->bits_end[p]));
     return H261B_OK;
 }
 
@@ -1851,7 +1869,7 @@ extern "C" int h261b_engine_step_timing(h261b_engine_t *e, h261b_step_timing_t *
     H261B_CUDA_TRY(cudaEventElapsedTime(&b, e->t_h2d[p], e->k_start[p]));
     H261B_CUDA_TRY(cudaEventElapsedTime(&c, e->k_start[p], e->k_end[p]));
     if (e->step_bits_ran[p])
-        H261B_CUDA_TRY(cudaEventElapsedTime(&d, e->k_end[p], e->b_end[p]));
+        H261B_CUDA_TRY(cudaEventElapsedTime(&d, e->k_end[p], e->bits_end[p]));
     H261B_CUDA_TRY(cudaEventElapsedTime(&f, e->t_begin[p], e->t_end[p]));
     t->step = e->done_step;
     t->upload_ms = a;

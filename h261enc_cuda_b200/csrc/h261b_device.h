@@ -205,7 +205,7 @@ int h261b_set_quant_table(void);
 int h261b_launch_team_picture(const h261b_session_dev_t *session, int32_t phases, void *stream);
 /* copy two spans from pinned host memory into device memory and zero a third
  * by a kernel (all 16-byte aligned, sizes in bytes, multiples of 16) */
-#define H261B_FETCH_MAX (256 * 1024)   /* bytes up to which a step uses it */
+#define H261B_FETCH_MAX (2048 * 1024)  /* bytes up to which a step uses it */
 int h261b_launch_fetch(void *dst0, const void *src0, int64_t bytes0, void *dst1, const void *src1, int64_t bytes1,
                        void *zero, int64_t zero_bytes, int32_t sm_count, void *stream);
 /* the picture QUANT of every session with rc (one thread per session) */

@@ -1182,27 +1182,33 @@ __device__ __forceinline__ BlockRow chroma_row(const StageBuf s, const h261b_ses
     return o;
 }
 
-/* frame-end denoise update by the session's last warp (mbgpu_kernels.cuh:478-503) */
+/* frame-end denoise update by the session's last warp (mbgpu_kernels.cuh:478-503).
+ * Every other warp has published, and this one has acquired their counts: it
+ * alone holds the state until the launch ends, so plain loads from L2, all in
+ * flight together, and stores do (one exchange after another was 2 us at the
+ * end of every launch). */
 __device__ __forceinline__ void denoise_frame_end(h261b_denoise_dev_t *dn, int lane)
 {
-    int32_t cnt0 = 0, cnt1 = 0;
-    if (lane == 0) {
-        cnt0 = atomicExch(&dn->count[0], 0);
-        cnt1 = atomicExch(&dn->count[1], 0);
+    const int32_t cnt0 = __ldcg(&dn->count[0]), cnt1 = __ldcg(&dn->count[1]), strength = dn->denoise;
+    int32_t n0[2], n1[2];
+#pragma unroll
+    for (int h = 0; h < 2; h++) {
+        n0[h] = __ldcg(&dn->noise[0][lane + 32 * h]);
+        n1[h] = __ldcg(&dn->noise[1][lane + 32 * h]);
     }
-    cnt0 = __shfl_sync(FULL, cnt0, 0);
-    cnt1 = __shfl_sync(FULL, cnt1, 0);
-    for (int p = lane; p < 64; p += 32) {
-        const int32_t n1 = atomicExch(&dn->noise[1][p], 0);
-        const int32_t n0 = atomicExch(&dn->noise[0][p], 0);
-        const int u = p & 7, v = p >> 3;
+#pragma unroll
+    for (int h = 0; h < 2; h++) {
+        const int p = lane + 32 * h, u = p & 7, v = p >> 3;
         /* the reference keeps Int32 offsets and loads them as UInt16 */
-        dn->offset[1][u][v] = (uint16_t)((cnt1 * dn->denoise + n1 / 2) / (n1 + 1));
-        dn->offset[0][u][v] = (uint16_t)((cnt0 * dn->denoise + n0 / 2) / (n0 + 1));
+        dn->offset[1][u][v] = (uint16_t)((cnt1 * strength + n1[h] / 2) / (n1[h] + 1));
+        dn->offset[0][u][v] = (uint16_t)((cnt0 * strength + n0[h] / 2) / (n0[h] + 1));
+        dn->noise[0][p] = dn->noise[1][p] = 0;
     }
-    __threadfence();
-    if (lane == 0)
-        atomicExch(&dn->ticket, 0u);
+    __syncwarp();   /* every lane has the counts */
+    if (lane == 0) {
+        dn->count[0] = dn->count[1] = 0;
+        dn->ticket = 0u;
+    }
 }
 
 /* publish a warp's statistics for a run of n MBs of one session and type,
