@@ -3,8 +3,9 @@
  * the sm_100a core.
  *
  * Same contract as src/gpu_device.cu: one process-global encoder, every
- * call synchronous on return, results in pinned host arrays owned by the
- * library, void returns.  What differs inside:
+ * call synchronous on return (an uploaded plane is the library's, a result is
+ * complete), results in pinned host arrays owned by the library, void
+ * returns.  What differs inside:
  *   - pictures live in plain device memory (packed planes) instead of
  *     cudaArray textures; every fetch of the reference is in bounds, so
  *     plain loads read the same pixels (gpu_device.cu:90-145);
@@ -45,6 +46,13 @@ struct Compat {
     h261b_denoise_dev_t *dn_dev = nullptr;
     h261_mb_mode_decision_t *md_dev = nullptr;
     int status = H261B_OK;
+    /* pinned: the planes on their way up (current, then reference picture)
+     * and the caller's mode decisions, which the kernel reads from there */
+    uint8_t *stage = nullptr;
+    bool staged[6] = {};          /* copies of the planes that may be in flight */
+    h261_mb_mode_decision_t *md_host = nullptr;
+    int32_t md_n = 0;
+    int32_t sms = 0;
 };
 
 Compat g;
@@ -123,12 +131,24 @@ void base_desc(h261b_session_dev_t &d)
     d.me_mode = g.me_mode;
 }
 
-void upload(const char *where, uint8_t *pic, size_t off, const uint8_t *data, int32_t w, int32_t h,
-            int32_t ew, int32_t eh)
+/* the stream's work is done, the staging free */
+cudaError_t drain()
+{
+    memset(g.staged, 0, sizeof(g.staged));
+    return cudaStreamSynchronize(g.stream);
+}
+
+/* One plane of the current (which = 0) or reference (1) picture.  The bytes are
+ * the library's when the call returns: copied into pinned memory, from where
+ * they go up in the order of the stream the kernels run on (a pageable copy
+ * would wait for the device six times a picture). */
+void upload(const char *where, int which, int plane, const uint8_t *data, int32_t w, int32_t h, int32_t ew,
+            int32_t eh)
 {
     if (!ensure_ready(where))
         return;
-    if (!pic) {
+    uint8_t *pic = which ? g.ref : g.cur;
+    if (!pic || !g.stage) {
         fail_arg(where, "h261_gpu_device_init_textures has not been called");
         return;
     }
@@ -136,8 +156,18 @@ void upload(const char *where, uint8_t *pic, size_t off, const uint8_t *data, in
         fail_arg(where, "plane size does not match the initialised picture");
         return;
     }
-    CK(where, cudaMemcpy(pic + off, data, (size_t)w * h, cudaMemcpyHostToDevice));
+    const size_t off = plane == 0 ? g.lay.off_y : plane == 1 ? g.lay.off_cb : g.lay.off_cr;
+    bool &busy = g.staged[3 * which + plane];
+    if (busy)
+        CK(where, drain());
+    uint8_t *from = g.stage + (which ? g.lay.bytes : 0) + off;
+    memcpy(from, data, (size_t)w * h);
+    busy = true;
+    CK(where, cudaMemcpyAsync(pic + off, from, (size_t)w * h, cudaMemcpyHostToDevice, g.stream));
 }
+
+/* whether a launch of the boundary takes a team of warps per MB */
+bool team_size(int32_t nmb) { return nmb <= H261B_TEAM_PER_SM * g.sms; }
 
 } // namespace
 
@@ -161,6 +191,7 @@ extern "C" void h261_gpu_init(void)
     }
     if (!g.desc_dev)
         CK("h261_gpu_init", cudaMalloc(&g.desc_dev, sizeof(h261b_session_dev_t)));
+    CK("h261_gpu_init", cudaDeviceGetAttribute(&g.sms, cudaDevAttrMultiProcessorCount, g.device));
     g.ready = true;
 }
 
@@ -183,10 +214,16 @@ extern "C" void h261_gpu_device_init_textures(int32_t w, int32_t h)
     CK(where, cudaMemset(g.cur, 0, g.lay.bytes));
     CK(where, cudaMemset(g.ref, 0, g.lay.bytes));
     CK(where, cudaMemset(g.rec, 0, g.lay.bytes));
+    CK(where, cudaMallocHost(&g.stage, 2 * g.lay.bytes));
+    CK(where, cudaDeviceSynchronize());   /* cleared before the stream's copies */
 }
 
 extern "C" void h261_gpu_device_deinit_textures(void)
 {
+    if (g.stream)
+        drain();   /* planes on their way up */
+    cudaFreeHost(g.stage);
+    g.stage = nullptr;
     cudaFree(g.cur);
     cudaFree(g.ref);
     cudaFree(g.rec);
@@ -195,27 +232,27 @@ extern "C" void h261_gpu_device_deinit_textures(void)
 
 extern "C" void h261_gpu_device_set_current(uint8_t *d, int32_t w, int32_t h)
 {
-    upload("h261_gpu_device_set_current", g.cur, g.lay.off_y, d, w, h, g.w, g.h);
+    upload("h261_gpu_device_set_current", 0, 0, d, w, h, g.w, g.h);
 }
 extern "C" void h261_gpu_device_set_current_chroma_cb(uint8_t *d, int32_t w, int32_t h)
 {
-    upload("h261_gpu_device_set_current_chroma_cb", g.cur, g.lay.off_cb, d, w, h, g.w / 2, g.h / 2);
+    upload("h261_gpu_device_set_current_chroma_cb", 0, 1, d, w, h, g.w / 2, g.h / 2);
 }
 extern "C" void h261_gpu_device_set_current_chroma_cr(uint8_t *d, int32_t w, int32_t h)
 {
-    upload("h261_gpu_device_set_current_chroma_cr", g.cur, g.lay.off_cr, d, w, h, g.w / 2, g.h / 2);
+    upload("h261_gpu_device_set_current_chroma_cr", 0, 2, d, w, h, g.w / 2, g.h / 2);
 }
 extern "C" void h261_gpu_device_set_reference(uint8_t *d, int32_t w, int32_t h)
 {
-    upload("h261_gpu_device_set_reference", g.ref, g.lay.off_y, d, w, h, g.w, g.h);
+    upload("h261_gpu_device_set_reference", 1, 0, d, w, h, g.w, g.h);
 }
 extern "C" void h261_gpu_device_set_reference_chroma_cb(uint8_t *d, int32_t w, int32_t h)
 {
-    upload("h261_gpu_device_set_reference_chroma_cb", g.ref, g.lay.off_cb, d, w, h, g.w / 2, g.h / 2);
+    upload("h261_gpu_device_set_reference_chroma_cb", 1, 1, d, w, h, g.w / 2, g.h / 2);
 }
 extern "C" void h261_gpu_device_set_reference_chroma_cr(uint8_t *d, int32_t w, int32_t h)
 {
-    upload("h261_gpu_device_set_reference_chroma_cr", g.ref, g.lay.off_cr, d, w, h, g.w / 2, g.h / 2);
+    upload("h261_gpu_device_set_reference_chroma_cr", 1, 2, d, w, h, g.w / 2, g.h / 2);
 }
 
 extern "C" void h261_gpu_device_init_me(me_gpu_t **pps, int32_t w, int32_t h)
@@ -265,6 +302,7 @@ extern "C" void h261_gpu_device_init_me(me_gpu_t **pps, int32_t w, int32_t h)
                          cudaMemcpyHostToDevice));
     CK(where, cudaMemset(s->ps_candidate_vector_device, 0, sizeof(me_gpu_mv_t) * n));
     CK(where, cudaMemset(s->prgs_macroblocks_device, 0, sizeof(me_gpu_mb_t) * n));
+    CK(where, cudaDeviceSynchronize());   /* cleared before the stream's kernels */
     *pps = s;
 }
 
@@ -300,28 +338,29 @@ extern "C" void h261_gpu_device_me(me_gpu_t *s)
     h261b_session_dev_t d;
     base_desc(d);
     d.frame_type = H261B_FRAME_TYPE_INTER;
+    /* the kernel leaves the results on the device and on the host, and the
+     * final vector in the starting-vector array and, as the reference's copy
+     * does, in the candidate one (gpu_device.cu:403-422) */
     d.me_out = s->prgs_macroblocks_device;
-    CK(where, cudaMemcpyAsync(g.desc_dev, &d, sizeof(d), cudaMemcpyHostToDevice, g.stream));
-    int rc = h261b_launch_step(g.desc_dev, g.work_dev, n,
-                               H261B_PHASE_ME | H261B_ABI_OUT | (g.me_mode ? H261B_LAUNCH_ME_FULL : 0) |
-                                   (g.fmad ? H261B_FMAD_BIT : 0),
-                               4, 0, nullptr, g.stream);
+    d.me_host = s->prgs_macroblocks_result;
+    d.start_mv = s->ps_starting_vector_device;
+    d.cand_mv = s->ps_candidate_vector_device;
+    const int phases = H261B_PHASE_ME | H261B_ABI_OUT | (g.me_mode ? H261B_LAUNCH_ME_FULL : 0) |
+                       (g.fmad ? H261B_FMAD_BIT : 0);
+    int rc;
+    if (team_size(n)) {
+        rc = h261b_launch_team_picture(&d, phases, g.stream);
+    } else {
+        CK(where, cudaMemcpyAsync(g.desc_dev, &d, sizeof(d), cudaMemcpyHostToDevice, g.stream));
+        rc = h261b_launch_step(g.desc_dev, g.work_dev, n, phases, 4, 0, nullptr, g.stream);
+    }
     if (rc) {
         fail(where, (cudaError_t)rc);
         return;
     }
-    CK(where, cudaMemcpyAsync(s->prgs_macroblocks_result, s->prgs_macroblocks_device, sizeof(me_gpu_mb_t) * n,
-                              cudaMemcpyDeviceToHost, g.stream));
-    CK(where, cudaStreamSynchronize(g.stream));
-    /* the reference leaves the final vector in the starting-vector arrays
-     * and copies it to the candidate ones (gpu_device.cu:403-422) */
+    CK(where, drain());
     for (int32_t i = 0; i < n; i++)
         s->ps_starting_vector_host[i] = s->prgs_macroblocks_result[i].s_16x16_mv;
-    CK(where, cudaMemcpyAsync(s->ps_starting_vector_device, s->ps_starting_vector_host, sizeof(me_gpu_mv_t) * n,
-                              cudaMemcpyHostToDevice, g.stream));
-    CK(where, cudaMemcpyAsync(s->ps_candidate_vector_device, s->ps_starting_vector_device,
-                              sizeof(me_gpu_mv_t) * n, cudaMemcpyDeviceToDevice, g.stream));
-    CK(where, cudaStreamSynchronize(g.stream));
 }
 
 extern "C" void h261_init_macroblocks(h261_macroblocks_t **pps, int32_t w, int32_t h, int32_t denoise)
@@ -376,6 +415,7 @@ extern "C" void h261_init_macroblocks(h261_macroblocks_t **pps, int32_t w, int32
         cudaFree(g.dn_dev);
     CK(where, cudaMalloc(&g.dn_dev, sizeof(dn0)));
     CK(where, cudaMemcpy(g.dn_dev, &dn0, sizeof(dn0), cudaMemcpyHostToDevice));
+    CK(where, cudaDeviceSynchronize());   /* in place before the stream's kernels */
     s->ps_denoise_device = (h261_dct_denoise_t *)g.dn_dev;
     if (g.md_dev)
         cudaFree(g.md_dev);
@@ -423,8 +463,10 @@ extern "C" void h261_deinit_macroblocks(h261_macroblocks_t *s)
     cudaFreeHost(s);
     cudaFree(g.dn_dev);
     cudaFree(g.md_dev);
+    cudaFreeHost(g.md_host);
     g.dn_dev = nullptr;
-    g.md_dev = nullptr;
+    g.md_dev = g.md_host = nullptr;
+    g.md_n = 0;
 }
 
 extern "C" void h261_gpu_device_encode_macroblocks(h261_context_t *ctx)
@@ -473,27 +515,40 @@ extern "C" void h261_gpu_device_encode_macroblocks(h261_context_t *ctx)
         s->pi_mb_mv_y_host[i] = m.i_mv_y;
         s->pi_mb_quant_host[i] = q < 1 ? 1 : q > 31 ? 31 : q;
     }
-    CK(where, cudaMemcpyAsync(g.md_dev, md->prgs_mb, sizeof(h261_mb_mode_decision_t) * n, cudaMemcpyHostToDevice,
-                              g.stream));
+    if (g.md_n < n) {
+        cudaFreeHost(g.md_host);
+        g.md_host = nullptr;
+        g.md_n = 0;
+        CK(where, cudaMallocHost(&g.md_host, sizeof(h261_mb_mode_decision_t) * n));
+        g.md_n = n;
+    }
+    memcpy(g.md_host, md->prgs_mb, sizeof(h261_mb_mode_decision_t) * n);
     h261b_session_dev_t d;
     base_desc(d);
     d.quant = pq;
     d.dn = g.dn_dev;
-    d.md_in = g.md_dev;
     d.abi_out = s->ps_macroblocks_device;
     d.frame_type = ctx->s_picture.i_frame_type;
-    CK(where, cudaMemcpyAsync(g.desc_dev, &d, sizeof(d), cudaMemcpyHostToDevice, g.stream));
-    int rc = h261b_launch_step(g.desc_dev, g.work_dev, n,
-                               H261B_PHASE_ENCDEC | H261B_ABI_OUT | (g.me_mode ? H261B_LAUNCH_ME_FULL : 0) |
-                                   (g.fmad ? H261B_FMAD_BIT : 0),
-                               4, 0, nullptr, g.stream);
+    const int phases = H261B_PHASE_ENCDEC | H261B_ABI_OUT | (g.me_mode ? H261B_LAUNCH_ME_FULL : 0) |
+                       (g.fmad ? H261B_FMAD_BIT : 0);
+    int rc;
+    if (team_size(n)) {
+        d.md_in = g.md_host;
+        rc = h261b_launch_team_picture(&d, phases, g.stream);
+    } else {
+        CK(where, cudaMemcpyAsync(g.md_dev, g.md_host, sizeof(h261_mb_mode_decision_t) * n, cudaMemcpyHostToDevice,
+                                  g.stream));
+        d.md_in = g.md_dev;
+        CK(where, cudaMemcpyAsync(g.desc_dev, &d, sizeof(d), cudaMemcpyHostToDevice, g.stream));
+        rc = h261b_launch_step(g.desc_dev, g.work_dev, n, phases, 4, 0, nullptr, g.stream);
+    }
     if (rc) {
         fail(where, (cudaError_t)rc);
         return;
     }
     CK(where, cudaMemcpyAsync(s->ps_macroblocks, s->ps_macroblocks_device, sizeof(h261_macroblock_t) * n,
                               cudaMemcpyDeviceToHost, g.stream));
-    CK(where, cudaStreamSynchronize(g.stream));
+    CK(where, drain());
 }
 
 extern "C" void h261_gpu_device_decode_macroblocks(h261_context_t *ctx)

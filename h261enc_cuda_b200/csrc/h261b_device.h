@@ -139,6 +139,11 @@ typedef struct {
      * sums when it finishes the picture (pinned host memory), or NULL */
     h261b_mb_info_t *host_info;
     unsigned long long *host_ssd;
+    /* the gpu_device.h boundary: the ME results once more in pinned host
+     * memory, and the final vectors in the reference's two device arrays; any
+     * may be NULL */
+    me_gpu_mb_t *me_host;
+    me_gpu_mv_t *start_mv, *cand_mv;
 } h261b_session_dev_t;
 
 /* coefficient bits of one MB at most: six blocks of an 8-bit DC or a first
@@ -176,7 +181,8 @@ typedef struct {
 #define H261B_STAGE_SHORT   0x20000
 /*   bit 18       the exhaustive +-15 search (the sessions' me_mode 1)
  *   bit 19       the launch may write the reference-layout outputs
- *                (abi_out, me_out, stage1_out: the gpu_device.h boundary) */
+ *                (abi_out, me_out, me_host, start_mv, cand_mv, stage1_out: the
+ *                gpu_device.h boundary) */
 /*   bit 20       sessions with bits_out: each MB's coefficient bit string is
  *                made by the warp that encodes it */
 #define H261B_CODE_INLINE   0x100000
@@ -201,7 +207,8 @@ int h261b_launch_step(const h261b_session_dev_t *sessions_dev, const uint32_t *w
                       int32_t *sched_dev, void *stream);
 int h261b_set_quant_table(void);
 /* a team launch over one picture whose descriptor (host memory) travels with
- * the launch; nothing is counted in its mbs_done */
+ * the launch; nothing is counted in its mbs_done.  With H261B_ABI_OUT for one
+ * of the boundary's two calls: the ME phase, or ENCDEC from md_in */
 int h261b_launch_team_picture(const h261b_session_dev_t *session, int32_t phases, void *stream);
 /* copy two spans from pinned host memory into device memory and zero a third
  * by a kernel (all 16-byte aligned, sizes in bytes, multiples of 16) */

@@ -872,6 +872,32 @@ __device__ __forceinline__ void motion_estimate(const StageBuf s, const h261b_se
     res.s_16x16_mv.i8_my = (int8_t)vy;
 }
 
+/* a MB's ME results where the gpu_device.h boundary wants them */
+__device__ __forceinline__ void me_results_out(const h261b_session_dev_t &S, int mb, const me_gpu_mb_t &me)
+{
+    if (S.me_out)
+        S.me_out[mb] = me;
+    if (S.me_host)
+        S.me_host[mb] = me;
+    if (S.start_mv)
+        S.start_mv[mb] = S.cand_mv[mb] = me.s_16x16_mv;
+}
+
+/* a coded MB's record in the reference's layout (without its levels) */
+__device__ __forceinline__ void abi_record_out(h261_macroblock_t *o, const MbDecision &m, int flags, int quant,
+                                               uint32_t cbp, int mbx, int mby)
+{
+    o->i_macroblock_address = 0;
+    o->i_macroblock_type = m.type;
+    o->i_macroblock_type_flags = flags;
+    o->i_macroblock_quant = quant;
+    o->rgi_mv[0] = m.mvx;
+    o->rgi_mv[1] = m.mvy;
+    o->i_coded_block_pattern = (int32_t)cbp;
+    o->i_mb_x = mbx * 16;
+    o->i_mb_y = mby * 16;
+}
+
 /* h261_moded.c:53-95 */
 __device__ __forceinline__ MbDecision mode_decide(const me_gpu_mb_t &g, int frame_type)
 {
@@ -1445,8 +1471,7 @@ __global__ void __launch_bounds__(256, KIND == KIND_SEARCH ? H261B_SEARCH_MIN_BL
             (void)H261B_CHECK(S.me_mode == (FULL_SEARCH ? 1 : 0), CHK_WORK_ITEM, S.me_mode);
             motion_estimate<FULL_SEARCH>(b, S, mbx, mby, lane, me, s1x, s1y);
             if (ABI && lane == 0) {
-                if (S.me_out)
-                    S.me_out[mb] = me;
+                me_results_out(S, mb, me);
                 if (S.stage1_out) {
                     S.stage1_out[mb].i8_mx = s1x;
                     S.stage1_out[mb].i8_my = s1y;
@@ -1535,18 +1560,8 @@ __global__ void __launch_bounds__(256, KIND == KIND_SEARCH ? H261B_SEARCH_MIN_BL
                 }
             }
             if (lane == 0) {
-                if (ABI && S.abi_out) {
-                    h261_macroblock_t *o = &S.abi_out[mb];
-                    o->i_macroblock_address = 0;
-                    o->i_macroblock_type = m.type;
-                    o->i_macroblock_type_flags = flags;
-                    o->i_macroblock_quant = quant;
-                    o->rgi_mv[0] = m.mvx;
-                    o->rgi_mv[1] = m.mvy;
-                    o->i_coded_block_pattern = (int32_t)cbp;
-                    o->i_mb_x = mbx * 16;
-                    o->i_mb_y = mby * 16;
-                }
+                if (ABI && S.abi_out)
+                    abi_record_out(&S.abi_out[mb], m, flags, quant, cbp, mbx, mby);
                 if (S.info_out) {
                     h261b_mb_info_t inf;
                     inf.type = (int16_t)m.type;
@@ -1721,7 +1736,7 @@ __device__ __forceinline__ void team_search(TeamSmem &sm, const StageBuf s, cons
 
 /* one MB of picture S.  phases as in step_kernel, every warp of the CTA
  * together; mbs_done may be NULL. */
-template <int FMAD, bool FULL_SEARCH, bool CODE>
+template <int FMAD, bool FULL_SEARCH, bool ABI, bool CODE>
 __device__ __forceinline__ void team_mb(TeamSmem &sm, const h261b_session_dev_t &S, int mb, int phases,
                                         int32_t *mbs_done)
 {
@@ -1781,6 +1796,8 @@ __device__ __forceinline__ void team_mb(TeamSmem &sm, const h261b_session_dev_t 
         me.i_16x16_cost = sm.cost[0];
         me.i_16x16_filter_cost = sm.cost[1];
         me.i_intra_cost = sm.cost[2];
+        if (ABI && tid == 0)
+            me_results_out(S, mb, me);
     } else if (phases & H261B_PHASE_MD) {
         me.i_intra_cost = intra_cost(b, lane);   /* every warp: no exchange */
     }
@@ -1801,6 +1818,8 @@ __device__ __forceinline__ void team_mb(TeamSmem &sm, const h261b_session_dev_t 
             S.md_out[mb] = o;
         }
     } else {
+        if (ABI && !enc)
+            return;   /* the boundary's motion estimation alone */
         const h261_mb_mode_decision_t &d = S.md_in[mb];
         m.type = d.i_mb_type;
         m.flags = d.i_mb_flags;
@@ -1829,7 +1848,7 @@ __device__ __forceinline__ void team_mb(TeamSmem &sm, const h261b_session_dev_t 
             noise[v] = 0.0f;
         uint32_t ssd = 0;
         const BlockRow row = warp == 0 ? luma_row(b, S, mbx, mby, m, lane) : chroma_row(b, S, mbx, mby, m, ref, lane);
-        const uint32_t cbp = encdec_pass<FMAD, false, CODE>(sm.t[warp], sm.vlc.cm, row, S, mb, m, quant, offw,
+        const uint32_t cbp = encdec_pass<FMAD, ABI, CODE>(sm.t[warp], sm.vlc.cm, row, S, mb, m, quant, offw,
                                                             warp == 0, lane, fwd_c, inv_c, noise, ssd);
         if (lane == 0)
             sm.cbp[warp] = cbp;
@@ -1860,6 +1879,8 @@ __device__ __forceinline__ void team_mb(TeamSmem &sm, const h261b_session_dev_t 
             }
         }
         if (lane == 0) {
+            if (ABI && S.abi_out)
+                abi_record_out(&S.abi_out[mb], m, flags, quant, cbp, mbx, mby);
             if (S.info_out) {
                 h261b_mb_info_t inf;
                 inf.type = (int16_t)m.type;
@@ -1909,17 +1930,17 @@ __global__ void __launch_bounds__(TEAM_THREADS, 4)
     team_begin<CODE>(sm);
     const uint32_t item = work[blockIdx.x];
     const h261b_session_dev_t &S = sessions[item >> 12];
-    team_mb<FMAD, FULL_SEARCH, CODE>(sm, S, (int)(item & 0xFFFu), phases, const_cast<int32_t *>(&S.mbs_done));
+    team_mb<FMAD, FULL_SEARCH, false, CODE>(sm, S, (int)(item & 0xFFFu), phases, const_cast<int32_t *>(&S.mbs_done));
 }
 
 /* MB blockIdx.x of one picture whose descriptor comes with the launch */
-template <int FMAD, bool FULL_SEARCH>
+template <int FMAD, bool FULL_SEARCH, bool ABI>
 __global__ void __launch_bounds__(TEAM_THREADS, 4)
     team_picture_kernel(const __grid_constant__ h261b_session_dev_t S, int32_t phases)
 {
     __shared__ TeamSmem sm;
     team_begin<false>(sm);
-    team_mb<FMAD, FULL_SEARCH, false>(sm, S, (int)blockIdx.x, phases, nullptr);
+    team_mb<FMAD, FULL_SEARCH, ABI, false>(sm, S, (int)blockIdx.x, phases, nullptr);
 }
 
 } // namespace
@@ -2121,12 +2142,21 @@ extern "C" int h261b_launch_step(const h261b_session_dev_t *sessions_dev, const 
     return (int)cudaLaunchKernelEx(&cfg, fn, sessions_dev, work_dev, n_work, chunk, ph, sched_dev);
 }
 
+namespace {
+
+template <int FMAD, bool ABI>
+auto team_picture_fn(bool full)
+{
+    return full ? team_picture_kernel<FMAD, true, ABI> : team_picture_kernel<FMAD, false, ABI>;
+}
+
+} // namespace
+
 extern "C" int h261b_launch_team_picture(const h261b_session_dev_t *session, int32_t phases, void *stream)
 {
-    const int fmad = (phases >> 8) & 1;
-    const bool full = (phases & H261B_LAUNCH_ME_FULL) != 0;
-    auto fn = fmad ? (full ? team_picture_kernel<1, true> : team_picture_kernel<1, false>)
-                   : (full ? team_picture_kernel<0, true> : team_picture_kernel<0, false>);
+    const bool fmad = (phases & H261B_FMAD_BIT) != 0, full = (phases & H261B_LAUNCH_ME_FULL) != 0;
+    const auto fn = (phases & H261B_ABI_OUT) ? (fmad ? team_picture_fn<1, true>(full) : team_picture_fn<0, true>(full))
+                                             : (fmad ? team_picture_fn<1, false>(full) : team_picture_fn<0, false>(full));
     fn<<<session->mbw * session->mbh, TEAM_THREADS, 0, (cudaStream_t)stream>>>(*session, phases & 0xFF);
     return (int)cudaGetLastError();
 }
