@@ -364,6 +364,7 @@ struct h261b_engine_s {
     } work_list[NSLOT];
     int64_t last_h2d = 0, last_d2h = 0;  /* bytes copied by the last step */
     HostArena bits[NSLOT];     /* pictures written by the bitstream kernel */
+    HostArena recon_host;      /* a reconstruction on its way to the caller */
     size_t bits_want = 0;      /* capacity the arenas grow to              */
     /* slots of closed sessions, returned to the pool once the last step
      * that may use them (second field) has completed */
@@ -704,6 +705,7 @@ extern "C" int h261b_engine_destroy(h261b_engine_t *e)
         cudaEventDestroy(e->fork_ev[p]);
         cudaEventDestroy(e->join_ev[p]);
     }
+    e->recon_host.release();
     if (e->sched_dev)
         cudaFree(e->sched_dev);
     delete e;
@@ -1784,11 +1786,17 @@ extern "C" int h261b_session_recon(h261b_engine_t *e, int32_t id, uint8_t *y, ui
     int rc = sync_all(e);
     if (rc)
         return rc;
-    const uint8_t *rec = s->rec[s->rec_cur];
+    /* one copy of the picture into pinned memory: a copy per plane straight to
+     * the caller's pageable memory waits for the device three times */
+    if ((rc = e->recon_host.reserve(s->lay.bytes)))
+        return rc;
+    uint8_t *pic = e->recon_host.host;
     const size_t ny = (size_t)s->w * s->h, nc = ny / 4;
-    H261B_CUDA_TRY(cudaMemcpy(y, rec + s->lay.off_y, ny, cudaMemcpyDeviceToHost));
-    H261B_CUDA_TRY(cudaMemcpy(cb, rec + s->lay.off_cb, nc, cudaMemcpyDeviceToHost));
-    H261B_CUDA_TRY(cudaMemcpy(cr, rec + s->lay.off_cr, nc, cudaMemcpyDeviceToHost));
+    H261B_CUDA_TRY(cudaMemcpyAsync(pic, s->rec[s->rec_cur], s->lay.bytes, cudaMemcpyDeviceToHost, e->stream[0]));
+    H261B_CUDA_TRY(cudaStreamSynchronize(e->stream[0]));
+    memcpy(y, pic + s->lay.off_y, ny);
+    memcpy(cb, pic + s->lay.off_cb, nc);
+    memcpy(cr, pic + s->lay.off_cr, nc);
     return H261B_OK;
 }
 
