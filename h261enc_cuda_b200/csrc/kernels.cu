@@ -2116,6 +2116,10 @@ extern "C" int h261b_launch_step(const h261b_session_dev_t *sessions_dev, const 
     /* one wave of resident CTAs */
     int ctas = max_ctas > 0 ? max_ctas : nsm * per_sm;
     int chunk;
+    /* a MB a warp at most: nothing to balance, and no draw (an atomic's round
+     * trip before the first MB and one more after the last) */
+    if (n_work <= (long long)ctas * warps_per_cta)
+        sched_dev = nullptr;
     if (sched_dev) {
         /* static runs of all but about `tail` items per warp, the rest drawn
          * from the scheduler (tail_code: tail + 1, 0 for the default 2) */
