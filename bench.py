@@ -744,8 +744,8 @@ def ours(args, world, rank, local, dist):
         # the committed ncu figure is for batch64 in reference mode
         "issue_roofline": (issue_roofline(mb_per_step, mean_kernel, local, clk.summary())
                            if args.workload == "batch64" and not me_mode else None),
-        # encode (search + encode when split), codes, layout, pack (which also copies)
-        "gpu_launches": (5 if plan["kernel_split"] == 2 else 4) * args.steps,
+        # fetch (descriptors), encode (search + encode when split), codes, layout, pack (which also copies)
+        "gpu_launches": (6 if plan["kernel_split"] == 2 else 5) * args.steps,
         "graphs": {"captures": graph_caps, "replays": graph_reps,
                    "note": "steps whose launch signature repeats replay a captured CUDA graph"},
         "launch_plan": {"plan": plan, "tuning_ms": [[p["warps_per_cta"], p["kernel_split"], p["tail_items"],
