@@ -7,15 +7,16 @@
  * call cudaMalloc.  Queued source pictures sit in a pinned upload arena
  * (copied there by h261b_session_submit, or written there directly by the
  * caller through h261b_session_input); a step moves the whole arena with
- * one copy, runs one launch over the flat (session, MB) work list, and
- * brings the compact results of all sessions back with one copy.
+ * one copy (with a kernel that reads it, where it is small) and runs one
+ * launch over the flat (session, MB) work list; the kernels write the
+ * compact results of all sessions into pinned host memory.
  *
  * Pipelining: steps rotate over NSLOT (3) slots, each with its CUDA stream
- * and its set of arenas.  Within a step the order is upload -> kernel ->
- * download; across steps only the kernels are ordered (step k+1's kernel
+ * and its set of arenas.  Within a step the order is upload -> encode ->
+ * bitstreams; across steps only the encode kernels are ordered (step k+1's
  * waits for step k's, whose reconstructions are its references), so step
- * k+1's upload overlaps step k's kernel and step k's download overlaps step
- * k+1's kernel.  Results of step k stay readable until step k+3 is issued,
+ * k+1's upload overlaps step k's kernels and step k's bitstreams overlap
+ * step k+1's encode.  Results of step k stay readable until step k+3 is issued,
  * so a caller can issue step k+1 while it has still to read step k-1.
  *
  * Tuning: when warps_per_cta is 0 the first steps try each launch shape on
@@ -377,8 +378,9 @@ struct h261b_engine_s {
     std::unique_ptr<CopyPool> copier;   /* batched submissions */
     std::vector<CopyJob> copy_jobs;
 
-    /* graph replay of steps (use_graphs) */
-    StepGraph graph[NSLOT];
+    /* graph replay of steps (use_graphs): a slot's steps that keep their work
+     * list, and those that upload it */
+    StepGraph graph[NSLOT][2];
     bool graphs_off = false;
     int64_t graph_captures = 0, graph_replays = 0;
 
@@ -686,7 +688,8 @@ extern "C" int h261b_engine_destroy(h261b_engine_t *e)
         if (e->stream[p])
             cudaStreamSynchronize(e->stream[p]);
     for (int p = 0; p < NSLOT; p++) {
-        e->graph[p].reset();
+        e->graph[p][0].reset();
+        e->graph[p][1].reset();
         e->upload[p].release();
         e->results[p].release();
         e->desc[p].release();
@@ -1389,7 +1392,8 @@ extern "C" int h261b_engine_step(h261b_engine_t *e)
         }
     }
     cudaStream_t st = e->stream[p];
-    const size_t desc_bytes = wl.uploaded ? work_off : align_up(work_off + (size_t)n_work * sizeof(uint32_t), 16);
+    const bool list_up = !wl.uploaded;
+    const size_t desc_bytes = !list_up ? work_off : align_up(work_off + (size_t)n_work * sizeof(uint32_t), 16);
     wl.uploaded = false;   /* until this step's launches are issued */
     e->copier->join();   /* pictures of h261b_engine_submit_batch_async */
     LaunchPlan plan;
@@ -1560,13 +1564,17 @@ extern "C" int h261b_engine_step(h261b_engine_t *e)
      * shape) replay one CUDA graph per slot: the descriptor and work-list
      * contents differ, but they are data in pinned memory that the graph's
      * upload copies.  A signature is captured the second time in a row it
-     * comes on its slot.  Tuning steps, an engine's first step and engines
+     * comes on its slot.  Steps that upload the work list have a graph of
+     * their own, so that sessions which come and go, and take the list with
+     * them every few steps, do not cost a capture (about 1 ms) each time: 64
+     * streams of 30 to 300 pictures, end to end, 64 M MB/s with one graph a
+     * slot.  Tuning steps, an engine's first step and engines
      * with use_graphs = 0 launch directly. */
     const StepKey key = { dm.host, dm.dev, um.host, um.dev, rm.host, rm.dev, bits_dev_or_null(e, p, n_bits),
                           n_bits ? e->bits[p].cap : 0, desc_off, work_off, desc_bytes, upload_bytes, ssd_base,
                           d2h, (int64_t)n, n_work, rc_begin, n_rc, (n_ssd ? 1 : 0) | (direct ? 2 : 0), warps, ctas, phases,
                           (int32_t)std::min<int64_t>(id, NSLOT - 1) };
-    StepGraph &gr = e->graph[p];
+    StepGraph &gr = e->graph[p][list_up ? 1 : 0];
     const bool repeated = gr.has_last_direct && gr.last_direct == key;
     const bool capturable = e->cfg.use_graphs && !e->graphs_off && !tuning && id > 0;
     if (capturable && !(gr.exec && gr.key == key) && !repeated) {

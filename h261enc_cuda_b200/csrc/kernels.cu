@@ -36,7 +36,9 @@
  * Denoise statistics are summed per warp over its run of MBs of one session
  * and published when the session changes; the warp whose publication
  * completes a session's frame (a ticket counting MBs) turns the statistics
- * into the next frame's offsets (:478-503).  No warp waits on another.
+ * into the next frame's offsets (:478-503).  No warp waits on another, but
+ * for the teams of four warps per macroblock of small launches
+ * (team_kernel), which share each step's work and meet at CTA barriers.
  */
 #include <cuda_runtime.h>
 #include <stdint.h>

@@ -7,11 +7,11 @@
  *   2. this batched engine: many independent encode sessions of mixed size
  *      and QUANT share one device; each h261b_engine_step() encodes the next
  *      picture of every session that has one queued, in one launch over a
- *      flat macroblock work list.  Source pictures go up
- *      in one host-to-device copy per step, compact results come back in one
- *      copy, reconstructions stay in HBM as the next reference.  Steps
- *      alternate between two streams so that one step's copies overlap the
- *      neighbouring steps' kernels.
+ *      flat macroblock work list.  Source pictures go up in one transfer per
+ *      step, the kernels write the compact results into pinned host memory,
+ *      reconstructions stay in HBM as the next reference.  Steps rotate over
+ *      three streams so that one step's transfers overlap the neighbouring
+ *      steps' kernels.
  *
  * All functions return H261B_OK (0) or a negative status; the text of the
  * last failure on the calling thread is available from h261b_last_error().

@@ -48,3 +48,32 @@ def test_changing_sessions(gpu, graphs):
                 off[k] += sizes[at[k]]
                 at[k] += 1
         assert e.step() == 0   # nothing queued
+
+
+def test_changing_sessions_do_not_capture_again(gpu):
+    """Streams of a few pictures that end and begin keep the step's shape; their steps replay the slots' graphs (at
+    most two a slot: with the work list's upload and without), as steps of unchanged sessions do."""
+    rng = np.random.default_rng(5)
+    clips = {s: synth.clip(2, *s, 77, 4) for s in (Q, C)}
+    with Engine(max_sessions=16) as e:
+        live = [(e.open(*s, 10, bitstream=1), s) for s in (Q, C, Q, Q, C, Q)]
+
+        def steps(k, churn):
+            for t in range(k):
+                if churn and t % 4 == 0:
+                    # a stream of each size ends and its successor begins, in the other's slot
+                    for s in (Q, C):
+                        i = int(rng.choice([j for j, (_, z) in enumerate(live) if z == s]))
+                        e.close(live.pop(i)[0])
+                    live.extend((e.open(*s, 10, bitstream=1), s) for s in ((C, Q) if rng.random() < 0.5 else (Q, C)))
+                for sid, s in live:
+                    e.submit_frame(sid, clips[s][t % 4])
+                assert e.step() == len(live)
+            e.sync()
+
+        steps(60, False)      # the plan's trial, and the graphs of unchanged sessions
+        before, _ = e.graph_stats()
+        steps(120, True)
+        captures, replays = e.graph_stats()
+    assert captures - before <= 2 * 3
+    assert replays >= 100
