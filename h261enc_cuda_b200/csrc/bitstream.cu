@@ -479,8 +479,8 @@ __global__ void __launch_bounds__(LAYOUT_THREADS) layout_kernel(const h261b_sess
 constexpr int PACK_DONE_MAX = 64;   /* pictures a CTA copies together at its end */
 
 /* a finished picture into the host arena by threads t0, t0 + nt, ..., with
- * its MB records and squared errors where the step wants them on the host,
- * and its picture record (bytes, offset, status, QUANT) by thread t0 */
+ * its squared errors where the step wants them on the host, and its picture
+ * record (bytes, offset, status, QUANT) by thread t0 */
 __device__ __forceinline__ void copy_picture(const h261b_session_dev_t &S, uint8_t *host_arena, int t0, int nt)
 {
     const int total = S.vlc_total[0];
@@ -494,19 +494,12 @@ __device__ __forceinline__ void copy_picture(const h261b_session_dev_t &S, uint8
             for (int c = 0; c < 3; c++)
                 S.host_ssd[c] = __ldcg(S.ssd_out + c);
     }
-    /* other SMs wrote the words and records: read them from L2 */
+    /* other SMs wrote the words: read them from L2 */
     const int units = off < 0 || !host_arena ? 0 : ((bytes + 15) & ~15) / 16;
     const uint4 *s4 = reinterpret_cast<const uint4 *>(S.bits_out);
     uint4 *d4 = reinterpret_cast<uint4 *>(host_arena + off);
     for (int i = t0; i < units; i += nt)
         d4[i] = __ldcg(s4 + i);
-    if (S.host_info) {
-        const uint4 *r4 = reinterpret_cast<const uint4 *>(S.info_out);
-        uint4 *h4 = reinterpret_cast<uint4 *>(S.host_info);
-        const int nmb = S.mbw * S.mbh;
-        for (int i = t0; i < nmb; i += nt)
-            h4[i] = __ldcg(r4 + i);
-    }
 }
 
 /* ---- fetch: a small step's uploads, read from pinned host memory.  Each
@@ -561,6 +554,20 @@ __global__ void __launch_bounds__(VLC_THREADS) pack_kernel(const h261b_session_d
     int lo, hi;
     warp_range(n_work, lo, hi);
     pdl_wait();   /* the layout kernel's positions */
+    /* The records of the CTA's MBs, complete since they were coded, go to the
+     * host now, by consecutive threads, and cross the bus while the CTA packs.
+     * From the CTA that finishes a picture, with its bytes, they ended the
+     * launch: encode end to the last picture 26.6 us for 13,464 MBs and 144
+     * for 101,376, against 23.5 and 120. */
+    const int cta_items = (n_work + (int)gridDim.x * VLC_WARPS - 1) / ((int)gridDim.x * VLC_WARPS) * VLC_WARPS;
+    const int cta_hi = min(((int)blockIdx.x + 1) * cta_items, n_work);
+    for (int w = (int)blockIdx.x * cta_items + (int)threadIdx.x; w < cta_hi; w += VLC_THREADS) {
+        const uint32_t item = work[w];
+        const h261b_session_dev_t &S = sessions[item >> 12];
+        if (S.host_info)
+            reinterpret_cast<uint4 *>(S.host_info)[item & 4095u] =
+                __ldcg(reinterpret_cast<const uint4 *>(S.info_out) + (item & 4095u));
+    }
     int run_s = -1, run_n = 0;
     /* the half-warp's finished MBs of picture run_s: published once it
      * moves on; the publication that completes the picture queues its copy */

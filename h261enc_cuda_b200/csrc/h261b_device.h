@@ -135,8 +135,9 @@ typedef struct {
      * take up a picture as soon as its count is complete, while the encode launch
      * still works on other pictures */
     int32_t mbs_done;
-    /* where the pack kernel copies the picture's records and squared-error
-     * sums when it finishes the picture (pinned host memory), or NULL */
+    /* where the pack kernel copies the picture's records as it starts and
+     * its squared-error sums when it finishes the picture (pinned host
+     * memory), or NULL */
     h261b_mb_info_t *host_info;
     unsigned long long *host_ssd;
     /* the gpu_device.h boundary: the ME results once more in pinned host
