@@ -101,6 +101,7 @@ __device__ __forceinline__ StageBuf stage_view(const uint32_t *wbuf, int k) { re
 constexpr size_t kSearchWarpBytes = sizeof(uint32_t) * WIN_ROWS * WIN_PITCH_W + 2 * sizeof(uint64_t);
 constexpr size_t kEncodeWarpBytes = offsetof(WarpSmem, vlc);
 static_assert(kEncodeWarpBytes % 16 == 0 && sizeof(WarpSmem) % 16 == 0, "warp shared layout");
+static_assert(alignof(WarpSmem) >= alignof(VlcTables), "the tables follow the warps' shared memory");
 static_assert(kSearchWarpBytes % 16 == 0 && offsetof(WarpSmem, t) == kSearchWarpBytes, "warp shared layout");
 
 /* what a launch of the step kernel does per MB */
@@ -1629,7 +1630,7 @@ constexpr int TEAM_WARPS = 4, TEAM_THREADS = 32 * TEAM_WARPS;
 
 struct TeamSmem {
     alignas(16) uint32_t buf[WIN_ROWS * WIN_PITCH_W];   /* buffer 0 of the one-warp layout */
-    float t[2][4][TB_BLOCK];                            /* luma, chroma                    */
+    alignas(16) float t[2][4][TB_BLOCK];                /* luma, chroma                    */
     VlcScratch vlc;
     VlcTables tables;
     uint32_t best[2][TEAM_WARPS];                       /* each warp's key, two stages     */

@@ -18,6 +18,7 @@
  * first. */
 #pragma once
 
+#include <cstddef>
 #include <cstdint>
 
 #include "h261b_device.h"
@@ -42,14 +43,15 @@ __host__ __device__ constexpr int zigzag_index(int v, int u)
  * same values the reference's src/h261_tables.c holds), in device memory so
  * that a CTA loads them with one coalesced access a thread; lanes look them
  * up at different places, which constant memory would serve one by one */
-struct VlcTables {
+struct alignas(16) VlcTables {
     /* TCOEFF without the sign bit, run 0..26 x level 0..15 (level 0 unused):
      * length << 8 | code; 0 = send with the 20-bit escape */
     uint16_t tc[27][16];
     /* column-major index (u * 8 + v) of the k-th coefficient sent */
     uint8_t cm[64];
 };
-static_assert(sizeof(VlcTables) % 16 == 0, "loaded as 16-byte words");
+static_assert(sizeof(VlcTables) % 16 == 0 && alignof(VlcTables) >= 16, "loaded as 16-byte words");
+static_assert(offsetof(VlcTables, cm) % 4 == 0, "read as 4-byte words");
 
 #define VLC(code, len) (uint16_t)(((len) << 8) | (code))
 constexpr VlcTables make_vlc_tables()
