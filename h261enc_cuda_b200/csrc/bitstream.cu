@@ -468,6 +468,10 @@ __global__ void __launch_bounds__(LAYOUT_THREADS) layout_kernel(const h261b_sess
         }
         S.vlc_total[2] = off;
         S.vlc_total[3] = 0;   /* MBs the pack kernel has finished */
+        /* the picture's QUANT, for its record: the rate control may choose the
+         * next picture's (in the next step, which waits for this kernel but
+         * not for pack) before pack writes this one's record */
+        S.vlc_total[4] = gq;
         /* the rate control learns the picture's size */
         if (S.rc && S.vlc_total[1] == 0)
             rc_update(*S.rc, S.frame_type, (int32_t)((total + 7) >> 3));
@@ -489,7 +493,7 @@ __device__ __forceinline__ void copy_picture(const h261b_session_dev_t &S, uint8
     const int off = st == 0 ? S.vlc_total[2] : -1;
     const int bytes = (total + 7) >> 3;
     if (t0 == 0) {
-        *S.pic_out = h261b_pic_info_t{ st == 0 ? bytes : 0, off, st, S.rc ? S.rc->picture_quant : S.quant };
+        *S.pic_out = h261b_pic_info_t{ st == 0 ? bytes : 0, off, st, S.vlc_total[4] };
         if (S.host_ssd)
             for (int c = 0; c < 3; c++)
                 S.host_ssd[c] = __ldcg(S.ssd_out + c);

@@ -121,7 +121,7 @@ typedef struct {
     int32_t *vlc_pos;             /* per MB: bit position in the picture     */
     uint32_t *vlc_plan;           /* per MB: header fields                   */
     int32_t *vlc_total;           /* [0] picture bits, [1] status, [2] host
-                                     arena offset, [3] MBs packed            */
+                                     arena offset, [3] MBs packed, [4] QUANT */
     /* CBR sessions: the step's first encode launch runs search and mode
      * decision (into md_out, costs summed into rc), the rate control picks
      * the picture QUANT, a second launch encodes (md_in = md_out) */
