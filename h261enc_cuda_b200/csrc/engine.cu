@@ -123,6 +123,7 @@ struct Mirror {
     uint8_t *host = nullptr;
     uint8_t *dev = nullptr;
     size_t cap = 0;
+    uint64_t generation = 0;   /* of the two buffers: an address may come back, this does not */
     /* grow to at least `bytes`; the first `keep` host bytes survive */
     int reserve(size_t bytes, size_t keep = 0)
     {
@@ -148,6 +149,7 @@ struct Mirror {
         host = nh;
         dev = nd;
         cap = c;
+        generation++;
         return H261B_OK;
     }
     void release()
@@ -354,12 +356,12 @@ struct h261b_engine_s {
     std::vector<int32_t> queue;
     std::vector<int32_t> step_sessions[NSLOT];
     /* what each slot's work list holds: the sizes of its sessions in order
-     * (and whether rate-controlled), where it lies, and whether the device
-     * copy is the same.  Steps of the same sessions, a stream's usual case,
-     * write and upload it once. */
+     * (and whether rate-controlled), where it lies (in which buffers of the
+     * descriptor arena), and whether the device copy is the same.  Steps of
+     * the same sessions, a stream's usual case, write and upload it once. */
     struct WorkList {
         std::vector<uint32_t> sizes;
-        const void *host = nullptr, *dev = nullptr;
+        uint64_t generation = 0;
         size_t off = 0;
         bool uploaded = false;
     } work_list[NSLOT];
@@ -1361,7 +1363,7 @@ extern "C" int h261b_engine_step(h261b_engine_t *e)
      * rate-controlled ones (the second encode launch takes that tail) */
     h261b_engine_s::WorkList &wl = e->work_list[p];
     {
-        bool same = wl.host == dm.host && wl.dev == dm.dev && wl.off == work_off && wl.sizes.size() == n;
+        bool same = wl.generation == dm.generation && wl.off == work_off && wl.sizes.size() == n;
         for (size_t k = 0; k < n; k++) {
             const Session &s = e->sessions[(size_t)list[k]];
             const uint32_t size = (uint32_t)s.nmb | (s.rc ? 1u << 31 : 0u);
@@ -1371,8 +1373,7 @@ extern "C" int h261b_engine_step(h261b_engine_t *e)
                 rc_begin += s.nmb;
         }
         if (!same) {
-            wl.host = dm.host;
-            wl.dev = dm.dev;
+            wl.generation = dm.generation;
             wl.off = work_off;
             wl.uploaded = false;
             wl.sizes.resize(n);
