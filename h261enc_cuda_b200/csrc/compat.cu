@@ -103,6 +103,9 @@ bool ensure_work(const char *where, int32_t nmb)
     cudaError_t e1 = cudaMalloc(&g.work_dev, sizeof(uint32_t) * nmb);
     cudaError_t e2 = e1 == cudaSuccess ? cudaMemcpy(g.work_dev, host, sizeof(uint32_t) * nmb, cudaMemcpyHostToDevice)
                                        : e1;
+    /* (the copy of a pageable list may outlive its call) */
+    if (e2 == cudaSuccess)
+        e2 = cudaStreamSynchronize(cudaStreamLegacy);
     free(host);
     if (e2 != cudaSuccess) {
         fail(where, e2);

@@ -614,7 +614,9 @@ extern "C" int h261b_engine_create(const h261b_engine_config_t *cfg, h261b_engin
              cudaEventCreate(&e->t_end[p]) == cudaSuccess;
     }
     ok = ok && cudaMalloc(&e->sched_dev, 2 * NSLOT * sizeof(int32_t)) == cudaSuccess &&
-         cudaMemset(e->sched_dev, 0, 2 * NSLOT * sizeof(int32_t)) == cudaSuccess;
+         cudaMemset(e->sched_dev, 0, 2 * NSLOT * sizeof(int32_t)) == cudaSuccess &&
+         /* the clear may outlive its call, and the engine's streams do not wait for this one */
+         cudaStreamSynchronize(cudaStreamLegacy) == cudaSuccess;
     if (!ok) {
         set_error("h261b_engine_create: device setup failed: %s", cudaGetErrorString(cudaGetLastError()));
         h261b_engine_destroy(e);

@@ -2002,7 +2002,9 @@ extern "C" int h261b_set_quant_table(void)
     tab[0] = 0.0f;
     for (int q = 1; q < 32; q++)
         tab[q] = (float)(1.0 / (double)(float)(q * 2));
-    return (int)cudaMemcpyToSymbol(c_inv_quant, tab, sizeof(tab));
+    const cudaError_t err = cudaMemcpyToSymbol(c_inv_quant, tab, sizeof(tab));
+    /* in place before a stream that does not wait for the legacy stream */
+    return (int)(err != cudaSuccess ? err : cudaStreamSynchronize(cudaStreamLegacy));
 }
 
 namespace {

@@ -72,6 +72,9 @@ int scratch_for_device(int dev, uint32_t **out, int *sms)
         for (uint32_t i = 0; i < H261B_NOALLOC_MAX_MB; i++)
             work[i] = i;
         err = cudaMemcpy((uint8_t *)addr + kDescBytes, work, sizeof(work), cudaMemcpyHostToDevice);
+        /* the copy may outlive its call; the caller's stream may not wait for this one */
+        if (err == cudaSuccess)
+            err = cudaStreamSynchronize(cudaStreamLegacy);
         if (err == cudaSuccess)
             err = cudaDeviceGetAttribute(&g_sms[dev], cudaDevAttrMultiProcessorCount, dev);
         if (err != cudaSuccess || h261b_set_quant_table() != 0) {
