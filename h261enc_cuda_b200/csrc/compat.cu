@@ -89,6 +89,16 @@ bool ensure_ready(const char *where)
     return true;
 }
 
+/* the picture memory is there, all of it */
+bool ensure_textures(const char *where)
+{
+    if (!g.cur || !g.ref || !g.rec || !g.stage) {
+        fail_arg(where, "h261_gpu_device_init_textures has not been called");
+        return false;
+    }
+    return true;
+}
+
 /* one work list covering every MB of the picture */
 bool ensure_work(const char *where, int32_t nmb)
 {
@@ -148,13 +158,9 @@ cudaError_t drain()
 void upload(const char *where, int which, int plane, const uint8_t *data, int32_t w, int32_t h, int32_t ew,
             int32_t eh)
 {
-    if (!ensure_ready(where))
+    if (!ensure_ready(where) || !ensure_textures(where))
         return;
     uint8_t *pic = which ? g.ref : g.cur;
-    if (!pic || !g.stage) {
-        fail_arg(where, "h261_gpu_device_init_textures has not been called");
-        return;
-    }
     if (!data || w != ew || h != eh) {
         fail_arg(where, "plane size does not match the initialised picture");
         return;
@@ -329,9 +335,9 @@ extern "C" void h261_gpu_device_deinit_me(me_gpu_t **pps)
 extern "C" void h261_gpu_device_me(me_gpu_t *s)
 {
     const char *where = "h261_gpu_device_me";
-    if (!ensure_ready(where))
+    if (!ensure_ready(where) || !ensure_textures(where))
         return;
-    if (!s || !g.cur || s->i_mb_width != g.w / 16 || s->i_mb_height != g.h / 16) {
+    if (!s || s->i_mb_width != g.w / 16 || s->i_mb_height != g.h / 16) {
         fail_arg(where, "ME state does not match the initialised picture");
         return;
     }
@@ -475,7 +481,7 @@ extern "C" void h261_deinit_macroblocks(h261_macroblocks_t *s)
 extern "C" void h261_gpu_device_encode_macroblocks(h261_context_t *ctx)
 {
     const char *where = "h261_gpu_device_encode_macroblocks";
-    if (!ensure_ready(where))
+    if (!ensure_ready(where) || !ensure_textures(where))
         return;
     if (!ctx || !ctx->ps_macroblocks || !ctx->ps_mode_decision || !ctx->ps_mode_decision->prgs_mb || !g.dn_dev) {
         fail_arg(where, "context is missing macroblocks or mode decision");
@@ -557,7 +563,7 @@ extern "C" void h261_gpu_device_encode_macroblocks(h261_context_t *ctx)
 extern "C" void h261_gpu_device_decode_macroblocks(h261_context_t *ctx)
 {
     const char *where = "h261_gpu_device_decode_macroblocks";
-    if (!ensure_ready(where))
+    if (!ensure_ready(where) || !ensure_textures(where))
         return;
     if (!ctx || !ctx->ps_macroblocks) {
         fail_arg(where, "context is missing macroblocks");

@@ -33,6 +33,8 @@ static char *fake_base;
 static bool fake_used[kSlots];
 /* an address for an allocation of `bytes` (pinned: host memory), or NULL */
 static std::function<void *(size_t bytes, bool pinned)> fake_pick;
+/* allocations that succeed before one fails (-1: none fails) */
+static int fake_fail_after = -1;
 /* legacy-stream work that may still be under way when its call returns:
  * copies from pageable memory to the device and clears.  Done by a wait for
  * the device or for the legacy stream. */
@@ -71,9 +73,18 @@ static void fake_run_pending()
 }
 
 extern "C" {
-cudaError_t cudaMalloc(void **p, size_t n) { *p = fake_alloc(n, false); return cudaSuccess; }
-cudaError_t cudaHostAlloc(void **p, size_t n, unsigned) { *p = fake_alloc(n, true); return cudaSuccess; }
-cudaError_t cudaMallocHost(void **p, size_t n) { *p = fake_alloc(n, true); return cudaSuccess; }
+static cudaError_t fake_alloc_to(void **p, size_t n, bool pinned)
+{
+    if (fake_fail_after == 0)
+        return cudaErrorMemoryAllocation;
+    if (fake_fail_after > 0)
+        fake_fail_after--;
+    *p = fake_alloc(n, pinned);
+    return cudaSuccess;
+}
+cudaError_t cudaMalloc(void **p, size_t n) { return fake_alloc_to(p, n, false); }
+cudaError_t cudaHostAlloc(void **p, size_t n, unsigned) { return fake_alloc_to(p, n, true); }
+cudaError_t cudaMallocHost(void **p, size_t n) { return fake_alloc_to(p, n, true); }
 cudaError_t cudaHostGetDevicePointer(void **d, void *h, unsigned) { *d = h; return cudaSuccess; }
 cudaError_t cudaFree(void *p)
 {
