@@ -571,6 +571,10 @@ extern "C" void h261_gpu_device_decode_macroblocks(h261_context_t *ctx)
     }
     h261_macroblocks_t *s = ctx->ps_macroblocks;
     const size_t ny = (size_t)g.w * g.h, nc = ny / 4;
+    if (ny > (size_t)s->i_num_mb * 256) {
+        fail_arg(where, "the picture is larger than the macroblock state's host arrays");
+        return;
+    }
     CK(where, cudaMemcpyAsync(s->pui8_reconstructed_Y_host, g.rec + g.lay.off_y, ny, cudaMemcpyDeviceToHost,
                               g.stream));
     CK(where, cudaMemcpyAsync(s->pui8_reconstructed_Cb_host, g.rec + g.lay.off_cb, nc, cudaMemcpyDeviceToHost,

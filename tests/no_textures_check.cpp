@@ -82,6 +82,13 @@ int main()
     }
     h261_gpu_device_init_textures(w, h);
     calls("with textures again", true);
+    /* a picture larger than the macroblock state's host arrays */
+    h261_gpu_device_init_textures(2 * w, 2 * h);
+    g.status = H261B_OK;
+    ctx.ps_macroblocks->pui8_reconstructed_Y_host[(size_t)n * 256 - 1] = 99;
+    h261_gpu_device_decode_macroblocks(&ctx);
+    CHECK_THAT(h261b_abi_last_status() == H261B_ERR_ARG, "a picture of another size was decoded");
+    CHECK_THAT(ctx.ps_macroblocks->pui8_reconstructed_Y_host[(size_t)n * 256 - 1] == 99, "and written");
     h261_deinit_macroblocks(ctx.ps_macroblocks);
     h261_gpu_device_deinit_me(&me);
     h261_gpu_device_deinit_textures();
