@@ -2107,17 +2107,16 @@ extern "C" int h261b_launch_step(const h261b_session_dev_t *sessions_dev, const 
         if (!sms[dev]) {
             if ((err = cudaDeviceGetAttribute(&sms[dev], cudaDevAttrMultiProcessorCount, dev)) != cudaSuccess)
                 return (int)err;
-            const int max_smem = (int)(sizeof(WarpSmem) * 8 + sizeof(VlcTables));
-            for (int f = 0; f < 2; f++)
-                for (int k = 0; k < 4; k++)
-                    for (int x = 0; x < 16; x++)
-                        if ((err = cudaFuncSetAttribute(step_fn(f, k, x & 1, (x >> 1) & 1, (x >> 2) & 1, x >> 3),
-                                                        cudaFuncAttributeMaxDynamicSharedMemorySize, max_smem)) !=
-                            cudaSuccess)
-                            return (int)err;
         }
         int &r = resident[dev][fmad][kind][full][abi][bulk][code][warps_per_cta];
         if (!r) {
+            /* the first launch of this instantiation.  CUDA loads a kernel when
+             * it is first named: naming all 52 here took 2.5 ms of a process's
+             * first launch (a QCIF stream's first 40 pictures 14.2 ms, 12.0 so) */
+            err = cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                       (int)(sizeof(WarpSmem) * 8 + sizeof(VlcTables)));
+            if (err != cudaSuccess)
+                return (int)err;
             err = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&r, fn, threads, smem);
             if (err != cudaSuccess)
                 return (int)err;
