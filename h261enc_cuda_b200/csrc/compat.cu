@@ -194,10 +194,6 @@ extern "C" void h261_gpu_init(void)
     CK("h261_gpu_init", cudaSetDevice(g.device));
     if (!g.stream)
         CK("h261_gpu_init", cudaStreamCreateWithFlags(&g.stream, cudaStreamNonBlocking));
-    if (h261b_set_quant_table() != 0) {
-        fail("h261_gpu_init", cudaGetLastError());
-        return;
-    }
     if (!g.desc_dev)
         CK("h261_gpu_init", cudaMalloc(&g.desc_dev, sizeof(h261b_session_dev_t)));
     CK("h261_gpu_init", cudaDeviceGetAttribute(&g.sms, cudaDevAttrMultiProcessorCount, g.device));

@@ -601,7 +601,7 @@ extern "C" int h261b_engine_create(const h261b_engine_config_t *cfg, h261b_engin
         copiers = std::max(1, std::min(8, (int)std::thread::hardware_concurrency() / 2));
     e->copier.reset(new CopyPool(copiers - 1));   /* the caller is one of them */
     cudaDeviceProp prop;
-    bool ok = cudaGetDeviceProperties(&prop, cfg->device) == cudaSuccess && h261b_set_quant_table() == 0;
+    bool ok = cudaGetDeviceProperties(&prop, cfg->device) == cudaSuccess;
     for (int p = 0; p < NSLOT && ok; p++) {
         ok = cudaStreamCreateWithFlags(&e->stream[p], cudaStreamNonBlocking) == cudaSuccess &&
              cudaStreamCreateWithFlags(&e->side[p], cudaStreamNonBlocking) == cudaSuccess &&

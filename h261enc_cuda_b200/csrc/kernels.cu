@@ -43,10 +43,8 @@
 #include <cuda_runtime.h>
 #include <stdint.h>
 
-#include <algorithm>
-#include <mutex>
-
 #include "h261b_device.h"
+#include "parts.h"
 #include "vlc_coder.h"
 
 namespace {
@@ -104,19 +102,6 @@ static_assert(kEncodeWarpBytes % 16 == 0 && sizeof(WarpSmem) % 16 == 0, "warp sh
 static_assert(alignof(WarpSmem) >= alignof(VlcTables), "the tables follow the warps' shared memory");
 static_assert(kSearchWarpBytes % 16 == 0 && offsetof(WarpSmem, t) == kSearchWarpBytes, "warp shared layout");
 
-/* what a launch of the step kernel does per MB */
-enum StepKind {
-    KIND_FUSED = 0,    /* the phases the launch asks for, in one pass       */
-    KIND_SEARCH = 1,   /* search, costs and mode decision (into md_out)     */
-    KIND_ENCODE = 2,   /* MC ... reconstruction from md_in, after a search
-                          launch (programmatic dependent launch: waits for
-                          that grid before it reads anything)               */
-    KIND_FULL = 3,     /* KIND_FUSED with every phase (search, mode decision,
-                          encode): the engine's and the no-allocation
-                          entry point's launch, compiled without the paths
-                          of partial launches                               */
-};
-
 /* the coarse grid's offsets { -14, -11, -8, -5, -2, 0, 2, 5, 8, 11, 14 }
  * (megpu_kernels.cuh:27-166), by arithmetic: lanes index it at 11 places
  * at once, which a constant-memory table would serve one address at a time */
@@ -127,7 +112,13 @@ __device__ __forceinline__ int stage1_offset(int t)
 /* float tables initialised from double literals like the reference's */
 __constant__ float c_fwd_post[8] = { 1.0, 0.720960, 0.765367, 0.850430, 1.0, 1.272759, 1.847759, 3.624510 };
 __constant__ float c_inv_pre[8] = { 1.0, 1.387040, 1.306563, 1.175876, 1.0, 0.785695, 0.541196, 0.275899 };
-__constant__ float c_inv_quant[32];
+/* f_inv_quant = 1.0 / ( float ) ( i_quant * 2 ) (mbgpu_kernels.cuh:685), an
+ * IEEE double rounded to float; by QUANT, 0 unused */
+#define INV_QUANT(q) (float)(1.0 / (double)(float)((q) * 2))
+#define INV_QUANT4(q) INV_QUANT(q), INV_QUANT(q + 1), INV_QUANT(q + 2), INV_QUANT(q + 3)
+__constant__ float c_inv_quant[32] = { 0.0f,           INV_QUANT(1),   INV_QUANT(2),   INV_QUANT(3),  INV_QUANT4(4),
+                                       INV_QUANT4(8),  INV_QUANT4(12), INV_QUANT4(16), INV_QUANT4(20),
+                                       INV_QUANT4(24), INV_QUANT4(28) };
 
 /* ------------------------------------------------ debug bounds checks
  *
@@ -299,18 +290,6 @@ __device__ __forceinline__ bool mbar_wait_bounded(uint64_t *bar, uint32_t parity
     if (lane == 0)
         atomicAdd(&g_stage_timeouts, 1u);
     return false;
-}
-
-/* sum of |a_i - b_i| over the four bytes, added to acc: one instruction,
- * one ALU-pipe slot (2.1 cycles a warp on an SM quarter).  The accumulating
- * form is written in PTX because acc += __vsadu4(a, b) compiles to a
- * separate add (5.1 against 4.05 cycles a word with its funnel shift), and
- * __vabsdiffu4 + __dp4a issues two instructions for the same ALU time. */
-__device__ __forceinline__ uint32_t sad4(uint32_t a, uint32_t b, uint32_t acc)
-{
-    uint32_t d;
-    asm("vabsdiff4.u32.u32.u32.add %0, %1, %2, %3;" : "=r"(d) : "r"(a), "r"(b), "r"(acc));
-    return d;
 }
 
 __device__ __forceinline__ uint32_t sad16(uint4 c, const uint32_t w[4], uint32_t acc)
@@ -1626,8 +1605,6 @@ __global__ void __launch_bounds__(256, KIND == KIND_SEARCH ? H261B_SEARCH_MIN_BL
  * eight vectors each of the exhaustive search, the three costs on three
  * warps, luma and chroma passes side by side, and the coding of the bits on a
  * third warp.  The arithmetic is the one-warp kernel's throughout. */
-constexpr int TEAM_WARPS = 4, TEAM_THREADS = 32 * TEAM_WARPS;
-
 struct TeamSmem {
     alignas(16) uint32_t buf[WIN_ROWS * WIN_PITCH_W];   /* buffer 0 of the one-warp layout */
     alignas(16) float t[2][4][TB_BLOCK];                /* luma, chroma                    */
@@ -1657,7 +1634,7 @@ __device__ __forceinline__ uint32_t sad_rows(const StageBuf s, int vx, int vy, i
 
 /* SADs of eight vectors one below the other from (vx, vy0) on: each window
  * row is aligned once for all of them */
-__device__ __forceinline__ void sad_column8(const StageBuf s, int vx, int vy0, uint32_t sad[8])
+[[maybe_unused]] __device__ __forceinline__ void sad_column8(const StageBuf s, int vx, int vy0, uint32_t sad[8])
 {
     const int b = 16 + vx;
     const uint32_t *p = s.win(15 + vy0, b >> 2);
@@ -1677,7 +1654,7 @@ __device__ __forceinline__ void sad_column8(const StageBuf s, int vx, int vy0, u
 }
 
 /* the least of the team's keys */
-__device__ __forceinline__ uint32_t team_min(TeamSmem &sm, int stage, uint32_t key, int tid)
+[[maybe_unused]] __device__ __forceinline__ uint32_t team_min(TeamSmem &sm, int stage, uint32_t key, int tid)
 {
     key = __reduce_min_sync(FULL, key);
     if ((tid & 31) == 0)
@@ -1956,286 +1933,83 @@ __global__ void __launch_bounds__(TEAM_THREADS, 4)
 
 } // namespace
 
-extern "C" int h261b_debug_check_status(int32_t *enabled, int64_t *violations, int32_t *first_site,
-                                        int32_t *first_value)
+namespace {
+
+constexpr int PART_FMAD = (H261B_PART >> 2) & 1;
+constexpr bool PART_FULL = ((H261B_PART >> 1) & 1) != 0, PART_BULK = (H261B_PART & 1) != 0;
+
+/* the instantiation of a launch's flags: the encode kind has no search and
+ * writes no reference-layout output, the search kind no encode output */
+template <bool CODE>
+StepFn step_of(int kind)
 {
-    if (!enabled || !violations || !first_site || !first_value)
-        return H261B_ERR_ARG;
-    *violations = 0;
-    *first_site = *first_value = 0;
+    if constexpr (!PART_FULL)
+        if (kind == KIND_ENCODE)
+            return step_kernel<PART_FMAD, KIND_ENCODE, false, false, PART_BULK, CODE>;
+    return kind == KIND_FULL ? step_kernel<PART_FMAD, KIND_FULL, PART_FULL, false, PART_BULK, CODE>
+                             : step_kernel<PART_FMAD, KIND_FUSED, PART_FULL, false, PART_BULK, CODE>;
+}
+
+StepFn part_step(int kind, int abi, int code)
+{
+    if (kind == KIND_SEARCH)
+        return step_kernel<PART_FMAD, KIND_SEARCH, PART_FULL, false, PART_BULK, false>;
+#if !(H261B_PART & 1)
+    if (abi)
+        return step_kernel<PART_FMAD, KIND_FUSED, PART_FULL, true, false, false>;
+#else
+    (void)abi;
+#endif
+    return code ? step_of<true>(kind) : step_of<false>(kind);
+}
+
+#if H261B_PART & 1
+/* (bulk staging: no team kernels) */
+TeamFn part_team(int) { return nullptr; }
+TeamPictureFn part_team_picture(int) { return nullptr; }
+#else
+TeamFn part_team(int code)
+{
+    return code ? team_kernel<PART_FMAD, PART_FULL, true> : team_kernel<PART_FMAD, PART_FULL, false>;
+}
+
+TeamPictureFn part_team_picture(int abi)
+{
+    return abi ? team_picture_kernel<PART_FMAD, PART_FULL, true> : team_picture_kernel<PART_FMAD, PART_FULL, false>;
+}
+#endif
+
+int part_checks(unsigned long long *n, int first[2])
+{
+    *n = 0;
 #ifdef H261B_DEBUG_CHECKS
-    *enabled = 1;
-    unsigned long long n = 0;
-    int first[2] = { 0, 0 };
     const unsigned long long zero = 0;
-    if (cudaMemcpyFromSymbol(&n, g_check_count, sizeof(n)) != cudaSuccess ||
-        cudaMemcpyFromSymbol(first, g_check_first, sizeof(first)) != cudaSuccess ||
+    if (cudaMemcpyFromSymbol(n, g_check_count, sizeof(*n)) != cudaSuccess ||
+        cudaMemcpyFromSymbol(first, g_check_first, 2 * sizeof(int)) != cudaSuccess ||
         cudaMemcpyToSymbol(g_check_count, &zero, sizeof(zero)) != cudaSuccess)
         return H261B_ERR_CUDA;
-    *violations = (int64_t)n;
-    *first_site = first[0];
-    *first_value = first[1];
 #else
-    *enabled = 0;
+    (void)first;
 #endif
     return H261B_OK;
 }
 
-extern "C" int h261b_stage_status(int64_t *timeouts)
+int part_timeouts(unsigned int *n)
 {
-    if (!timeouts)
-        return H261B_ERR_ARG;
-    unsigned int n = 0;
     const unsigned int zero = 0;
-    if (cudaMemcpyFromSymbol(&n, g_stage_timeouts, sizeof(n)) != cudaSuccess ||
+    if (cudaMemcpyFromSymbol(n, g_stage_timeouts, sizeof(*n)) != cudaSuccess ||
         cudaMemcpyToSymbol(g_stage_timeouts, &zero, sizeof(zero)) != cudaSuccess)
         return H261B_ERR_CUDA;
-    *timeouts = (int64_t)n;
     return H261B_OK;
 }
 
-extern "C" int h261b_set_quant_table(void)
-{
-    /* f_inv_quant = 1.0 / ( float ) ( i_quant * 2 ) (mbgpu_kernels.cuh:685),
-     * evaluated on the host in IEEE double and rounded to float */
-    float tab[32];
-    tab[0] = 0.0f;
-    for (int q = 1; q < 32; q++)
-        tab[q] = (float)(1.0 / (double)(float)(q * 2));
-    const cudaError_t err = cudaMemcpyToSymbol(c_inv_quant, tab, sizeof(tab));
-    /* in place before a stream that does not wait for the legacy stream */
-    return (int)(err != cudaSuccess ? err : cudaStreamSynchronize(cudaStreamLegacy));
-}
-
-namespace {
-
-using StepFn = void (*)(const h261b_session_dev_t *, const uint32_t *, int32_t, int32_t, int32_t, int32_t *);
-
-/* the instantiation of a launch's flags: the encode kind has no search and
- * writes no reference-layout output, the search kind no encode output */
-template <int FMAD, bool BULK, bool CODE>
-StepFn step_fn_of(int kind, int full)
-{
-    if (kind == KIND_ENCODE)
-        return step_kernel<FMAD, KIND_ENCODE, false, false, BULK, CODE>;
-    if (kind == KIND_FULL)
-        return full ? step_kernel<FMAD, KIND_FULL, true, false, BULK, CODE>
-                    : step_kernel<FMAD, KIND_FULL, false, false, BULK, CODE>;
-    return full ? step_kernel<FMAD, KIND_FUSED, true, false, BULK, CODE>
-                : step_kernel<FMAD, KIND_FUSED, false, false, BULK, CODE>;
-}
-
-template <int FMAD, bool BULK>
-StepFn step_fn_of(int kind, int full, int code)
-{
-    if (kind == KIND_SEARCH)
-        return full ? step_kernel<FMAD, KIND_SEARCH, true, false, BULK, false>
-                    : step_kernel<FMAD, KIND_SEARCH, false, false, BULK, false>;
-    return code ? step_fn_of<FMAD, BULK, true>(kind, full) : step_fn_of<FMAD, BULK, false>(kind, full);
-}
-
-template <int FMAD>
-StepFn step_fn_of(int kind, int full, int abi, int bulk, int code)
-{
-    if (abi && kind != KIND_ENCODE && kind != KIND_SEARCH)
-        return full ? step_kernel<FMAD, KIND_FUSED, true, true, false, false>
-                    : step_kernel<FMAD, KIND_FUSED, false, true, false, false>;
-    return bulk ? step_fn_of<FMAD, true>(kind, full, code) : step_fn_of<FMAD, false>(kind, full, code);
-}
-
-using TeamFn = void (*)(const h261b_session_dev_t *, const uint32_t *, int32_t);
-
-template <int FMAD>
-TeamFn team_fn(bool full, bool code)
-{
-    if (code)
-        return full ? team_kernel<FMAD, true, true> : team_kernel<FMAD, false, true>;
-    return full ? team_kernel<FMAD, true, false> : team_kernel<FMAD, false, false>;
-}
-
-StepFn step_fn(int fmad, int kind, int full, int abi, int bulk, int code)
-{
-    return fmad ? step_fn_of<1>(kind, full, abi, bulk, code) : step_fn_of<0>(kind, full, abi, bulk, code);
-}
-
 } // namespace
 
-extern "C" int h261b_launch_step(const h261b_session_dev_t *sessions_dev, const uint32_t *work_dev,
-                                 int32_t n_work, int32_t phases, int32_t warps_per_cta, int32_t max_ctas,
-                                 int32_t *sched_dev, void *stream)
-{
-    if (n_work <= 0)
-        return 0;
-    if (warps_per_cta < 1 || warps_per_cta > 8)
-        return (int)cudaErrorInvalidValue;
-    const int fmad = (phases >> 8) & 1;
-    if (phases & H261B_LAUNCH_TEAM) {
-        const bool full = (phases & H261B_LAUNCH_ME_FULL) != 0, code = (phases & H261B_CODE_INLINE) != 0;
-        if (phases & (H261B_ABI_OUT | H261B_STAGE_BULK | (3 << H261B_KIND_SHIFT)))
-            return (int)cudaErrorInvalidValue;
-        const TeamFn fn = fmad ? team_fn<1>(full, code) : team_fn<0>(full, code);
-        fn<<<n_work, TEAM_THREADS, 0, (cudaStream_t)stream>>>(sessions_dev, work_dev, phases & 0xFF);
-        return (int)cudaGetLastError();
-    }
-    int kind = (phases >> H261B_KIND_SHIFT) & 3;
-    /* a fused launch of every phase runs the kernel compiled for exactly that */
-    const int all_phases = H261B_PHASE_ME | H261B_PHASE_MD | H261B_PHASE_ENCDEC;
-    if (kind == KIND_FUSED && (phases & all_phases) == all_phases)
-        kind = KIND_FULL;
-    const int full = (phases & H261B_LAUNCH_ME_FULL) ? 1 : 0, abi = (phases & H261B_ABI_OUT) ? 1 : 0;
-    const int bulk = (phases & H261B_STAGE_BULK) ? 1 : 0;
-    const int code = (phases & H261B_CODE_INLINE) ? 1 : 0;
-    const bool pdl = (phases & H261B_LAUNCH_PDL) != 0;
-    const int tail_code = (phases >> H261B_TAIL_SHIFT) & 15;
-    if (kind > KIND_FULL)
-        return (int)cudaErrorInvalidValue;
-    const int ph = phases & (0xFF | H261B_STAGE_SHORT | H261B_LAUNCH_PDL);
-    const int threads = warps_per_cta * 32;
-    const bool codes = code && kind != KIND_SEARCH && !abi;
-    const size_t warp_bytes = kind == KIND_SEARCH ? kSearchWarpBytes : codes ? sizeof(WarpSmem) : kEncodeWarpBytes;
-    const size_t smem = warp_bytes * (size_t)warps_per_cta + (codes ? sizeof(VlcTables) : 0);
-    const StepFn fn = step_fn(fmad, kind, full, abi, bulk, code);
-    static std::mutex mu;
-    static int sms[64], resident[64][2][4][2][2][2][2][9];
-    int dev = 0;
-    cudaError_t err = cudaGetDevice(&dev);
-    if (err != cudaSuccess || dev < 0 || dev >= 64)
-        return (int)(err != cudaSuccess ? err : cudaErrorInvalidDevice);
-    int per_sm = 0, nsm = 0;
-    {
-        std::lock_guard<std::mutex> lock(mu);
-        if (!sms[dev]) {
-            if ((err = cudaDeviceGetAttribute(&sms[dev], cudaDevAttrMultiProcessorCount, dev)) != cudaSuccess)
-                return (int)err;
-        }
-        int &r = resident[dev][fmad][kind][full][abi][bulk][code][warps_per_cta];
-        if (!r) {
-            /* the first launch of this instantiation.  CUDA loads a kernel when
-             * it is first named: naming all 52 here took 2.5 ms of a process's
-             * first launch (a QCIF stream's first 40 pictures 14.2 ms, 12.0 so) */
-            err = cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                       (int)(sizeof(WarpSmem) * 8 + sizeof(VlcTables)));
-            if (err != cudaSuccess)
-                return (int)err;
-            err = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&r, fn, threads, smem);
-            if (err != cudaSuccess)
-                return (int)err;
-            r = r < 1 ? 1 : r;
-        }
-        per_sm = r;
-        nsm = sms[dev];
-    }
-    /* one wave of resident CTAs */
-    int ctas = max_ctas > 0 ? max_ctas : nsm * per_sm;
-    int chunk;
-    /* a MB a warp at most: nothing to balance, and no draw (an atomic's round
-     * trip before the first MB and one more after the last) */
-    if (n_work <= (long long)ctas * warps_per_cta)
-        sched_dev = nullptr;
-    if (sched_dev) {
-        /* static runs of all but about `tail` items per warp, the rest drawn
-         * from the scheduler (tail_code: tail + 1, 0 for the default 2) */
-        const int tail = tail_code ? tail_code - 1 : 2;
-        ctas = (int)std::min<long long>(ctas, (n_work + warps_per_cta - 1) / warps_per_cta);
-        const long long total_warps = (long long)ctas * warps_per_cta;
-        chunk = (int)std::max<long long>(0, n_work / total_warps - tail);
-    } else {
-        /* contiguous runs covering every item */
-        const long long total_warps = (long long)ctas * warps_per_cta;
-        chunk = (int)((n_work + total_warps - 1) / total_warps);
-        ctas = (n_work + chunk * warps_per_cta - 1) / (chunk * warps_per_cta);
-    }
-    cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = dim3((unsigned)ctas);
-    cfg.blockDim = dim3((unsigned)threads);
-    cfg.dynamicSmemBytes = smem;
-    cfg.stream = (cudaStream_t)stream;
-    cudaLaunchAttribute attr[1];
-    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-    attr[0].val.programmaticStreamSerializationAllowed = 1;
-    cfg.attrs = attr;
-    cfg.numAttrs = pdl ? 1 : 0;
-    return (int)cudaLaunchKernelEx(&cfg, fn, sessions_dev, work_dev, n_work, chunk, ph, sched_dev);
-}
-
-namespace {
-
-template <int FMAD, bool ABI>
-auto team_picture_fn(bool full)
-{
-    return full ? team_picture_kernel<FMAD, true, ABI> : team_picture_kernel<FMAD, false, ABI>;
-}
-
-} // namespace
-
-extern "C" int h261b_launch_team_picture(const h261b_session_dev_t *session, int32_t phases, void *stream)
-{
-    const bool fmad = (phases & H261B_FMAD_BIT) != 0, full = (phases & H261B_LAUNCH_ME_FULL) != 0;
-    const auto fn = (phases & H261B_ABI_OUT) ? (fmad ? team_picture_fn<1, true>(full) : team_picture_fn<0, true>(full))
-                                             : (fmad ? team_picture_fn<1, false>(full) : team_picture_fn<0, false>(full));
-    fn<<<session->mbw * session->mbh, TEAM_THREADS, 0, (cudaStream_t)stream>>>(*session, phases & 0xFF);
-    return (int)cudaGetLastError();
-}
-
-/* ------------------------------------------------ SAD primitive peak */
-
-namespace {
-
-/* the motion search's inner step, on registers: one funnel shift and one
- * 4-pixel SAD per word, eight independent chains per thread */
-__global__ void __launch_bounds__(256) sad_peak_kernel(const uint32_t *__restrict__ in, uint32_t *__restrict__ out,
-                                                       int iters)
-{
-    uint32_t c[8], r[8];
-#pragma unroll
-    for (int i = 0; i < 8; i++) {
-        c[i] = in[(threadIdx.x + i) & 255];
-        r[i] = in[(threadIdx.x * 7 + i) & 255];
-    }
-    uint32_t acc = 0;
-    for (int it = 0; it < iters; it++) {
-#pragma unroll
-        for (int i = 0; i < 8; i++) {
-            acc = sad4(c[i], r[i], acc);
-            r[i] = __funnelshift_r(r[i], r[(i + 1) & 7], 8);
-        }
-    }
-    out[blockIdx.x * blockDim.x + threadIdx.x] = acc;
-}
-
-} // namespace
-
-extern "C" int h261b_measure_sad_peak(int32_t device, double *absdiff_per_s)
-{
-    if (!absdiff_per_s)
-        return -1;
-    int sms = 0;
-    if (cudaSetDevice(device) != cudaSuccess ||
-        cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device) != cudaSuccess)
-        return -2;
-    const int blocks = sms * 8, threads = 256, iters = 2048;
-    uint32_t *in = nullptr, *out = nullptr;
-    uint32_t h[256];
-    for (int i = 0; i < 256; i++)
-        h[i] = (uint32_t)i * 2654435761u;
-    cudaEvent_t a, b;
-    float ms = 0.f;
-    int rc = -2;
-    if (cudaMalloc(&in, sizeof(h)) == cudaSuccess && cudaMalloc(&out, sizeof(uint32_t) * blocks * threads) == cudaSuccess &&
-        cudaMemcpy(in, h, sizeof(h), cudaMemcpyHostToDevice) == cudaSuccess && cudaEventCreate(&a) == cudaSuccess &&
-        cudaEventCreate(&b) == cudaSuccess) {
-        sad_peak_kernel<<<blocks, threads>>>(in, out, 64);
-        cudaEventRecord(a);
-        sad_peak_kernel<<<blocks, threads>>>(in, out, iters);
-        cudaEventRecord(b);
-        if (cudaEventSynchronize(b) == cudaSuccess && cudaEventElapsedTime(&ms, a, b) == cudaSuccess && ms > 0.f) {
-            *absdiff_per_s = (double)blocks * threads * iters * 8 * 4 / (ms * 1e-3);
-            rc = 0;
-        }
-        cudaEventDestroy(a);
-        cudaEventDestroy(b);
-    }
-    cudaFree(in);
-    cudaFree(out);
-    return rc;
+#define PART_NAME2(n) kernel_part_##n
+#define PART_NAME(n) PART_NAME2(n)
+namespace h261b {
+const KernelPart PART_NAME(H261B_PART) = {
+    part_step, part_team, part_team_picture, part_checks, part_timeouts,
+    kSearchWarpBytes, kEncodeWarpBytes, sizeof(WarpSmem), sizeof(VlcTables),
+};
 }

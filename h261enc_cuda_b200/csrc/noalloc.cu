@@ -77,9 +77,8 @@ int scratch_for_device(int dev, uint32_t **out, int *sms)
             err = cudaStreamSynchronize(cudaStreamLegacy);
         if (err == cudaSuccess)
             err = cudaDeviceGetAttribute(&g_sms[dev], cudaDevAttrMultiProcessorCount, dev);
-        if (err != cudaSuccess || h261b_set_quant_table() != 0) {
-            set_error("h261b_encode_picture_noalloc: device set-up failed: %s",
-                      cudaGetErrorString(err != cudaSuccess ? err : cudaGetLastError()));
+        if (err != cudaSuccess) {
+            set_error("h261b_encode_picture_noalloc: device set-up failed: %s", cudaGetErrorString(err));
             return H261B_ERR_CUDA;
         }
         g_addr[dev] = (uint32_t *)addr;

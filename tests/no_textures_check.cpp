@@ -8,7 +8,6 @@
 #include "compat.cu"
 
 static int launches;
-extern "C" int h261b_set_quant_table(void) { return 0; }
 void h261b::set_error(const char *, ...) {}
 extern "C" int h261b_launch_team_picture(const h261b_session_dev_t *d, int32_t, void *)
 {

@@ -10,7 +10,6 @@
 static int steps_run;
 static std::vector<const void *> desc_host, desc_dev;   /* the descriptor arenas, by step slot */
 
-extern "C" int h261b_set_quant_table(void) { return 0; }
 extern "C" int64_t h261b_bits_slot_bytes(int32_t, int32_t) { return 0; }
 extern "C" h261b_bits_layout_t h261b_bits_layout(int32_t, int32_t) { return h261b_bits_layout_t{}; }
 extern "C" int h261b_launch_ratectrl(h261b_session_dev_t *, int32_t, void *) { return 0; }
