@@ -104,7 +104,6 @@ typedef struct {
     const h261_mb_mode_decision_t *md_in;
     /* outputs, any may be NULL */
     me_gpu_mb_t *me_out;          /* ME results per MB                      */
-    me_gpu_mv_t *stage1_out;      /* stage-1 vector per MB                  */
     h261_mb_mode_decision_t *md_out;
     h261_macroblock_t *abi_out;   /* reference layout, int32 levels         */
     h261b_mb_info_t *info_out;    /* compact layout                         */
@@ -182,8 +181,8 @@ typedef struct {
 #define H261B_STAGE_SHORT   0x20000
 /*   bit 18       the exhaustive +-15 search (the sessions' me_mode 1)
  *   bit 19       the launch may write the reference-layout outputs
- *                (abi_out, me_out, me_host, start_mv, cand_mv, stage1_out: the
- *                gpu_device.h boundary) */
+ *                (abi_out, me_out, me_host, start_mv, cand_mv: the gpu_device.h
+ *                boundary) */
 /*   bit 20       sessions with bits_out: each MB's coefficient bit string is
  *                made by the warp that encodes it */
 #define H261B_CODE_INLINE   0x100000

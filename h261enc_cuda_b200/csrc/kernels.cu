@@ -832,7 +832,7 @@ __device__ __forceinline__ void stage_mb(uint32_t *wbuf, int k, const h261b_sess
  * cache less) */
 template <bool FULL_SEARCH>
 __device__ __forceinline__ void motion_estimate(const StageBuf s, const h261b_session_dev_t &S, int mbx, int mby,
-                                                int lane, me_gpu_mb_t &res, int8_t &s1x, int8_t &s1y)
+                                                int lane, me_gpu_mb_t &res)
 {
     const int bx = mbx * 16, by = mby * 16;
     /* per-MB limits, gpu_device.cu:226-265 */
@@ -846,12 +846,9 @@ __device__ __forceinline__ void motion_estimate(const StageBuf s, const h261b_se
         const uint32_t best = full_search(s, lminx, lmaxx, lminy, lmaxy, lane) & 1023u;
         vx = (int)compact8(best) - 15;
         vy = (int)compact8(best >> 1) - 15;
-        s1x = s1y = 0;
     } else {
         const uint32_t coarse = grid_search(s, lminx, lmaxx, lminy, lmaxy, lane) & 1023u; /* Z-order index only */
         const int v1x = stage1_offset((int)compact8(coarse)), v1y = stage1_offset((int)compact8(coarse >> 1));
-        s1x = (int8_t)v1x;
-        s1y = (int8_t)v1y;
         const uint32_t best = refine_search(s, v1x, v1y, lminx, lmaxx, lminy, lmaxy, lane) & 1023u;
         vx = v1x + (int)compact8(best) - 3;
         vy = v1y + (int)compact8(best >> 1) - 3;
@@ -1288,7 +1285,7 @@ __device__ __forceinline__ void publish_run(const h261b_session_dev_t &S, int t,
 /* FMAD: the arithmetic of the reference's default build; KIND: what the
  * launch does per MB; FULL_SEARCH: the exhaustive search instead of the
  * reference's; ABI: the launch may write the reference-layout outputs
- * (h261_macroblock_t records, ME results, stage-1 vectors) that only the
+ * (h261_macroblock_t records, ME results and vectors) that only the
  * gpu_device.h boundary asks for; BULK: the search window comes by bulk row
  * copies; CODE: the launch makes the MBs' coefficient bit strings.  Each launch runs the instantiation for its flags
  * (h261b_launch_step), so no launch carries code it never runs: instruction
@@ -1453,20 +1450,14 @@ __global__ void __launch_bounds__(256, KIND == KIND_SEARCH ? H261B_SEARCH_MIN_BL
         me_gpu_mb_t me;
         me.i_intra_cost = me.i_zero_cost = me.i_16x16_cost = me.i_16x16_filter_cost = 0;
         me.s_16x16_mv.i8_mx = me.s_16x16_mv.i8_my = 0;
-        int8_t s1x = 0, s1y = 0;
         if (do_me || (phases & H261B_PHASE_MD))
             me.i_intra_cost = intra_cost(b, lane);   /* all that an intra picture needs */
         if (do_me) {
             /* the launch's search mode is the session's (checking build) */
             (void)H261B_CHECK(S.me_mode == (FULL_SEARCH ? 1 : 0), CHK_WORK_ITEM, S.me_mode);
-            motion_estimate<FULL_SEARCH>(b, S, mbx, mby, lane, me, s1x, s1y);
-            if (ABI && lane == 0) {
+            motion_estimate<FULL_SEARCH>(b, S, mbx, mby, lane, me);
+            if (ABI && lane == 0)
                 me_results_out(S, mb, me);
-                if (S.stage1_out) {
-                    S.stage1_out[mb].i8_mx = s1x;
-                    S.stage1_out[mb].i8_my = s1y;
-                }
-            }
         }
 
         MbDecision m;
