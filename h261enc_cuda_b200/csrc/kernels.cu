@@ -1946,7 +1946,7 @@ StepFn part_step(int kind, int abi, int code)
     if (kind == KIND_SEARCH)
         return step_kernel<PART_FMAD, KIND_SEARCH, PART_FULL, false, PART_BULK, false>;
 #if !(H261B_PART & 1)
-    if (abi)
+    if (abi && kind != KIND_ENCODE)
         return step_kernel<PART_FMAD, KIND_FUSED, PART_FULL, true, false, false>;
 #else
     (void)abi;

@@ -105,10 +105,11 @@ extern "C" int h261b_launch_step(const h261b_session_dev_t *sessions_dev, const 
         return (int)cudaErrorInvalidValue;
     const int ph = phases & (0xFF | H261B_STAGE_SHORT | H261B_LAUNCH_PDL);
     const int threads = warps_per_cta * 32;
-    const bool codes = code && kind != KIND_SEARCH && !abi;
-    /* the reference-layout outputs come with cp.async staging, the encode kind
-     * with the reference search's part */
-    const KernelPart &part = part_of(fmad, full && kind != KIND_ENCODE, bulk && !(abi && kind == KIND_FUSED));
+    /* the reference-layout outputs come with cp.async staging and no coding,
+     * the encode kind with the reference search's part */
+    const bool fused_abi = abi && kind != KIND_SEARCH && kind != KIND_ENCODE;
+    const bool codes = code && kind != KIND_SEARCH && !fused_abi;
+    const KernelPart &part = part_of(fmad, full && kind != KIND_ENCODE, bulk && !fused_abi);
     const size_t warp_bytes = kind == KIND_SEARCH ? part.search_bytes : codes ? part.code_bytes : part.encode_bytes;
     const size_t smem = warp_bytes * (size_t)warps_per_cta + (codes ? part.table_bytes : 0);
     const StepFn fn = part.step(kind, abi, code);
