@@ -10,12 +10,13 @@
  *     the table has no entry;
  *   - EOB (10) after the block.
  *
- * The encode kernel's warp codes each macroblock as soon as it has its
- * levels, from shared memory: the levels are put into transmission order,
- * each block gets a mask of its nonzero positions, and then every code of the
- * macroblock -- the levels of all of its blocks and an EOB after each -- has
- * a lane of its own.  The codes are ORed into a zeroed word buffer, MSB
- * first. */
+ * A warp codes a macroblock from its levels in shared memory -- in a small
+ * step the encode kernel's, as soon as it has them, in a larger one the codes
+ * kernel's (bitstream.cu), which loads them: the levels are put into
+ * transmission order, each block gets a mask of its nonzero positions, and
+ * then every code of the macroblock -- the levels of all of its blocks and an
+ * EOB after each -- has a lane of its own.  The codes are ORed into a zeroed
+ * word buffer, MSB first. */
 #pragma once
 
 #include <cstddef>

@@ -344,11 +344,14 @@ int h261b_stage_status(int64_t *timeouts);
  * or pool, or an allocation is not allowed where they run).  The caller
  * passes every input, output and state buffer as device memory; the small
  * scratch the kernel needs (descriptor and work list) is a fixed static
- * device array inside the library, so the call allocates nothing.  Limits:
+ * device array inside the library, so the call allocates nothing.  (A picture
+ * of up to four macroblocks a multiprocessor takes its descriptor with the
+ * launch and no scratch.)  Limits:
  * pictures of at most H261B_NOALLOC_MAX_MB macroblocks (larger ones are
  * refused with H261B_ERR_ARG); the first call on a device sets up the
- * scratch address and should come before any stream capture; calls whose
- * work overlaps on the GPU race on the shared scratch (use one stream). */
+ * scratch address and should come before any stream capture; calls on
+ * larger pictures whose work overlaps on the GPU race on the shared scratch
+ * (use one stream). */
 #define H261B_NOALLOC_MAX_MB      4096
 #define H261B_NOALLOC_STATE_BYTES 1040   /* per-stream denoise state          */
 

@@ -19,7 +19,8 @@
  *
  * Errors: like the reference, the entry points return nothing.  A failure
  * is printed to stderr and recorded; h261b_last_error() (declared in
- * h261b.h) returns the last recorded status.
+ * h261b.h) returns the last recorded message, h261b_abi_last_status() its
+ * status.
  */
 #ifndef H261B_ABI_H
 #define H261B_ABI_H
@@ -250,7 +251,11 @@ void h261_gpu_device_init_textures(int32_t i_width, int32_t i_height);
 void h261_gpu_device_deinit_textures(void);
 
 /* src/gpu_device.h:13-19 -- upload one packed plane (stride = width) of the
- * current (source) picture or of the reference (previous reconstruction). */
+ * current (source) picture or of the reference (previous reconstruction).
+ * When the call returns the bytes are the library's and the caller may change
+ * or free them; the transfer to the device may still be under way, as a
+ * pageable cudaMemcpy's may.  The next motion estimation or encode call waits
+ * for it, and an error that shows only then is that call's status. */
 void h261_gpu_device_set_current(uint8_t *pui8_frame_data, int32_t i_width, int32_t i_height);
 void h261_gpu_device_set_current_chroma_cb(uint8_t *pui8_frame_data, int32_t i_width, int32_t i_height);
 void h261_gpu_device_set_current_chroma_cr(uint8_t *pui8_frame_data, int32_t i_width, int32_t i_height);
