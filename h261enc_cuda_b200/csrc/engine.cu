@@ -9,7 +9,8 @@
  * caller through h261b_session_input); a step moves the whole arena with
  * one copy (with a kernel that reads it, where it is small) and runs one
  * launch over the flat (session, MB) work list; the kernels write the
- * compact results of all sessions into pinned host memory.
+ * compact results into pinned host memory where they make all of a step's
+ * there, and one copy brings them otherwise.
  *
  * Pipelining: steps rotate over NSLOT (3) slots, each with its CUDA stream
  * and its set of arenas.  Within a step the order is upload -> encode ->

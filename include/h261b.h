@@ -8,8 +8,8 @@
  *      and QUANT share one device; each h261b_engine_step() encodes the next
  *      picture of every session that has one queued, in one launch over a
  *      flat macroblock work list.  Source pictures go up in one transfer per
- *      step, the kernels write the compact results into pinned host memory,
- *      reconstructions stay in HBM as the next reference.  Steps rotate over
+ *      step, the compact results end in pinned host memory (written there by
+ *      the kernels, or by one copy), reconstructions stay in HBM as the next reference.  Steps rotate over
  *      three streams so that one step's transfers overlap the neighbouring
  *      steps' kernels.
  *
